@@ -446,7 +446,7 @@ def section_c4(qs, torch):
     ops = [qs.Hamiltonian(qs.SpinBasis1D(L, nup=13, pauli=False, **sy), terms) for sy in syms]
     t_build = time.perf_counter() - t
     sizes = [o.Ns for o in ops]
-    # warm-up: tile autotuning (cached per size class) and graph capture
+    # warm-up: graph capture and the pooled buffers
     t = time.perf_counter()
     for prec in ("fp64", "fp64df", "fp32"):
         qs.eigsh_batch(ops, k=1, tol=1e-10, precision=prec)

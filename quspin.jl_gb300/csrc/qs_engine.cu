@@ -354,31 +354,100 @@ __device__ __forceinline__ double block_sum(A v, double* sh) {
     return t;
 }
 
+// Warp totals of N per-lane accumulators by recursive halving: at each xor
+// distance a lane keeps half of its accumulators and hands the other half to
+// its partner, so N = 21 takes 11 + 6 + 3 + 2 + 1 = 23 adds a lane instead of
+// the 5 N = 105 of a butterfly over every accumulator (an FP64 add occupies the
+// SM's FP64 pipe for 16 cycles a warp whatever the lanes do with it: at 4,096
+// rows a block the butterflies were 30 % of the fused dots).  Every total is
+// the butterfly's own tree of additions, bit for bit.  Lane l ends with the
+// total of accumulator halve_pos<N>(l) in v[0] (-1: with nothing).
+template <class A, int N, int OFF, int M>
+__device__ __forceinline__ void halve_sums(A (&v)[M], int lane) {
+    if constexpr (OFF > 0) {
+        if constexpr (N == 1) {
+            v[0] = add(v[0], shfl(v[0], OFF));
+            halve_sums<A, 1, OFF / 2>(v, lane);
+        } else {
+            constexpr int H = (N + 1) / 2;
+            const bool up = (lane & OFF) != 0;
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const A hi = i + H < N ? v[i + H < N ? i + H : 0] : zero<A>();
+                const A keep = up ? hi : v[i], send = up ? v[i] : hi;
+                v[i] = add(keep, shfl(send, OFF));
+            }
+            halve_sums<A, H, OFF / 2>(v, lane);
+        }
+    }
+}
+template <int N, int OFF = 16>
+__device__ __forceinline__ int halve_pos(int lane) {
+    if constexpr (OFF == 0) {
+        return 0;
+    } else if constexpr (N == 1) {
+        return halve_pos<1, OFF / 2>(lane);
+    } else {
+        constexpr int H = (N + 1) / 2;
+        int p = halve_pos<H, OFF / 2>(lane);
+        if (p >= 0 && (lane & OFF)) p += H;
+        return p < N ? p : -1;
+    }
+}
+
+// Block totals of N accumulators; thread t < N returns the total of v[t].
+template <class A, int N>
+__device__ __forceinline__ double block_totals(A (&v)[N]) {
+    __shared__ double sh[kT / 32][N];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    halve_sums<A, N, 16>(v, lane);
+    const int pos = halve_pos<N>(lane);
+    if (pos >= 0) sh[wid][pos] = to_d(v[0]);
+    __syncthreads();
+    double t = 0;
+    if (threadIdx.x < N)
+        for (int q = 0; q < kT / 32; ++q) t += sh[q][threadIdx.x];
+    __syncthreads();   // sh is reused by the next call
+    return t;
+}
+
 // Block sums of the jt<A>() accumulators into row[(base + q) * 2 + {re, im}] for
 // the vectors i0 + q < nv (row: the block's slice of the partial buffer).
 template <class A>
 __device__ __forceinline__ void dots_epilogue(A* re, A* im, bool cv, int i0, int nv, int base, double* row) {
-    __shared__ double sh[kT / 32][2 * jt<A>()];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int J = jt<A>();
+    if (cv) {
+        A v[2 * J];
 #pragma unroll
-    for (int q = 0; q < jt<A>(); ++q) {
-        for (int o = 16; o > 0; o >>= 1) {
-            re[q] = add(re[q], shfl(re[q], o));
-            if (cv) im[q] = add(im[q], shfl(im[q], o));
+        for (int q = 0; q < J; ++q) {
+            v[2 * q] = re[q];
+            v[2 * q + 1] = im[q];
         }
-        if (lane == 0) {
-            sh[wid][2 * q] = to_d(re[q]);
-            sh[wid][2 * q + 1] = cv ? to_d(im[q]) : 0.0;
+        const double t = block_totals<A, 2 * J>(v);
+        if (threadIdx.x < 2 * J && i0 + (int)threadIdx.x / 2 < nv) row[base * 2 + threadIdx.x] = t;
+    } else {
+        A v[J];
+#pragma unroll
+        for (int q = 0; q < J; ++q) v[q] = re[q];
+        const double t = block_totals<A, J>(v);
+        if (threadIdx.x < J && i0 + (int)threadIdx.x < nv) {
+            row[(base + threadIdx.x) * 2] = t;
+            row[(base + threadIdx.x) * 2 + 1] = 0.0;
         }
     }
-    __syncthreads();
-    if (threadIdx.x < 2 * jt<A>()) {
-        double t = 0;
-        for (int q = 0; q < kT / 32; ++q) t += sh[q][threadIdx.x];
-        const int q = threadIdx.x / 2;
-        if (i0 + q < nv) row[(base + q) * 2 + (threadIdx.x & 1)] = t;
+}
+
+// The fused kernels' block sums: accumulators 0 .. nv-1 into their vectors'
+// partials and accumulator NV (a norm, when kept) into partial index mmax.
+template <class A, int NV>
+__device__ __forceinline__ void fused_epilogue(A (&acc)[NV + 1], int nv, bool norm, int mmax, double* row) {
+    const double t = block_totals<A, NV + 1>(acc);
+    const int i = threadIdx.x;
+    const int at = i < nv ? i : (i == NV && norm ? mmax : -1);
+    if (i <= NV && at >= 0) {
+        row[at * 2] = t;
+        row[at * 2 + 1] = 0.0;
     }
-    __syncthreads();   // sh is reused by the next call
 }
 
 template <class A>
@@ -431,17 +500,16 @@ __global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3) eng_do
 // (all loads before the arithmetic) and every column's sum advances, where
 // eng_dots reads w once per tile of jt columns.  Per thread the rows and the
 // multiply-add order of each column's sum and of ||w||^2 are those of
-// dots_rows, and the block sums go through dots_epilogue / block_sum, so the
-// partials are bit-identical to dots_block's.
+// dots_rows, and the block sums add in the order of dots_epilogue / block_sum,
+// so the partials are bit-identical to dots_block's.
 template <class A, int NV>
 __device__ __forceinline__ void dots_fused_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const void* w,
                                                 bool want_wn, int mmax, double* partial, int bx) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, false>();
-    A acc[NV];
+    A acc[NV + 1];   // the dots, then ||w||^2
 #pragma unroll
-    for (int t = 0; t < NV; ++t) acc[t] = zero<A>();
-    A wn = zero<A>();
+    for (int t = 0; t <= NV; ++t) acc[t] = zero<A>();
     for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
         A v[NV];
 #pragma unroll
@@ -451,30 +519,9 @@ __device__ __forceinline__ void dots_fused_rows(const SlotDev& S, int64_t r0, in
 #pragma unroll
         for (int t = 0; t < NV; ++t)
             if (t < nv) mac(acc[t], v[t], wr);
-        if (want_wn) mac(wn, wr, wr);
+        if (want_wn) mac(acc[NV], wr, wr);
     }
-    const int P = mmax + 1;
-    double* row = partial + (size_t)bx * P * 2;
-#pragma unroll
-    for (int c0 = 0; c0 < NV; c0 += jt<A>()) {
-        if (c0 < nv) {
-            A re[jt<A>()], im[jt<A>()];
-#pragma unroll
-            for (int q = 0; q < jt<A>(); ++q) {
-                re[q] = c0 + q < NV ? acc[c0 + q < NV ? c0 + q : 0] : zero<A>();
-                im[q] = zero<A>();
-            }
-            dots_epilogue<A>(re, im, false, c0, nv, c0, row);
-        }
-    }
-    if (want_wn) {
-        __shared__ double sw[kT / 32];
-        const double t = block_sum(wn, sw);
-        if (threadIdx.x == 0) {
-            partial[((size_t)bx * P + mmax) * 2] = t;
-            partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
-        }
-    }
+    fused_epilogue<A, NV>(acc, nv, want_wn, mmax, partial + (size_t)bx * (mmax + 1) * 2);
 }
 
 template <class A>
@@ -719,7 +766,7 @@ __global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3) eng_up
 // the second-pass dots acc[t] += V[r, t] w'[r] from the same registers (no
 // second read of V).  Per thread the rows, the terms and the argument order
 // of every multiply-add are those of update_rows followed by dots_rows, and
-// the block sums go through the same dots_epilogue, so the results are
+// the block sums add in the same order, so the results are
 // bit-identical to update_block's.
 __device__ __forceinline__ double ld_volatile(const volatile double* p) { return *p; }
 __device__ __forceinline__ float ld_volatile(const volatile float* p) { return *p; }
@@ -731,10 +778,9 @@ __device__ __forceinline__ void update_fused_rows(const SlotDev& S, int64_t r0, 
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, false>();
     void* w = (void*)(V + (size_t)(S.j + 1) * cs);
-    A acc[NV];
+    A acc[NV + 1];   // the second-pass dots, then ||w'||^2
 #pragma unroll
-    for (int t = 0; t < NV; ++t) acc[t] = zero<A>();
-    A nacc = zero<A>();
+    for (int t = 0; t <= NV; ++t) acc[t] = zero<A>();
     for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
         A v[NV];
 #pragma unroll
@@ -750,31 +796,12 @@ __device__ __forceinline__ void update_fused_rows(const SlotDev& S, int64_t r0, 
         A o = ldv<A, false>(w, r).re;
         o = sub(o, ar);
         stv<A, false>(w, r, CA<A>{o, zero<A>()});
-        mac(nacc, o, o);
+        mac(acc[NV], o, o);
 #pragma unroll
         for (int t = 0; t < NV; ++t)
             if (t < nv) mac(acc[t], v[t], o);
     }
-    __shared__ double sh[kT / 32];
-    const double tn = block_sum(nacc, sh);
-    const int P = mmax + 1;
-    if (threadIdx.x == 0) {
-        partial[((size_t)bx * P + mmax) * 2] = tn;
-        partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
-    }
-    double* row = partial + (size_t)bx * P * 2;
-#pragma unroll
-    for (int c0 = 0; c0 < NV; c0 += jt<A>()) {
-        if (c0 < nv) {
-            A re[jt<A>()], im[jt<A>()];
-#pragma unroll
-            for (int q = 0; q < jt<A>(); ++q) {
-                re[q] = c0 + q < NV ? acc[c0 + q < NV ? c0 + q : 0] : zero<A>();
-                im[q] = zero<A>();
-            }
-            dots_epilogue<A>(re, im, false, c0, nv, c0, row);
-        }
-    }
+    fused_epilogue<A, NV>(acc, nv, true, mmax, partial + (size_t)bx * (mmax + 1) * 2);
 }
 
 template <class A>
@@ -1173,19 +1200,31 @@ VKind store_kind(Store st, bool cv) {
     return cv ? VKind::C128 : VKind::F64;
 }
 
-// ------------------------------------------------------------ autotuner
-struct TuneKey {
-    int st;
-    bool cv, cm;
-    int size_class;
-    bool operator<(const TuneKey& o) const {
-        return std::tie(st, cv, cm, size_class) < std::tie(o.st, o.cv, o.cm, o.size_class);
-    }
-};
-std::mutex g_tune_mu;
-std::map<TuneKey, Tiles> g_tuned;
+// ------------------------------------------------------------ tiles
+// Rows per BLAS block and slices per SpMV block, by the slot's rows alone: a
+// slot's reductions add in the order of its row blocks, so its result is the
+// same alone and in any batch, and repeats from run to run.
+// rpb: the fused dots and update hold two blocks per SM (128 registers a
+// thread), so the row blocks are whole waves of 304 equal blocks, of at most
+// 8,192 rows (the double-float solve of 4.7 M rows: 88 ms with two waves, 94
+// with one) and at least 768 (below that a block's epilogue outweighs its
+// rows: 12 complex slots of 112,000 rows solve in 177 ms at 384 rows a block,
+// 154 at 1,024).  Ground state of 358,584 rows, FP64: 12.1 ms with 304 blocks,
+// 14.1 with 351, 16.0 with 88 (4,096 rows a block).
+// spb: one slice per warp spreads a slot of 90,000 rows over 352 blocks (5.9
+// ms a solve; 16 slices 6.3, 64 slices 8.7); from 20,000 slices on there are
+// blocks enough and two slices per warp save the value table's staging
+// (4.7 M rows: 128.8 against 130.4 ms).
+constexpr int kWaveBlocks = 304;
 
-int size_class(int64_t n) { return (int)std::floor(2.0 * std::log2((double)std::max<int64_t>(n, 1))); }
+Tiles tiles_for(int64_t n, int64_t nslices) {
+    Tiles t;
+    const int64_t waves = (n + (int64_t)kWaveBlocks * 8192 - 1) / ((int64_t)kWaveBlocks * 8192);
+    const int64_t blocks = kWaveBlocks * std::max<int64_t>(1, waves);
+    t.rpb = (int)std::max<int64_t>(768, ((n + blocks - 1) / blocks + 63) / 64 * 64);
+    t.spb = nslices < 20000 ? 8 : 16;
+    return t;
+}
 
 }  // namespace
 
@@ -1222,62 +1261,13 @@ Engine::~Engine() {
     if (graph_) cudaGraphDestroy(graph_);
 }
 
-Tiles Engine::tune(Op& op, int m, bool cv) {
-    const TuneKey key{(int)st_, cv, op.complex_mat, size_class(op.basis->n)};
-    {
-        std::lock_guard<std::mutex> g(g_tune_mu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) return it->second;
-    }
-    // time a few steps of this operator alone for every candidate tile pair
-    const int mt = std::min(m, 12);
-    Engine E(st_, s_);
-    int id = E.add(op, mt, cv, false);
-    E.seed(id, 1);
-    E.normalize({id});
-    cudaEvent_t e0, e1;
-    QS_CUDA(cudaEventCreate(&e0));
-    QS_CUDA(cudaEventCreate(&e1));
-    Tiles best;
-    float best_ms = 1e30f;
-    // only the SpMV's slices per block are timed: a row's product does not
-    // depend on them, while the BLAS row block fixes the order of every
-    // reduction and stays at its default (results repeat from run to run)
-    const int rpb = best.rpb;
-    for (int spb : {16, 64, 256}) {
-        E.slots_[id].d.rpb = rpb;
-        E.slots_[id].d.spb = spb;
-        E.maps_dirty_ = true;
-        E.start(id, 0);
-        E.run(2);  // captures the graph, warms up
-        E.start(id, 2);
-        QS_CUDA(cudaEventRecord(e0, s_));
-        E.run(std::min(6, mt - 2));
-        QS_CUDA(cudaEventRecord(e1, s_));
-        QS_CUDA(cudaEventSynchronize(e1));
-        float ms = 0;
-        QS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best_ms) {
-            best_ms = ms;
-            best.rpb = rpb;
-            best.spb = spb;
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    launches_ += E.launches();
-    std::lock_guard<std::mutex> g(g_tune_mu);
-    g_tuned[key] = best;
-    return best;
-}
-
 size_t Engine::slot_bytes(int64_t n, int m, bool cv, int tmp_cols, Store st) {
     const size_t es = store_bytes(st, cv);
     const int tc = tmp_cols > 0 ? tmp_cols : m - 1;
     return (size_t)(m + 1 + tc) * n * es + ((size_t)2 * m + (size_t)(m + 1) * m + (size_t)m * m) * 16 + 128;
 }
 
-int Engine::add(Op& op, int m, bool cv, bool tune_tiles, int tmp_cols, int orth) {
+int Engine::add(Op& op, int m, bool cv, int tmp_cols, int orth) {
     if (orth < 0 || orth > 2 || (orth == 2 && !op.hermitian))
         throw Error(QS_ERR_ARGUMENT, "the three-term recurrence needs a Hermitian operator");
     if (m < 2 || m > kMaxM) throw Error(QS_ERR_ARGUMENT, "Krylov basis size must lie in 2:256");
@@ -1333,9 +1323,7 @@ int Engine::add(Op& op, int m, bool cv, bool tune_tiles, int tmp_cols, int orth)
     d.carry = -1;
     d.orth = orth;
     sl.tcols = tc;
-    Tiles t;
-    // (a slot on the cluster step splits its slices by CTA, not by the tile)
-    if (tune_tiles && n >= 4096 && m >= 4 && cluster_size_for(d) == 0) t = tune(op, m, cv);
+    const Tiles t = tiles_for(n, M.nslices);
     d.rpb = t.rpb;
     d.spb = t.spb;
     sl.live = true;
@@ -2716,7 +2704,7 @@ void evolve_engine(Op& op, const double* v0, const std::vector<cd>& scales, doub
     auto copy_v0 = [&](int i) { std::copy(v0, v0 + 2 * n, out + (size_t)i * 2 * n); };
     Engine E(precision == 0 ? Store::F64 : Store::DF, op.stream);
     // one factorisation from v0 serves every time whose estimate passes
-    const int f = E.add(op, m, true, true, 1, orth);
+    const int f = E.add(op, m, true, 1, orth);
     E.load(f, 0, v0, false);
     const double beta = E.normalize({f})[0];
     bool all_zero = true;
@@ -2767,7 +2755,7 @@ void evolve_engine(Op& op, const double* v0, const std::vector<cd>& scales, doub
             std::vector<double*> outs;
             for (size_t q = w0; q < w1; ++q) {
                 const int i = failing[q];
-                const int id = E.add(op, m, true, true, 1, orth);
+                const int id = E.add(op, m, true, 1, orth);
                 E.load(id, 0, v0, false);
                 ids.push_back(id);
                 outs.push_back(out + (size_t)i * 2 * n);
@@ -2824,7 +2812,7 @@ void evolve_stepwise(Op& op, const double* v0, const std::vector<double>& offset
     for (int i : order) {
         const double d = offsets[i] - prev;
         if (d != 0.0) {
-            const int id = E.add(op, m, true, true, 1, herm ? 2 : 0);
+            const int id = E.add(op, m, true, 1, herm ? 2 : 0);
             E.load(id, 0, cur.as<double>(), true);
             const double beta = E.normalize({id})[0];
             if (beta > 0) {
@@ -2872,7 +2860,7 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
         n[b] = ops[b]->basis->n;
         m[b] = (int)std::max<int64_t>(2, std::min<int64_t>(std::min(krylov_dim, kMaxM), n[b]));
         herm[b] = ops[b]->hermitian;
-        f[b] = E.add(*ops[b], m[b], true, true, 1, herm[b] ? 2 : 0);
+        f[b] = E.add(*ops[b], m[b], true, 1, herm[b] ? 2 : 0);
         E.load(f[b], 0, v0s[b], true);
         fid.push_back(f[b]);
     }
@@ -2964,7 +2952,7 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
             const size_t per = Engine::slot_bytes(n[b], m[b], true, 1, E.store());
             if (w1 > w0 && used + per > fr / 2) break;
             used += per;
-            const int id = E.add(*ops[b], m[b], true, true, 1, herm[b] ? 2 : 0);
+            const int id = E.add(*ops[b], m[b], true, 1, herm[b] ? 2 : 0);
             E.load(id, 0, v0s[b], true);
             ids.push_back(id);
             wouts.push_back(outs[b] + (size_t)failing[w1].second * 2 * n[b]);

@@ -15,10 +15,9 @@
 // Vectors are stored either in FP64 or as double-float pairs (hi + lo float,
 // arithmetic on the FP32 pipe); both take 8 bytes per real component.  Each
 // slot has its own real/complex vector flag, so a slot's arithmetic does not
-// depend on which other slots share the launches.  The SpMV's slices per
-// block are per slot, chosen by a timing autotuner and cached per (storage,
-// flags, size class); the BLAS row block is fixed, so every reduction, and
-// with it every result, repeats from run to run.
+// depend on which other slots share the launches.  The tiles (SpMV
+// slices and BLAS rows per block) follow from a slot's rows alone, so every
+// reduction, and with it every result, repeats from run to run.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -89,11 +88,9 @@ struct SlotDev {
 // Storage of a slot's Krylov vectors (and the arithmetic of the step kernels).
 enum class Store : int32_t { F64 = 0, DF = 1, F32 = 2 };
 
-// rpb: rows per BLAS block (4096 measured best or within 3 % on single and
-// batched solves; fixed so that reductions repeat); spb: SELL slices per SpMV
-// block (timed per operator size class)
+// rpb: rows per BLAS block; spb: SELL slices per SpMV block (tiles_for)
 struct Tiles {
-    int rpb = 4096, spb = 64;
+    int rpb = 768, spb = 8;
 };
 
 // One slot's part of a rotate() call.
@@ -115,7 +112,7 @@ class Engine {
     // Adds a slot of basis size m on an assembled operator (assembled here if
     // needed).  cv: complex vectors (required for complex operators); tmp_cols:
     // most rotation outputs (m - 1 when 0).
-    int add(Op& op, int m, bool cv, bool tune = true, int tmp_cols = 0, int orth = 1);
+    int add(Op& op, int m, bool cv, int tmp_cols = 0, int orth = 1);
     // device bytes add() would allocate for a slot
     static size_t slot_bytes(int64_t n, int m, bool cv, int tmp_cols = 0, Store st = Store::F64);
     void remove(int id);
@@ -173,7 +170,6 @@ class Engine {
     int cluster_size_for(const SlotDev& d) const;   // 0: not in the cluster step
     bool cluster16_ok() const;
     void run_cluster(const std::vector<int>& ids, int nsteps, int C, cudaStream_t st);
-    Tiles tune(Op& op, int m, bool cv);
     Store st_;
     cudaStream_t s_;
     std::vector<Slot> slots_;
@@ -199,7 +195,6 @@ class Engine {
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     int64_t launches_ = 0;
-    friend struct EngineTuner;
 };
 
 // Runs `blocks` cooperative blocks through eight grid barriers (the persistent

@@ -453,7 +453,7 @@ void engine_loop(Server& S) {
                 // recurrence (three-term for Hermitian operators, else CGS2)
                 const int orth = q->r.kind == QS_REQ_EIGSH ? 1 : (q->op->op->hermitian ? 2 : 0);
                 q->lane = ln.id;
-                q->slot = E.add(*q->op->op, q->m, q->cv, true, q->r.kind == QS_REQ_EIGSH ? 0 : 1, orth);
+                q->slot = E.add(*q->op->op, q->m, q->cv, q->r.kind == QS_REQ_EIGSH ? 0 : 1, orth);
                 const int comps = q->cv ? 2 : 1;
                 if (!dev_v0.empty() && dev_v0[r]) {
                     E.load(q->slot, 0, dev_v0[r], true);

@@ -225,7 +225,7 @@ std::unique_ptr<LanczosSet> lanczos_run(Op& op, const qs_lanczos_opts& o, int ns
     }
     for (int s = 0; s < nstart; ++s) {
         // three-term recurrence as the reference; full_ortho: CGS2 against every kept vector
-        const int id = E.add(op, mm, L->cv, true, 1, o.full_ortho ? 0 : 2);
+        const int id = E.add(op, mm, L->cv, 1, o.full_ortho ? 0 : 2);
         E.load(id, 0, src + (size_t)s * n * comps, true);
         L->ids.push_back(id);
     }
