@@ -560,6 +560,18 @@ void detect_fast_group(Basis& b, const Closure& C, int kmom, int nT) {
     b.fast.allowed = allowed;
 }
 
+// sqrt(i) and 1/sqrt(i) of every stabiliser order, correctly rounded (a square
+// root or a division per row would cost more FP64 work than the row's sum)
+void build_sqrt_table(Basis& b) {
+    std::vector<double> t(2 * (kMaxGroup + 1), 0.0);
+    for (int i = 1; i <= kMaxGroup; ++i) {
+        t[i] = std::sqrt((double)i);
+        t[kMaxGroup + 1 + i] = 1.0 / std::sqrt((double)i);
+    }
+    b.d_sqrt.alloc(t.size() * sizeof(double));
+    QS_CUDA(cudaMemcpy(b.d_sqrt.p, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+}
+
 }  // namespace
 
 // ----------------------------------------------------------- basis_build
@@ -692,6 +704,7 @@ void basis_build(Basis& b) {
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
     b.d_binom.alloc(binom.size() * sizeof(uint64_t));
     QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    if (b.symmetric) build_sqrt_table(b);
     b.d_group.alloc(sizeof(GroupDesc));
     QS_CUDA(cudaMemcpy(b.d_group.p, &b.group, sizeof(GroupDesc), cudaMemcpyHostToDevice));
     detect_fast_group(b, C, kmom, nT);
@@ -869,6 +882,7 @@ void basis_build_general(Basis& b, const qs_general_spec& gs) {
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
     b.d_binom.alloc(binom.size() * sizeof(uint64_t));
     QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    if (b.symmetric) build_sqrt_table(b);
     b.d_gtab.alloc(std::max<size_t>(1, tables.size()) * sizeof(uint64_t));
     if (!tables.empty())
         QS_CUDA(cudaMemcpy(b.d_gtab.p, tables.data(), tables.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));

@@ -151,6 +151,7 @@ struct Basis {
     std::vector<cplx> fast_chi;      // character per fast element code
     std::vector<int> fast_to_elem;   // generic element index per fast element code
     DevBuf d_fast_chi;               // complex double, 4 * nT
+    DevBuf d_sqrt;                   // sqrt(i), then 1/sqrt(i), i = 0 .. kMaxGroup (symmetric bases)
     bool has_index = false;          // direct rank -> column table built
     std::vector<uint64_t> h_refrep;  // reference (argmax) representatives
     bool refrep_ready = false;
