@@ -558,6 +558,44 @@ void detect_fast_group(Basis& b, const Closure& C, int kmom, int nT) {
     for (int p = 0; p < L; ++p)
         if (((L - 1 - p) % a) == 0) allowed |= 1ull << p;
     b.fast.allowed = allowed;
+    if (L <= 32 && nt == 1) b.fast.win = 2;
+    else if (L <= 32 && a == 1) b.fast.win = 1;
+    for (int r = 0; r <= has_refl; ++r)
+        for (int f = 0; f <= has_flip; ++f)
+            for (int j = 1; j < nt; ++j) {
+                const cplx c0 = b.fast_chi[(r * 2 + f) * nt], cj = b.fast_chi[(r * 2 + f) * nt + j];
+                if (cj.re != c0.re || cj.im != c0.im) b.fast.need_j = 1;
+            }
+    for (int q = 2, rest = L; rest > 1; ++q) {
+        if (rest % q) continue;
+        while (rest % q == 0) rest /= q;
+        if (b.fast.nper < 3) b.fast.per[b.fast.nper++] = L / q;   // L <= 63 has at most three primes
+    }
+}
+
+// The split rank tables of a fixed-weight parent sector of at most 32 sites.
+void build_rank_split(Basis& b, const std::vector<uint64_t>& binom) {
+    if (b.nup < 0 || b.L > 32) return;
+    RankSplit& R = b.rank;
+    const int L = b.L;
+    R.w = (L + 3) / 4;
+    std::vector<uint32_t> tab;
+    for (int k = 0; k < 4; ++k) {
+        const int below = std::min(k * R.w, L);
+        const int p0 = std::max(0, b.nup - (L - below)), p1 = std::min(below, b.nup);
+        R.off[k] = (int)tab.size() - (p0 << R.w);
+        for (int p = p0; p <= p1; ++p)
+            for (uint32_t q = 0; q < (1u << R.w); ++q) {
+                uint64_t r = 0;
+                int particle = p;
+                for (int i = 0; i < R.w; ++i)
+                    if ((q >> i) & 1u) r += binom[(size_t)(k * R.w + i) * 65 + ++particle];
+                tab.push_back((uint32_t)r);
+            }
+    }
+    R.size = (int)tab.size();
+    b.d_rank.alloc(tab.size() * sizeof(uint32_t));
+    QS_CUDA(cudaMemcpy(b.d_rank.p, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
 }
 
 // sqrt(i) and 1/sqrt(i) of every stabiliser order, correctly rounded (a square
@@ -704,6 +742,7 @@ void basis_build(Basis& b) {
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
     b.d_binom.alloc(binom.size() * sizeof(uint64_t));
     QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    build_rank_split(b, binom);
     if (b.symmetric) build_sqrt_table(b);
     b.d_group.alloc(sizeof(GroupDesc));
     QS_CUDA(cudaMemcpy(b.d_group.p, &b.group, sizeof(GroupDesc), cudaMemcpyHostToDevice));
@@ -882,6 +921,7 @@ void basis_build_general(Basis& b, const qs_general_spec& gs) {
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
     b.d_binom.alloc(binom.size() * sizeof(uint64_t));
     QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
+    build_rank_split(b, binom);
     if (b.symmetric) build_sqrt_table(b);
     b.d_gtab.alloc(std::max<size_t>(1, tables.size()) * sizeof(uint64_t));
     if (!tables.empty())

@@ -67,6 +67,26 @@ struct TermProg {
     uint64_t need0, need1, flip, zmask, ymask;
 };
 
+// The same program as the row kernels read it (qs_rows.cuh): alive iff
+// (s & care) == value, image s ^ flip, sign (-1)^popc(s & zy) times its class's
+// amplitude (the constant part of the sign is in the class).  Programs that
+// touch a site twice (chars) pass the test on every state and are run by their
+// characters.
+struct RowProg {
+    uint64_t care, value, flip, zy;
+    uint32_t cls, chars;
+};
+constexpr uint32_t kCharsClass = 0xffffffffu;   // class of a program run by its characters
+
+// Combinadic ranks of fixed-weight states of at most 32 sites as four table
+// reads: piece k covers bits k w .. k w + w - 1; its entry for p particles below
+// and bit pattern q is tab[off[k] + (p << w) + q] (off may be negative: rows
+// start at the least p that a state of weight nup can have there).
+struct RankSplit {
+    int32_t w, size;
+    int32_t off[4];
+};
+
 // ---------------------------------------------------------------- bit ops
 QS_HD uint64_t low_mask(int L) { return L >= 64 ? ~0ull : ((1ull << L) - 1ull); }
 

@@ -151,6 +151,8 @@ struct Basis {
     std::vector<cplx> fast_chi;      // character per fast element code
     std::vector<int> fast_to_elem;   // generic element index per fast element code
     DevBuf d_fast_chi;               // complex double, 4 * nT
+    RankSplit rank{};                // split rank tables (fixed weight, L <= 32)
+    DevBuf d_rank;                   // uint32, rank.size entries
     DevBuf d_sqrt;                   // sqrt(i), then 1/sqrt(i), i = 0 .. kMaxGroup (symmetric bases)
     bool has_index = false;          // direct rank -> column table built
     std::vector<uint64_t> h_refrep;  // reference (argmax) representatives
@@ -201,6 +203,12 @@ struct Op {
     std::vector<TermProg> diag_progs;
     std::vector<std::complex<double>> user_diag;
     DevBuf d_progs;
+    // the programs as the row kernels read them, the amplitude of every class
+    // (complex double), and whether a sign depends on the state / a program
+    // changes the particle number / runs by its characters
+    DevBuf d_rowprogs, d_amp;
+    int nclass = 0;
+    bool any_zy = false, check_weight = false, any_chars = false, real_amp = true;
     DevBuf d_diag;                  // complex diagonal (user + extracted), 2*n doubles
     DevBuf d_diag32;                // single-precision copy
     DevBuf d_diag_re, d_diag32_re;  // real parts (read by real operators)

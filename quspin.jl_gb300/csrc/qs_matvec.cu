@@ -15,6 +15,12 @@
 // group.  No scatter, no atomics: every row is written once, and the summation
 // order per row is fixed, so repeated calls are bit-identical.
 //
+// The transitions of a row (which programs are alive, orbit minimum, rank) are
+// walked by qs_rows.cuh, shared with the assembly.  Bound: integer issue in the
+// orbit search; FP64 is one multiply-add per transition (amplitude times
+// character from a table, the rare sqrt(stab) != 1 and the row's 1/sqrt(stab)
+// apart), which GB300's FP64 pipe takes 16 cycles a warp for.
+//
 // Rank lookups: full 2^L space -> the state itself; fixed-weight sector
 // without spatial symmetry -> combinadic rank (src/discrete_basis.jl:1879-1906);
 // symmetric sector -> search of the sorted representatives with a
@@ -26,18 +32,21 @@
 
 #include <algorithm>
 #include <atomic>
+#include <map>
+#include <vector>
 
 #include "qs_device.cuh"
 #include "qs_df.cuh"
 #include "qs_internal.h"
+#include "qs_rows.cuh"
 
 namespace qs {
 
 namespace {
 
-constexpr int kMvThreads = 256;
+constexpr int kMvThreads = kRowThreads;
 constexpr int kMaxSplit = 2048;
-constexpr int kSmemProgs = 160;
+constexpr int kMvTable = 1024;   // (class, element) values staged in shared memory, at most
 
 template <typename T> struct V2;
 template <> struct V2<double> { using t = double2; };
@@ -53,10 +62,17 @@ struct MvArgs {
     int L, nup, pauli;
     const TermProg* progs;
     int nprog;
-    const int32_t* index;    // direct rank -> column table (mode 3)
-    FastGroup fast;          // zero-run orbit search when enabled
-    const double* fast_chi;  // complex character per fast element code
+    RowArgs row;             // the transitions (matvec_kernel, matvec_warp_rank_kernel)
+    const double* chi_re;    // character of element code e at [e * chi_stride]
+    const double* chi_im;
+    int chi_stride, nelem;   // nelem 1: every character is 1
+    const double2* amp;      // amplitude per program class
+    int nclass;
+    int table;               // amplitude x character staged per (class, element)
+    int any_chars;
+    const double* sq;        // sqrt(i), then 1/sqrt(i), i = 0 .. kMaxGroup
     const void* diag;        // complex, precision of the call
+    const void* diag_re;     // its real part (real operators)
     int conj_amp, conj_chi;
     double ar, ai, br, bi;
     int beta_zero;
@@ -163,32 +179,6 @@ __device__ __forceinline__ uint32_t unrank32(int64_t r, const uint32_t* binom32,
     return s;
 }
 
-// rank(t) from rank(s) = rs for fixed-weight states of equal weight that
-// differ only in bits lo .. hi: the set bits below lo and above hi keep their
-// particle numbers, so only the set bits inside the span change their terms
-// C(bit, particle).  A short span (a bond, a plaquette) costs a few table
-// reads instead of the nup of a full rank; a long one (the periodic bond of a
-// chain) takes the full rank of t.
-__device__ __forceinline__ int64_t rank_from32(uint32_t s, int64_t rs, uint32_t t, const uint32_t* binom32) {
-    const uint32_t f = s ^ t;
-    if (!f) return rs;
-    const int lo = __ffs((int)f) - 1, hi = 31 - __clz((int)f);
-    if (hi - lo > 8) return combinadic_rank32(t, binom32);
-    const uint32_t span = (hi == 31 ? 0xffffffffu : ((1u << (hi + 1)) - 1u)) & ~((1u << lo) - 1u);
-    const int m0 = __popc(s & ((1u << lo) - 1u));
-    int64_t d = 0;
-    uint32_t bs = s & span, bt = t & span;
-    for (int p = m0 + 1; bs; ++p) {
-        d -= binom32[(__ffs((int)bs) - 1) * 33 + p];
-        bs &= bs - 1;
-    }
-    for (int p = m0 + 1; bt; ++p) {
-        d += binom32[(__ffs((int)bt) - 1) * 33 + p];
-        bt &= bt - 1;
-    }
-    return rs + d;
-}
-
 template <typename T, bool kCV>
 __device__ __forceinline__ void load_x(const MvArgs& a, int64_t i, T& xr, T& xi) {
     if (kCV) {
@@ -201,126 +191,209 @@ __device__ __forceinline__ void load_x(const MvArgs& a, int64_t i, T& xr, T& xi)
     }
 }
 
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// (wr, wi) times the character of element code ec
+template <bool kCM, typename T>
+__device__ __forceinline__ void times_chi(const MvArgs& a, int ec, T& wr, T& wi) {
+    if (a.nelem == 1) return;
+    const T cr = (T)__ldg(a.chi_re + (size_t)ec * a.chi_stride);
+    if (kCM) {
+        T ci = (T)__ldg(a.chi_im + (size_t)ec * a.chi_stride);
+        if (a.conj_chi) ci = -ci;
+        const T nr = fma_r(-wi, ci, mul_rn(wr, cr)), ni = fma_r(wi, cr, mul_rn(wr, ci));
+        wr = nr;
+        wi = ni;
+    } else {
+        wr = mul_rn(wr, cr);
+    }
+}
+
+// amplitude of a program class, conjugated with the operator
+template <typename T>
+__device__ __forceinline__ void class_amp(const MvArgs& a, uint32_t cls, T& wr, T& wi) {
+    const double2 v = __ldg(a.amp + cls);
+    wr = (T)v.x;
+    wi = a.conj_amp ? -(T)v.y : (T)v.y;
+}
+
+// amplitude x character of every (class, element) pair, when they are few
+template <bool kCM, typename T>
+__device__ __forceinline__ void stage_values(const MvArgs& a, void* tab) {
+    if (!a.table) return;
+    for (int i = threadIdx.x; i < a.nclass * a.nelem; i += blockDim.x) {
+        T wr, wi;
+        class_amp<T>(a, i / a.nelem, wr, wi);
+        times_chi<kCM, T>(a, i % a.nelem, wr, wi);
+        if (kCM) {
+            typename V2<T>::t v;
+            v.x = wr;
+            v.y = wi;
+            ((typename V2<T>::t*)tab)[i] = v;
+        } else {
+            ((T*)tab)[i] = wr;
+        }
+    }
+}
+
+// Program k on s by its characters (a site acted on twice): false when it
+// annihilates the state.
+template <typename U>
+__device__ __noinline__ bool run_chars(const MvArgs& a, int k, U s, U& t, double& wr, double& wi) {
+    if (!run_prog<U, double>(a.progs[k], a.pauli, s, t, wr, wi)) return false;
+    if (a.conj_amp) wi = -wi;
+    return true;
+}
+
+// acc += w x with the character, sqrt(stab) of the column and the sign of a
+// transition of class cls (a program run by its characters brings its own w)
+template <bool kCM, bool kCV, typename T>
+__device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab, uint32_t cls, int ec, int st, int sign,
+                                               T wr, T wi, int64_t idx, T& acc_r, T& acc_i) {
+    if (cls == kCharsClass) {
+        times_chi<kCM, T>(a, ec, wr, wi);
+    } else if (a.table) {
+        const int i = (int)cls * a.nelem + (a.nelem == 1 ? 0 : ec);
+        if (kCM) {
+            const typename V2<T>::t v = ((const typename V2<T>::t*)tab)[i];
+            wr = v.x;
+            wi = v.y;
+        } else {
+            wr = ((const T*)tab)[i];
+        }
+    } else {
+        class_amp<T>(a, cls, wr, wi);
+        times_chi<kCM, T>(a, ec, wr, wi);
+    }
+    if (sign) {
+        wr = -wr;
+        wi = -wi;
+    }
+    if (st != 1) {
+        const T f = (T)__ldg(a.sq + st);
+        wr = mul_rn(wr, f);
+        if (kCM) wi = mul_rn(wi, f);
+    }
+    T xr, xi;
+    load_x<T, kCV>(a, idx, xr, xi);
+    acc_r = fma_r(wr, xr, acc_r);
+    if (kCM) {
+        acc_r = fma_r(-wi, xi, acc_r);
+        acc_i = fma_r(wr, xi, acc_i);
+        acc_i = fma_r(wi, xr, acc_i);
+    } else if (kCV) {
+        acc_i = fma_r(wr, xi, acc_i);
+    }
+}
+
+// y[r] = beta y[r] + alpha (d[r] x[r] + acc / sqrt(stab_r))
+template <bool kSym, bool kCM, bool kCV, typename T>
+__device__ __forceinline__ void store_row(const MvArgs& a, int64_t r, T acc_r, T acc_i) {
+    if (kSym) {
+        const int st = a.stab[r];
+        if (st != 1) {
+            const T f = (T)__ldg(a.sq + kMaxGroup + 1 + st);
+            acc_r *= f;
+            acc_i *= f;
+        }
+    }
+    // diagonal (user + extracted), conjugated with the operator
+    T xr, xi;
+    load_x<T, kCV>(a, r, xr, xi);
+    if (kCM) {
+        const typename V2<T>::t d = ((const typename V2<T>::t*)a.diag)[r];
+        const T dr = d.x, di = a.conj_amp ? -d.y : d.y;
+        acc_r += dr * xr - di * xi;
+        acc_i += dr * xi + di * xr;
+    } else {
+        const T dr = ((const T*)a.diag_re)[r];
+        acc_r += dr * xr;
+        if (kCV) acc_i += dr * xi;
+    }
+    if (kCV) {
+        typename V2<T>::t* y = (typename V2<T>::t*)a.y;
+        T yr = 0, yi = 0;
+        if (!a.beta_zero) {
+            const typename V2<T>::t yo = y[r];
+            yr = (T)a.br * yo.x - (T)a.bi * yo.y;
+            yi = (T)a.br * yo.y + (T)a.bi * yo.x;
+        }
+        typename V2<T>::t out;
+        out.x = yr + (T)a.ar * acc_r - (T)a.ai * acc_i;
+        out.y = yi + (T)a.ar * acc_i + (T)a.ai * acc_r;
+        y[r] = out;
+    } else {
+        T* y = (T*)a.y;
+        const T yr = a.beta_zero ? (T)0 : (T)a.br * y[r];
+        y[r] = yr + (T)a.ar * acc_r;
+    }
+}
+
+// dynamic shared memory: the staged values, then the split rank tables
+QS_HD size_t mv_table_bytes(int entries, bool cm, size_t real) {
+    return ((size_t)entries * real * (cm ? 2 : 1) + 15) / 16 * 16;
+}
+
 template <typename U, int kMode, bool kCM, bool kCV, typename T>
 __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
     constexpr bool kSym = kMode >= 2;
+    constexpr bool k32 = sizeof(U) == 4;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ RowSmem<U> sm;
     __shared__ GroupSmem g;
     __shared__ U spl[kMode == 2 ? kMaxSplit : 1];
-    constexpr bool kB32 = (kMode == 3 || kMode == 1) && sizeof(U) == 4;
-    __shared__ uint32_t binom32[kB32 ? 32 * 33 : 1];
-    __shared__ TermProg progs[kSmemProgs];
-    __shared__ double sqrt_stab[kMaxGroup + 1];
-    if (kSym) {
-        load_group_smem(g, a.group);
-        if (kMode == 2)
-            for (int i = threadIdx.x; i < a.nsplit; i += blockDim.x) spl[i] = ((const U*)a.split)[i];
-        for (int i = threadIdx.x; i <= kMaxGroup; i += blockDim.x) sqrt_stab[i] = sqrt((double)i);
-    }
+    __shared__ uint32_t binom32[kMode == 1 && k32 ? 32 * 33 : 1];
+    const RowArgs& R = a.row;
+    uint32_t* rtab = (uint32_t*)(dyn + (a.table ? mv_table_bytes(a.nclass * a.nelem, kCM, sizeof(T)) : 0));
+    if (kSym && !R.fast.enabled) load_group_smem(g, R.group);
+    if (kMode == 2)
+        for (int i = threadIdx.x; i < R.nsplit; i += blockDim.x) spl[i] = ((const U*)R.split)[i];
+    if (k32 && (kMode == 1 || kMode == 3))
+        for (int i = threadIdx.x; i < R.rank.size; i += blockDim.x) rtab[i] = R.rank_tab[i];
     // C(bit, p) for bit < 32, p <= 32: all below 2^32
-    if (kB32 && a.nup >= 0)
+    if (kMode == 1 && k32)
         for (int i = threadIdx.x; i < 32 * 33; i += blockDim.x)
             binom32[i] = (uint32_t)a.binom[(i / 33) * 65 + (i % 33)];
-    const int np_smem = a.nprog < kSmemProgs ? a.nprog : kSmemProgs;
-    for (int i = threadIdx.x; i < np_smem; i += blockDim.x) progs[i] = a.progs[i];
+    stage_values<kCM, T>(a, dyn);
+    load_row_progs(sm, R, 0);
     __syncthreads();
-    const double* chi_re = a.group->chi_re;
-    const double* chi_im = a.group->chi_im;
 
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.n; r += (int64_t)gridDim.x * blockDim.x) {
-        const U s = (kB32 && kMode == 1) ? (U)unrank32(r, binom32, a.L, a.nup) : row_state<U>(a, kSym ? 2 : kMode, r);
-        T inv_sr = 1;
-        if (kSym) inv_sr = (T)1 / (T)sqrt_stab[a.stab[r]];
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < a.n; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = base + threadIdx.x;
+        const bool valid = r < a.n;
+        U s = 0;
+        if (valid) s = (k32 && kMode == 1) ? (U)unrank32(r, binom32, a.L, a.nup) : row_state<U>(a, kSym ? 2 : kMode, r);
         T acc_r = 0, acc_i = 0;
-        for (int k = 0; k < a.nprog; ++k) {
-            const TermProg& p = (k < kSmemProgs) ? progs[k] : a.progs[k];
-            U t;
-            T wr, wi;
-            if (!run_prog<U, T>(p, a.pauli, s, t, wr, wi)) continue;
-            int64_t idx;
-            if (a.conj_amp) wi = -wi;
-            if (kSym) {
-                U m;
-                int bi, st;
-                const double* chr = chi_re;
-                const double* chi = chi_im;
-                int cstride = 1;
-                if (a.fast.enabled) {
-                    orbit_min_fast<U>(a.fast, t, m, bi, st);
-                    chr = a.fast_chi;
-                    chi = a.fast_chi + 1;
-                    cstride = 2;
-                } else {
-                    orbit_min<U>(g, t, m, bi, st);
+        for (int c0 = 0; c0 < R.nprog; c0 += kRowChunk) {
+            if (R.nprog > kRowChunk) {
+                __syncthreads();
+                load_row_progs(sm, R, c0);
+                __syncthreads();
+            }
+            row_hops<U>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
+                const uint32_t cls = sm.cls[i];
+                T wr = 0, wi = 0;
+                if (a.any_chars && cls == kCharsClass) {
+                    U tc;
+                    double dr, di;
+                    if (!run_chars<U>(a, c0 + i, s, tc, dr, di)) return;
+                    t = tc;
+                    wr = (T)dr;
+                    wi = (T)di;
                 }
-                if (kMode == 3) {
-                    int64_t rk;
-                    if (a.nup < 0) rk = (int64_t)m;
-                    else if (sizeof(U) == 4) rk = combinadic_rank32((uint32_t)m, binom32);
-                    else rk = combinadic_rank<U>(m, a.binom, 65);
-                    idx = __ldg(a.index + rk);
-                } else {
-                    idx = rank_search<U>((const U*)a.reps, a.n, spl, (int)a.nsplit, a.stride, m);
-                }
-                if (idx < 0) continue;
-                const T f = (T)sqrt_stab[st] * inv_sr;
-                if (kCM) {
-                    T cr = (T)__ldg(chr + bi * cstride), ci = (T)__ldg(chi + bi * cstride);
-                    if (a.conj_chi) ci = -ci;
-                    T nr = wr * cr - wi * ci, ni = wr * ci + wi * cr;
-                    wr = nr * f;
-                    wi = ni * f;
-                } else {
-                    wr *= (T)__ldg(chr + bi * cstride) * f;
-                }
-            } else if (kMode == 1) {
-                if (__popcll((unsigned long long)t) != a.nup) continue;
-                if (kB32) idx = rank_from32((uint32_t)s, r, (uint32_t)t, binom32);
-                else idx = combinadic_rank<U>(t, a.binom, 65);
-            } else {
-                idx = (int64_t)t;
-            }
-            T xr, xi;
-            load_x<T, kCV>(a, idx, xr, xi);
-            if (kCM) {
-                acc_r += wr * xr - wi * xi;
-                acc_i += wr * xi + wi * xr;
-            } else if (kCV) {
-                acc_r += wr * xr;
-                acc_i += wr * xi;
-            } else {
-                acc_r += wr * xr;
-            }
+                if (kMode != 0 && R.check_weight && __popcll((unsigned long long)t) != a.nup) return;
+                U m = t;
+                int ec = 0, st = 1;
+                if (kSym) row_orbit<U>(R, g, t, m, ec, st);
+                const int64_t idx = row_column<U, kMode>(R, spl, rtab, m);
+                if (kSym && idx < 0) return;
+                add_transition<kCM, kCV, T>(a, dyn, cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
+            });
         }
-        // diagonal (user + extracted), conjugated with the operator
-        {
-            typename V2<T>::t d = ((const typename V2<T>::t*)a.diag)[r];
-            T dr = d.x, di = a.conj_amp ? -d.y : d.y;
-            T xr, xi;
-            load_x<T, kCV>(a, r, xr, xi);
-            if (kCV) {
-                acc_r += dr * xr - di * xi;
-                acc_i += dr * xi + di * xr;
-            } else {
-                acc_r += dr * xr;
-            }
-        }
-        if (kCV) {
-            typename V2<T>::t* y = (typename V2<T>::t*)a.y;
-            T yr = 0, yi = 0;
-            if (!a.beta_zero) {
-                typename V2<T>::t yo = y[r];
-                yr = (T)a.br * yo.x - (T)a.bi * yo.y;
-                yi = (T)a.br * yo.y + (T)a.bi * yo.x;
-            }
-            typename V2<T>::t out;
-            out.x = yr + (T)a.ar * acc_r - (T)a.ai * acc_i;
-            out.y = yi + (T)a.ar * acc_i + (T)a.ai * acc_r;
-            y[r] = out;
-        } else {
-            T* y = (T*)a.y;
-            T yr = a.beta_zero ? (T)0 : (T)a.br * y[r];
-            y[r] = yr + (T)a.ar * acc_r;
-        }
+        if (valid) store_row<kSym, kCM, kCV, T>(a, r, acc_r, acc_i);
     }
 }
 
@@ -378,101 +451,47 @@ __device__ __forceinline__ int64_t rank_warp(const U* __restrict__ reps, int64_t
 
 // The symmetric-sector product of matvec_kernel with the rank of every
 // generated state found by rank_warp (QS_RANK_MODE=warp): rows are taken a
-// warp at a time so that all 32 lanes reach every lookup together.
+// warp at a time and programs in step, so that all 32 lanes reach every lookup
+// together.
 template <typename U, bool kCM, bool kCV, typename T>
 __global__ void __launch_bounds__(kMvThreads) matvec_warp_rank_kernel(MvArgs a) {
+    extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ GroupSmem g;
     __shared__ U spl[kMaxSplit];
-    __shared__ TermProg progs[kSmemProgs];
-    __shared__ double sqrt_stab[kMaxGroup + 1];
-    load_group_smem(g, a.group);
-    for (int i = threadIdx.x; i < a.nsplit; i += blockDim.x) spl[i] = ((const U*)a.split)[i];
-    for (int i = threadIdx.x; i <= kMaxGroup; i += blockDim.x) sqrt_stab[i] = sqrt((double)i);
-    const int np_smem = a.nprog < kSmemProgs ? a.nprog : kSmemProgs;
-    for (int i = threadIdx.x; i < np_smem; i += blockDim.x) progs[i] = a.progs[i];
+    const RowArgs& R = a.row;
+    load_group_smem(g, R.group);
+    for (int i = threadIdx.x; i < R.nsplit; i += blockDim.x) spl[i] = ((const U*)R.split)[i];
+    stage_values<kCM, T>(a, dyn);
     __syncthreads();
-    const double* chi_re = a.group->chi_re;
-    const double* chi_im = a.group->chi_im;
     const int lane = threadIdx.x & 31;
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); base < a.n; base += nthreads) {
         const int64_t r = base + lane;
         const bool rv = r < a.n;
         const U s = rv ? ((const U*)a.reps)[r] : (U)0;
-        const T inv_sr = rv ? (T)1 / (T)sqrt_stab[a.stab[r]] : (T)0;
         T acc_r = 0, acc_i = 0;
-        for (int k = 0; k < a.nprog; ++k) {
-            const TermProg& p = (k < kSmemProgs) ? progs[k] : a.progs[k];
-            U t = 0, m = 0;
+        for (int k = 0; k < R.nprog; ++k) {
+            const RowProg p = R.progs[k];
+            U t = s ^ (U)p.flip, m = 0;
             T wr = 0, wi = 0;
-            int bi = 0, st = 0;
-            const bool alive = rv && run_prog<U, T>(p, a.pauli, s, t, wr, wi);
-            const double* chr = chi_re;
-            const double* chi = chi_im;
-            int cstride = 1;
-            if (alive) {
-                if (a.conj_amp) wi = -wi;
-                if (a.fast.enabled) {
-                    orbit_min_fast<U>(a.fast, t, m, bi, st);
-                    chr = a.fast_chi;
-                    chi = a.fast_chi + 1;
-                    cstride = 2;
-                } else {
-                    orbit_min<U>(g, t, m, bi, st);
-                }
+            int ec = 0, st = 1;
+            bool alive = rv && (s & (U)p.care) == (U)p.value;
+            if (alive && p.cls == kCharsClass) {
+                U tc;
+                double dr, di;
+                alive = run_chars<U>(a, k, s, tc, dr, di);
+                t = tc;
+                wr = (T)dr;
+                wi = (T)di;
             }
-            const int64_t idx = rank_warp<U>((const U*)a.reps, a.n, spl, (int)a.nsplit, a.stride, m, alive);
+            if (R.check_weight && __popcll((unsigned long long)t) != a.nup) alive = false;
+            if (alive) row_orbit<U>(R, g, t, m, ec, st);
+            const int64_t idx = rank_warp<U>((const U*)R.reps, a.n, spl, (int)R.nsplit, R.stride, m, alive);
             if (!alive || idx < 0) continue;
-            const T f = (T)sqrt_stab[st] * inv_sr;
-            if (kCM) {
-                T cr = (T)__ldg(chr + bi * cstride), ci = (T)__ldg(chi + bi * cstride);
-                if (a.conj_chi) ci = -ci;
-                const T nr = wr * cr - wi * ci, ni = wr * ci + wi * cr;
-                wr = nr * f;
-                wi = ni * f;
-            } else {
-                wr *= (T)__ldg(chr + bi * cstride) * f;
-            }
-            T xr, xi;
-            load_x<T, kCV>(a, idx, xr, xi);
-            if (kCM) {
-                acc_r += wr * xr - wi * xi;
-                acc_i += wr * xi + wi * xr;
-            } else if (kCV) {
-                acc_r += wr * xr;
-                acc_i += wr * xi;
-            } else {
-                acc_r += wr * xr;
-            }
+            const int sign = __popcll((unsigned long long)(s & (U)p.zy)) & 1;
+            add_transition<kCM, kCV, T>(a, dyn, p.cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
         }
-        if (!rv) continue;
-        typename V2<T>::t d = ((const typename V2<T>::t*)a.diag)[r];
-        const T dr = d.x, di = a.conj_amp ? -d.y : d.y;
-        T xr, xi;
-        load_x<T, kCV>(a, r, xr, xi);
-        if (kCV) {
-            acc_r += dr * xr - di * xi;
-            acc_i += dr * xi + di * xr;
-        } else {
-            acc_r += dr * xr;
-        }
-        if (kCV) {
-            typename V2<T>::t* y = (typename V2<T>::t*)a.y;
-            T yr = 0, yi = 0;
-            if (!a.beta_zero) {
-                typename V2<T>::t yo = y[r];
-                yr = (T)a.br * yo.x - (T)a.bi * yo.y;
-                yi = (T)a.br * yo.y + (T)a.bi * yo.x;
-            }
-            typename V2<T>::t o;
-            o.x = yr + (T)a.ar * acc_r - (T)a.ai * acc_i;
-            o.y = yi + (T)a.ar * acc_i + (T)a.ai * acc_r;
-            y[r] = o;
-        } else {
-            T* y = (T*)a.y;
-            const T yr = a.beta_zero ? (T)0 : (T)a.br * y[r];
-            y[r] = yr + (T)a.ar * acc_r;
-        }
+        if (rv) store_row<true, kCM, kCV, T>(a, r, acc_r, acc_i);
     }
 }
 
@@ -602,11 +621,11 @@ __global__ void to_single_kernel(const double* in, float* out, int64_t n) {
         out[i] = (float)in[i];
 }
 
-int mv_grid(int64_t n) {
+int mv_grid(int64_t n, int threads = kMvThreads) {
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t blocks = (n + kMvThreads - 1) / kMvThreads;
+    int64_t blocks = (n + threads - 1) / threads;
     int64_t cap = (int64_t)sms * 8;
     return (int)std::max<int64_t>(1, std::min(blocks, cap));
 }
@@ -625,18 +644,66 @@ MvArgs base_args(const Op& op) {
     a.L = b.L;
     a.nup = b.nup;
     a.pauli = b.spec.pauli;
-    a.index = b.has_index ? b.d_index.as<int32_t>() : nullptr;
-    a.fast = b.fast;
-    a.fast_chi = b.fast.enabled ? b.d_fast_chi.as<double>() : nullptr;
     return a;
+}
+
+// What matvec_kernel and matvec_warp_rank_kernel take besides: the row walk and
+// the values.  `bwd`: the second half of the programs (the chain of A itself).
+void row_args(const Op& op, bool bwd, MvArgs& a) {
+    const Basis& b = *op.basis;
+    const size_t half = op.progs.size() / 2;
+    a.progs = op.d_progs.as<TermProg>() + (bwd ? half : 0);
+    a.nprog = (int)half;
+    a.row = op_row_args(op, bwd);
+    if (b.symmetric && b.fast.enabled) {
+        a.chi_re = b.d_fast_chi.as<double>();
+        a.chi_im = a.chi_re + 1;
+        a.chi_stride = 2;
+        a.nelem = 4 * b.fast.nT;
+    } else if (b.symmetric) {
+        a.chi_re = b.d_group.as<GroupDesc>()->chi_re;
+        a.chi_im = b.d_group.as<GroupDesc>()->chi_im;
+        a.chi_stride = 1;
+        a.nelem = b.group.ng;
+    }
+    bool ones = true;
+    for (int e = 0; b.symmetric && e < b.group.ng; ++e)
+        ones = ones && b.group.chi_re[e] == 1.0 && b.group.chi_im[e] == 0.0;
+    if (ones) a.nelem = 1;
+    a.amp = op.d_amp.as<double2>();
+    a.nclass = op.nclass;
+    a.table = (int64_t)op.nclass * a.nelem <= kMvTable;
+    a.any_chars = op.any_chars;
+    a.sq = b.d_sqrt.as<double>();
+}
+
+// Launches a row kernel with `dyn` bytes of dynamic shared memory; the rank
+// tables of the longest chains pass the default 48 KB.
+template <class K>
+void launch_rows(K kernel, int grid, int threads, size_t dyn, cudaStream_t s, const MvArgs& a) {
+    if (dyn > 16 * 1024)
+        QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    kernel<<<grid, threads, dyn, s>>>(a);
+}
+
+// Threads per block: at least four blocks per SM where the rows allow (one
+// product of 12,870 rows: 51 blocks of 256 threads left two SMs of three idle)
+int mv_threads(int64_t n) {
+    int t = kMvThreads;
+    while (t > 64 && n < (int64_t)t * 152 * 4) t /= 2;
+    return t;
 }
 
 template <typename U, int kMode, typename T>
 void launch_mode(const MvArgs& a, bool cm, bool cv, cudaStream_t s) {
-    int grid = mv_grid(a.n);
-    if (cm) matvec_kernel<U, kMode, true, true, T><<<grid, kMvThreads, 0, s>>>(a);
-    else if (cv) matvec_kernel<U, kMode, false, true, T><<<grid, kMvThreads, 0, s>>>(a);
-    else matvec_kernel<U, kMode, false, false, T><<<grid, kMvThreads, 0, s>>>(a);
+    const int threads = mv_threads(a.n);
+    const int grid = mv_grid(a.n, threads);
+    const bool ranks = sizeof(U) == 4 && (kMode == 1 || kMode == 3);
+    const size_t dyn = (a.table ? mv_table_bytes(a.nclass * a.nelem, cm, sizeof(T)) : 0) +
+                       (ranks ? (size_t)a.row.rank.size * sizeof(uint32_t) : 0);
+    if (cm) launch_rows(matvec_kernel<U, kMode, true, true, T>, grid, threads, dyn, s, a);
+    else if (cv) launch_rows(matvec_kernel<U, kMode, false, true, T>, grid, threads, dyn, s, a);
+    else launch_rows(matvec_kernel<U, kMode, false, false, T>, grid, threads, dyn, s, a);
 }
 
 // QS_RANK_MODE picks the rank lookup of a symmetric sector's generated states
@@ -657,15 +724,16 @@ void launch_matvec(const Basis& b, const MvArgs& a, bool cm, bool cv, cudaStream
     const int rm = b.symmetric ? rank_mode_env() : -1;
     if (rm == 4) {
         const int grid = mv_grid(a.n);
-        if (b.wide) {
-            if (cm) matvec_warp_rank_kernel<uint64_t, true, true, T><<<grid, kMvThreads, 0, s>>>(a);
-            else if (cv) matvec_warp_rank_kernel<uint64_t, false, true, T><<<grid, kMvThreads, 0, s>>>(a);
-            else matvec_warp_rank_kernel<uint64_t, false, false, T><<<grid, kMvThreads, 0, s>>>(a);
-        } else {
-            if (cm) matvec_warp_rank_kernel<uint32_t, true, true, T><<<grid, kMvThreads, 0, s>>>(a);
-            else if (cv) matvec_warp_rank_kernel<uint32_t, false, true, T><<<grid, kMvThreads, 0, s>>>(a);
-            else matvec_warp_rank_kernel<uint32_t, false, false, T><<<grid, kMvThreads, 0, s>>>(a);
-        }
+        const size_t dyn = a.table ? mv_table_bytes(a.nclass * a.nelem, cm, sizeof(T)) : 0;
+#define QS_WARP(U_)                                                                                                 \
+        do {                                                                                                        \
+            if (cm) launch_rows(matvec_warp_rank_kernel<U_, true, true, T>, grid, kMvThreads, dyn, s, a);           \
+            else if (cv) launch_rows(matvec_warp_rank_kernel<U_, false, true, T>, grid, kMvThreads, dyn, s, a);     \
+            else launch_rows(matvec_warp_rank_kernel<U_, false, false, T>, grid, kMvThreads, dyn, s, a);            \
+        } while (0)
+        if (b.wide) QS_WARP(uint64_t);
+        else QS_WARP(uint32_t);
+#undef QS_WARP
         return;
     }
     if (b.symmetric && rm == 2) {
@@ -680,8 +748,7 @@ void launch_matvec(const Basis& b, const MvArgs& a, bool cm, bool cv, cudaStream
         if (b.wide) launch_mode<uint64_t, 2, T>(a, cm, cv, s);
         else launch_mode<uint32_t, 2, T>(a, cm, cv, s);
     } else if (b.nup >= 0) {
-        // up to 32 sites: 32-bit states, the binomial table in shared memory
-        // and ranks updated from the row's own rank
+        // up to 32 sites: 32-bit states and the split rank tables
         if (b.wide) launch_mode<uint64_t, 1, T>(a, cm, cv, s);
         else launch_mode<uint32_t, 1, T>(a, cm, cv, s);
     } else {
@@ -710,6 +777,84 @@ Op::~Op() {
     if (own_stream) cudaStreamDestroy(own_stream);
 }
 
+namespace {
+
+// The programs as the row kernels read them (RowProg) and their amplitude
+// classes.
+void prepare_row_programs(Op& op) {
+    const Basis& b = *op.basis;
+    std::vector<RowProg> rows(op.progs.size());
+    std::map<std::pair<double, double>, uint32_t> seen;
+    std::vector<double> amp;
+    op.any_zy = op.check_weight = op.any_chars = false;
+    op.real_amp = true;
+    for (size_t k = 0; k < op.progs.size(); ++k) {
+        const TermProg& p = op.progs[k];
+        RowProg& r = rows[k];
+        r = RowProg{};
+        if (!p.distinct) {
+            // care = value = 0: alive on every state until its characters say otherwise
+            r.cls = kCharsClass;
+            r.chars = 1;
+            op.any_chars = true;
+            op.check_weight = b.nup >= 0;
+            continue;
+        }
+        r.care = p.need0 | p.need1;
+        r.value = p.need1;
+        r.flip = p.flip;
+        r.zy = p.zmask ^ p.ymask;
+        // popc(~s & z) = popc(z) - popc(s & z): the constant part joins the amplitude
+        const double sg = (__builtin_popcountll(p.zmask) & 1) ? -1.0 : 1.0;
+        const std::pair<double, double> v{sg * p.amp0_re, sg * p.amp0_im};
+        auto it = seen.find(v);
+        if (it == seen.end()) {
+            it = seen.emplace(v, (uint32_t)(amp.size() / 2)).first;
+            amp.push_back(v.first);
+            amp.push_back(v.second);
+        }
+        r.cls = it->second;
+        if (r.zy) op.any_zy = true;
+        if (v.second != 0.0) op.real_amp = false;
+        // the particle number: every flipped site raised or lowered, as many up as down
+        if ((p.flip & ~(p.need0 | p.need1)) != 0 ||
+            __builtin_popcountll(p.flip & p.need0) != __builtin_popcountll(p.flip & p.need1))
+            op.check_weight = op.check_weight || b.nup >= 0;
+    }
+    op.nclass = (int)(amp.size() / 2);
+    op.d_rowprogs.alloc(std::max<size_t>(1, rows.size()) * sizeof(RowProg));
+    op.d_amp.alloc(std::max<size_t>(2, amp.size()) * sizeof(double));
+    if (!rows.empty())
+        QS_CUDA(cudaMemcpy(op.d_rowprogs.p, rows.data(), rows.size() * sizeof(RowProg), cudaMemcpyHostToDevice));
+    if (!amp.empty()) QS_CUDA(cudaMemcpy(op.d_amp.p, amp.data(), amp.size() * sizeof(double), cudaMemcpyHostToDevice));
+}
+
+}  // namespace
+
+RowArgs op_row_args(const Op& op, bool bwd) {
+    const Basis& b = *op.basis;
+    RowArgs R{};
+    R.reps = b.symmetric ? b.d_reps.p : nullptr;
+    R.stab = b.d_stab.as<uint16_t>();
+    R.split = b.d_split.p;
+    R.n = b.n;
+    R.nsplit = b.nsplit;
+    R.stride = b.split_stride;
+    R.group = b.d_group.as<GroupDesc>();
+    R.binom = b.d_binom.as<uint64_t>();
+    R.index = b.has_index ? b.d_index.as<int32_t>() : nullptr;
+    R.L = b.L;
+    R.nup = b.nup;
+    R.nprog = (int)(op.progs.size() / 2);
+    R.progs = op.d_rowprogs.as<RowProg>() + (bwd ? R.nprog : 0);
+    R.any_zy = op.any_zy;
+    R.check_weight = op.check_weight;
+    R.fast = b.fast;
+    R.rank = b.rank;
+    R.rank_tab = b.d_rank.as<uint32_t>();
+    return R;
+}
+
 void op_prepare_device(Op& op) {
     Basis& b = *op.basis;
     if (!op.own_stream) {
@@ -720,6 +865,7 @@ void op_prepare_device(Op& op) {
     op.d_progs.alloc(np * sizeof(TermProg));
     if (!op.progs.empty())
         QS_CUDA(cudaMemcpy(op.d_progs.p, op.progs.data(), op.progs.size() * sizeof(TermProg), cudaMemcpyHostToDevice));
+    prepare_row_programs(op);
     // diagonal: user diagonal plus, when extracted, the diagonal programs
     DevBuf user(2 * b.n * sizeof(double));
     if (!op.user_diag.empty())
@@ -775,8 +921,7 @@ void op_matvec_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     a.y = c.y;
     // the pull form of op(A) runs the chain of op(A)^T; a transposed call runs
     // A's own chain (programs are stored for both)
-    if (T) a.progs = op.d_progs.as<TermProg>() + op.progs.size() / 2;
-    a.nprog = (int)op.progs.size() / 2;
+    row_args(op, T, a);
     const bool cm = op.complex_mat;
     const bool cv = c.y_complex;
     if (c.x_complex && !c.y_complex) throw Error(QS_ERR_ARGUMENT, "a complex input needs a complex output");
@@ -805,9 +950,11 @@ void op_matvec_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     if (c.df_io) throw Error(QS_ERR_UNSUPPORTED, "double-float vectors need an assembled operator");
     if (c.single) {
         a.diag = op.d_diag32.p;
+        a.diag_re = op.d_diag32_re.p;
         launch_matvec<float>(b, a, cm, cv, s);
     } else {
         a.diag = op.d_diag.p;
+        a.diag_re = op.d_diag_re.p;
         launch_matvec<double>(b, a, cm, cv, s);
     }
     QS_CUDA(cudaGetLastError());

@@ -30,6 +30,12 @@ struct FastGroup {
     int32_t has_refl, has_flip;
     uint64_t lmask;
     uint64_t allowed;    // bit p set when L-1-p is a multiple of a
+    // orbit minimum by windows (orbit_min_win): 1 one-site translations of at
+    // most 32 sites, 2 no translations (nT = 1), 0 not available
+    int32_t win;
+    int32_t need_j;      // the characters depend on the rotation
+    int32_t nper;        // L / q for the primes q of L: the rotations that fix a
+    int32_t per[3];      // state with any rotational symmetry
 };
 
 #ifdef __CUDACC__

@@ -47,7 +47,7 @@ using Clock = std::chrono::steady_clock;
 
 size_t basis_bytes(const Basis& b) {
     return b.d_group.bytes + b.d_reps.bytes + b.d_stab.bytes + b.d_split.bytes + b.d_binom.bytes + b.d_index.bytes +
-           b.d_fast_chi.bytes + b.d_level_groups.bytes + b.d_level0.bytes + b.d_sqrt.bytes;
+           b.d_fast_chi.bytes + b.d_level_groups.bytes + b.d_level0.bytes + b.d_rank.bytes + b.d_sqrt.bytes;
 }
 
 size_t op_bytes(const Op& o) {
