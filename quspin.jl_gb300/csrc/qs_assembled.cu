@@ -23,6 +23,7 @@
 #include "qs_device.cuh"
 #include "qs_df.cuh"
 #include "qs_internal.h"
+#include "qs_rows.cuh"
 
 namespace qs {
 
@@ -32,34 +33,29 @@ constexpr int kThreads = 256;
 constexpr int kMaxSplit = 2048;
 
 struct BuildArgs {
-    const void* reps;
-    const uint16_t* stab;
-    const void* split;
-    int64_t n, nsplit, stride;
-    const GroupDesc* group;
-    const uint64_t* binom;
-    const int32_t* index;
-    int L, nup, mode;      // mode: 0 full space, 1 combinadic, 2 search, 3 direct index
-    const TermProg* progs;
-    int nprog;
-    const uint16_t* prog_code;   // (aclass * 2 + sign) per program
-    const uint16_t* elem_code;   // (cclass * 2 + sign) per group element
+    RowArgs row;
+    const uint32_t* code_base;   // per (program class, element): value code without the stabiliser class
+    int nelem;                   // elements per class (1: no symmetry)
     const uint8_t* stab_class;   // dclass per stabiliser order
-    FastGroup fast;              // zero-run orbit search when enabled
-    const uint16_t* fast_code;   // (cclass * 2 + sign) per fast element code
-    int nC, nD, code_bits;
-    int32_t* counts;             // pass 1
-    const int64_t* rowptr;       // pass 2
+    int code_bits, packed;
+    // sliced-ELL form: first word of each slice, each row's length, and the
+    // totals (nonzeros, longest row)
+    const int64_t* sptr;
+    uint16_t* len;
+    unsigned long long* nnz;
+    int* maxlen;
+    // CSR form
+    int32_t* counts;
+    const int64_t* rowptr;
     uint32_t* words;
     uint16_t* codes;             // unpacked layout: code per nonzero
     int32_t* cols;               // unpacked layout: column per nonzero
-    int packed;
 };
 
 template <typename U>
-__device__ __forceinline__ U build_row_state(const BuildArgs& a, int64_t r) {
-    if (a.mode >= 2) return ((const U*)a.reps)[r];
-    if (a.mode == 0) return (U)r;
+__device__ __forceinline__ U build_row_state(const RowArgs& a, int mode, int64_t r) {
+    if (mode >= 2) return ((const U*)a.reps)[r];
+    if (mode == 0) return (U)r;
     U s = 0;
     int b = a.L - 1;
     int64_t rem = r;
@@ -72,73 +68,133 @@ __device__ __forceinline__ U build_row_state(const BuildArgs& a, int64_t r) {
     return s;
 }
 
-template <typename U, bool kWrite>
-__global__ void __launch_bounds__(kThreads) build_kernel(BuildArgs a) {
-    __shared__ GroupSmem g;
-    __shared__ U spl[kMaxSplit];
-    if (a.mode >= 2) {
-        load_group_smem(g, a.group);
-        if (a.mode == 2)
-            for (int i = threadIdx.x; i < a.nsplit; i += blockDim.x) spl[i] = ((const U*)a.split)[i];
-        __syncthreads();
-    }
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < a.n; r += (int64_t)gridDim.x * blockDim.x) {
-        const U s = build_row_state<U>(a, r);
-        int64_t out = kWrite ? a.rowptr[r] : 0;
-        int32_t cnt = 0;
-        for (int k = 0; k < a.nprog; ++k) {
-            const TermProg& p = a.progs[k];
-            if ((s & (U)p.need1) != (U)p.need1 || (s & (U)p.need0) != (U)0) continue;
-            U t = s ^ (U)p.flip;
-            int sign = (__popcll((unsigned long long)(~s & (U)p.zmask)) + __popcll((unsigned long long)(s & (U)p.ymask))) & 1;
-            int64_t idx;
-            int cclass = 0, dclass = 0;
-            if (a.mode >= 2) {
-                U m;
-                int bi, st;
-                int ec;
-                if (a.fast.enabled) {
-                    orbit_min_fast<U>(a.fast, t, m, bi, st);
-                    ec = a.fast_code[bi];
-                } else {
-                    orbit_min<U>(g, t, m, bi, st);
-                    ec = a.elem_code[bi];
-                }
-                if (a.mode == 3) {
-                    int64_t rk = a.nup >= 0 ? combinadic_rank<U>(m, a.binom, 65) : (int64_t)m;
-                    idx = __ldg(a.index + rk);
-                } else {
-                    idx = rank_search<U>((const U*)a.reps, a.n, spl, (int)a.nsplit, a.stride, m);
-                }
-                if (idx < 0) continue;
-                cclass = ec >> 1;
-                sign ^= ec & 1;
-                dclass = a.stab_class[st];
-            } else if (a.mode == 1) {
-                if (__popcll((unsigned long long)t) != a.nup) continue;
-                idx = combinadic_rank<U>(t, a.binom, 65);
-            } else {
-                idx = (int64_t)t;
+// Per slice of 32 rows, 32 x the most live programs of a row: the room its
+// words can need.  Programs whose images have no column (zero weight in the
+// sector) are counted too; their words stay unused.
+template <typename U>
+__global__ void __launch_bounds__(kRowThreads) live_kernel(RowArgs a, int mode, int64_t nslices, int64_t* slots) {
+    __shared__ RowSmem<U> sm;
+    load_row_progs(sm, a, 0);
+    __syncthreads();
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nslices * kSellSlice;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = base + threadIdx.x;
+        U s = 0;
+        if (r < a.n) s = build_row_state<U>(a, mode, r);
+        unsigned cnt = 0;
+        for (int c0 = 0; c0 < a.nprog; c0 += kRowChunk) {
+            if (a.nprog > kRowChunk) {
+                __syncthreads();
+                load_row_progs(sm, a, c0);
+                __syncthreads();
             }
-            if (kWrite) {
-                int pc = a.prog_code[k];
-                sign ^= pc & 1;
-                uint32_t code = (uint32_t)((((pc >> 1) * a.nC + cclass) * a.nD + dclass) * 2 + sign);
-                if (a.packed) a.words[out] = ((uint32_t)idx << a.code_bits) | code;
-                else {
-                    a.cols[out] = (int32_t)idx;
-                    a.codes[out] = (uint16_t)code;
-                }
-                ++out;
-            } else {
-                ++cnt;
-            }
+            const int nc = min(kRowChunk, a.nprog - c0);
+            for (int i = 0; i < nc; ++i) cnt += (s & sm.care[i]) == sm.value[i];
         }
-        if (!kWrite) a.counts[r] = cnt;
+        if (r >= a.n) cnt = 0;
+        cnt = __reduce_max_sync(0xffffffffu, cnt);
+        const int64_t sl = r / kSellSlice;
+        if ((threadIdx.x & 31) == 0 && sl < nslices) slots[sl] = (int64_t)cnt * kSellSlice;
     }
 }
 
-__global__ void counts_to_i64(const int32_t* c, int64_t* o, int64_t n) {
+// The rows' transitions as (column, value code) words, one thread per row, by
+// the walk of qs_rows.cuh: kOut 0 into the sliced-ELL form at once (one pass:
+// the slices' room comes from live_kernel), 1 counts per row, 2 into CSR.
+template <typename U, int kMode, int kOut>
+__global__ void __launch_bounds__(kRowThreads) build_kernel(BuildArgs a) {
+    constexpr bool kSym = kMode >= 2;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ RowSmem<U> sm;
+    __shared__ GroupSmem g;
+    __shared__ U spl[kMode == 2 ? kMaxSplit : 1];
+    const RowArgs& R = a.row;
+    uint32_t* rtab = (uint32_t*)dyn;
+    if (kSym && !R.fast.enabled) load_group_smem(g, R.group);
+    if (kMode == 2)
+        for (int i = threadIdx.x; i < R.nsplit; i += blockDim.x) spl[i] = ((const U*)R.split)[i];
+    if (sizeof(U) == 4 && (kMode == 1 || kMode == 3))
+        for (int i = threadIdx.x; i < R.rank.size; i += blockDim.x) rtab[i] = R.rank_tab[i];
+    load_row_progs(sm, R, 0);
+    __syncthreads();
+    unsigned long long total = 0;
+    int longest = 0;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < R.n; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = base + threadIdx.x;
+        const bool valid = r < R.n;
+        U s = 0;
+        int64_t out = 0;
+        if (valid) {
+            s = build_row_state<U>(R, kMode, r);
+            if (kOut == 0) out = a.sptr[r / kSellSlice] + (r % kSellSlice);
+            if (kOut == 2) out = a.rowptr[r];
+        }
+        int cnt = 0;
+        for (int c0 = 0; c0 < R.nprog; c0 += kRowChunk) {
+            if (R.nprog > kRowChunk) {
+                __syncthreads();
+                load_row_progs(sm, R, c0);
+                __syncthreads();
+            }
+            row_hops<U>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
+                if (kMode != 0 && R.check_weight && __popcll((unsigned long long)t) != R.nup) return;
+                U m = t;
+                int ec = 0, st = 1;
+                if (kSym) row_orbit<U>(R, g, t, m, ec, st);
+                const int64_t idx = row_column<U, kMode>(R, spl, rtab, m);
+                if (kSym && idx < 0) return;
+                ++cnt;
+                if (kOut == 1) return;
+                uint32_t code = __ldg(a.code_base + (size_t)sm.cls[i] * a.nelem + (kSym ? ec : 0)) ^ (uint32_t)sign;
+                if (kSym) code += 2u * a.stab_class[st];
+                if (a.packed) {
+                    a.words[out] = ((uint32_t)idx << a.code_bits) | code;
+                } else {
+                    a.cols[out] = (int32_t)idx;
+                    a.codes[out] = (uint16_t)code;
+                }
+                out += kOut == 0 ? kSellSlice : 1;
+            });
+        }
+        if (valid) {
+            if (kOut == 0) {
+                a.len[r] = (uint16_t)cnt;
+                total += (unsigned)cnt;
+                longest = max(longest, cnt);
+            }
+            if (kOut == 1) a.counts[r] = cnt;
+        }
+    }
+    if (kOut == 0) {
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(a.nnz, total);
+            atomicMax(a.maxlen, longest);
+        }
+    }
+}
+
+// Launches build_kernel for the basis' kind of states and lookup.
+template <int kOut>
+void launch_build(const Basis& b, const BuildArgs& a, int grid, cudaStream_t s) {
+    const int mode = b.symmetric ? (b.has_index ? 3 : 2) : (b.nup >= 0 ? 1 : 0);
+    const bool wide = b.symmetric ? b.wide : (b.wide || mode == 0);
+    const size_t dyn = !wide && (mode == 1 || mode == 3) ? (size_t)a.row.rank.size * sizeof(uint32_t) : 0;
+    auto go = [&](auto kernel) {
+        if (dyn > 16 * 1024)
+            QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+        kernel<<<grid, kThreads, dyn, s>>>(a);
+        QS_CUDA(cudaGetLastError());
+    };
+    if (mode == 0) go(build_kernel<uint64_t, 0, kOut>);
+    else if (mode == 1) wide ? go(build_kernel<uint64_t, 1, kOut>) : go(build_kernel<uint32_t, 1, kOut>);
+    else if (mode == 2) wide ? go(build_kernel<uint64_t, 2, kOut>) : go(build_kernel<uint32_t, 2, kOut>);
+    else wide ? go(build_kernel<uint64_t, 3, kOut>) : go(build_kernel<uint32_t, 3, kOut>);
+}
+
+template <typename C>
+__global__ void counts_to_i64(const C* c, int64_t* o, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         o[i] = c[i];
 }
@@ -388,11 +444,10 @@ __global__ void __launch_bounds__(kThreads) spmv_df_kernel(SpmvDFArgs da) {
 constexpr int kSlice = kSellSlice;
 
 __global__ void sell_fill_kernel(const int64_t* rowptr, const uint32_t* words, const int32_t* cols,
-                                 const uint16_t* codes, int packed, const int32_t* perm, const int64_t* sptr,
-                                 int64_t npos, uint32_t* swords, int32_t* scols, uint16_t* scodes) {
+                                 const uint16_t* codes, int packed, const int64_t* sptr, int64_t npos,
+                                 uint32_t* swords, int32_t* scols, uint16_t* scodes) {
     for (int64_t pos = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; pos < npos; pos += (int64_t)gridDim.x * blockDim.x) {
-        const int r = perm[pos];
-        if (r < 0) continue;
+        const int64_t r = pos;
         const int64_t s = pos / kSlice, l = pos % kSlice;
         const int64_t j0 = rowptr[r], j1 = rowptr[r + 1];
         const int64_t base = sptr[s] + l;
@@ -463,7 +518,6 @@ __device__ __forceinline__ void sell_tail(T acc_r, T acc_i, T sc, T dr, T di, T 
 
 struct SellArgs {
     const int64_t* sptr;
-    const int32_t* perm;
     const uint16_t* len;
     const uint32_t* words;
     const int32_t* cols;
@@ -1234,9 +1288,10 @@ int grid_rows(int64_t threads_needed) {
 
 }  // namespace
 
-// Sliced-ELL copy of the CSR words: slices of kSlice consecutive rows, words
-// column-major inside a slice; every row keeps its own length, so the padding
-// of a slice is allocated but never read.
+// Sliced-ELL copy of the CSR words (operators of more than 65,535 programs,
+// whose rows may be too long for the sliced layout): slices of kSlice
+// consecutive rows, words column-major inside a slice; every row keeps its own
+// length, so the padding of a slice is allocated but never read.
 void build_sell(const Basis& b, Assembled& M, cudaStream_t s) {
     const int64_t n = b.n;
     std::vector<int64_t> rp(n + 1);
@@ -1248,14 +1303,12 @@ void build_sell(const Basis& b, Assembled& M, cudaStream_t s) {
     while (((int64_t)1 << M.len_bits) < maxlen) ++M.len_bits;
     M.nslices = (n + kSlice - 1) / kSlice;
     const int64_t npos = M.nslices * kSlice;
-    std::vector<int32_t> perm(npos, -1);
     std::vector<uint16_t> len(npos, 0);
     // Rows stay in their natural order: each thread loops over its own row
     // only, so a slice's padding is never read, while the natural order keeps
     // y, the diagonal and x[r] coalesced and the x gathers of neighbouring
     // rows close together (sorting by length inside windows measured slower).
     for (int64_t r = 0; r < n; ++r) {
-        perm[r] = (int32_t)r;
         len[r] = (uint16_t)(rp[r + 1] - rp[r]);
     }
     std::vector<int64_t> sptr(M.nslices + 1, 0);
@@ -1266,10 +1319,8 @@ void build_sell(const Basis& b, Assembled& M, cudaStream_t s) {
     }
     const int64_t total = std::max<int64_t>(1, sptr[M.nslices]);
     M.sell_ptr.alloc((M.nslices + 1) * sizeof(int64_t));
-    M.sell_perm.alloc(npos * sizeof(int32_t));
     M.sell_len.alloc(npos * sizeof(uint16_t));
     QS_CUDA(cudaMemcpy(M.sell_ptr.p, sptr.data(), (M.nslices + 1) * sizeof(int64_t), cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMemcpy(M.sell_perm.p, perm.data(), npos * sizeof(int32_t), cudaMemcpyHostToDevice));
     QS_CUDA(cudaMemcpy(M.sell_len.p, len.data(), npos * sizeof(uint16_t), cudaMemcpyHostToDevice));
     if (M.packed) {
         M.sell_words.alloc(total * sizeof(uint32_t));
@@ -1279,7 +1330,7 @@ void build_sell(const Basis& b, Assembled& M, cudaStream_t s) {
     }
     sell_fill_kernel<<<grid_rows(npos), kThreads, 0, s>>>(M.rowptr.as<int64_t>(), M.words.as<uint32_t>(),
                                                          M.cols.as<int32_t>(), M.codes.as<uint16_t>(), M.packed,
-                                                         M.sell_perm.as<int32_t>(), M.sell_ptr.as<int64_t>(), npos,
+                                                         M.sell_ptr.as<int64_t>(), n,
                                                          M.sell_words.as<uint32_t>(), M.sell_cols.as<int32_t>(),
                                                          M.sell_codes.as<uint16_t>());
     QS_CUDA(cudaGetLastError());
@@ -1413,76 +1464,107 @@ void op_assemble(Op& op) {
     M.xsplit.alloc((size_t)b.n * 4 * sizeof(float));
 
     cudaStream_t s = op.stream;
-    std::vector<uint16_t> fast_code(std::max<size_t>(1, b.fast_to_elem.size()), 0);
-    for (size_t i = 0; i < b.fast_to_elem.size(); ++i) fast_code[i] = elem_code[b.fast_to_elem[i]];
-    DevBuf d_prog(fwd.size() * sizeof(TermProg) + 1), d_pc(prog_code.size() * 2), d_ec(kMaxGroup * 2),
-        d_sc(kMaxGroup + 1), d_fc(fast_code.size() * 2);
-    QS_CUDA(cudaMemcpy(d_fc.p, fast_code.data(), fast_code.size() * 2, cudaMemcpyHostToDevice));
-    if (!fwd.empty())
-        QS_CUDA(cudaMemcpy(d_prog.p, fwd.data(), fwd.size() * sizeof(TermProg), cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMemcpy(d_pc.p, prog_code.data(), prog_code.size() * 2, cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMemcpy(d_ec.p, elem_code.data(), kMaxGroup * 2, cudaMemcpyHostToDevice));
-    QS_CUDA(cudaMemcpy(d_sc.p, stab_class.data(), kMaxGroup + 1, cudaMemcpyHostToDevice));
+    // value code of a program's class reaching element e, without the
+    // stabiliser class: ((a nC + c) nD) 2 + sign
     BuildArgs a{};
-    a.reps = b.d_reps.p;
-    a.stab = b.d_stab.as<uint16_t>();
-    a.split = b.d_split.p;
-    a.n = b.n;
-    a.nsplit = b.nsplit;
-    a.stride = b.split_stride;
-    a.group = b.d_group.as<GroupDesc>();
-    a.binom = b.d_binom.as<uint64_t>();
-    a.index = b.has_index ? b.d_index.as<int32_t>() : nullptr;
-    a.L = b.L;
-    a.nup = b.nup;
-    a.mode = b.symmetric ? (b.has_index ? 3 : 2) : (b.nup >= 0 ? 1 : 0);
-    a.progs = d_prog.as<TermProg>();
-    a.nprog = (int)fwd.size();
-    a.prog_code = d_pc.as<uint16_t>();
-    a.elem_code = d_ec.as<uint16_t>();
+    a.row = op_row_args(op, false);
+    a.nelem = !b.symmetric ? 1 : (b.fast.enabled ? (int)b.fast_to_elem.size() : G.ng);
+    std::vector<uint32_t> base((size_t)std::max(1, op.nclass) * a.nelem, 0);
+    for (size_t k = 0; k < nfwd; ++k) {
+        // the row walk's sign leaves out the constant part of popc(~s & z)
+        const int sk = (prog_code[k] & 1) ^ (__builtin_popcountll(fwd[k].zmask) & 1);
+        for (int e = 0; e < a.nelem; ++e) {
+            const int ge = b.symmetric && b.fast.enabled ? b.fast_to_elem[e] : e;
+            const int ec = b.symmetric ? elem_code[ge] : 0;
+            base[(size_t)op.prog_class[k] * a.nelem + e] = (uint32_t)((((prog_code[k] >> 1) * nC + (ec >> 1)) * nD) * 2 + (sk ^ (ec & 1)));
+        }
+    }
+    PoolBuf d_base(base.size() * sizeof(uint32_t), s), d_sc(kMaxGroup + 1, s);
+    QS_CUDA(cudaMemcpyAsync(d_base.p, base.data(), base.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    QS_CUDA(cudaMemcpyAsync(d_sc.p, stab_class.data(), kMaxGroup + 1, cudaMemcpyHostToDevice, s));
+    a.code_base = d_base.as<uint32_t>();
     a.stab_class = d_sc.as<uint8_t>();
-    a.fast = b.fast;
-    a.fast_code = d_fc.as<uint16_t>();
-    a.nC = nC;
-    a.nD = nD;
     a.code_bits = code_bits;
     a.packed = packed;
-    DevBuf cnt32(b.n * sizeof(int32_t)), cnt64(b.n * sizeof(int64_t));
-    M.rowptr.alloc((b.n + 1) * sizeof(int64_t));
-    a.counts = cnt32.as<int32_t>();
-    int grid = grid_rows(b.n);
-    const bool wide = b.symmetric ? b.wide : true;
-    if (wide) build_kernel<uint64_t, false><<<grid, kThreads, 0, s>>>(a);
-    else build_kernel<uint32_t, false><<<grid, kThreads, 0, s>>>(a);
-    QS_CUDA(cudaGetLastError());
-    counts_to_i64<<<grid, kThreads, 0, s>>>(cnt32.as<int32_t>(), cnt64.as<int64_t>(), b.n);
-    QS_CUDA(cudaGetLastError());
-    scan_i64(cnt64.as<int64_t>(), M.rowptr.as<int64_t>(), b.n, s);
-    int64_t last = 0, lastc = 0;
-    QS_CUDA(cudaMemcpyAsync(&last, M.rowptr.as<int64_t>() + b.n - 1, 8, cudaMemcpyDeviceToHost, s));
-    QS_CUDA(cudaMemcpyAsync(&lastc, cnt64.as<int64_t>() + b.n - 1, 8, cudaMemcpyDeviceToHost, s));
-    QS_CUDA(cudaStreamSynchronize(s));
-    M.nnz = last + lastc;
-    QS_CUDA(cudaMemcpy(M.rowptr.as<int64_t>() + b.n, &M.nnz, 8, cudaMemcpyHostToDevice));
-    if (packed) {
-        M.words.alloc(std::max<int64_t>(1, M.nnz) * sizeof(uint32_t));
-        a.words = M.words.as<uint32_t>();
+    const int grid = grid_rows(b.n);
+    if (nfwd <= 65535) {
+        // one pass into the sliced form: room per slice from the live programs,
+        // then the words, the rows' lengths and the totals
+        M.nslices = (b.n + kSlice - 1) / kSlice;
+        M.sell_ptr.alloc((M.nslices + 1) * sizeof(int64_t));
+        M.sell_len.alloc(M.nslices * kSlice * sizeof(uint16_t));
+        PoolBuf slots((M.nslices + 1) * sizeof(int64_t), s), totals(2 * sizeof(unsigned long long), s);
+        QS_CUDA(cudaMemsetAsync(slots.p, 0, slots.bytes, s));
+        QS_CUDA(cudaMemsetAsync(totals.p, 0, totals.bytes, s));
+        const int mode = b.symmetric ? 2 : (b.nup >= 0 ? 1 : 0);
+        if (b.symmetric ? !b.wide : (!b.wide && mode == 1))
+            live_kernel<uint32_t><<<grid, kThreads, 0, s>>>(a.row, mode, M.nslices, slots.as<int64_t>());
+        else
+            live_kernel<uint64_t><<<grid, kThreads, 0, s>>>(a.row, mode, M.nslices, slots.as<int64_t>());
+        QS_CUDA(cudaGetLastError());
+        scan_i64(slots.as<int64_t>(), M.sell_ptr.as<int64_t>(), M.nslices + 1, s);
+        int64_t room = 0;
+        QS_CUDA(cudaMemcpyAsync(&room, M.sell_ptr.as<int64_t>() + M.nslices, 8, cudaMemcpyDeviceToHost, s));
+        QS_CUDA(cudaStreamSynchronize(s));
+        room = std::max<int64_t>(1, room);
+        if (packed) {
+            M.sell_words.alloc(room * sizeof(uint32_t));
+        } else {
+            M.sell_cols.alloc(room * sizeof(int32_t));
+            M.sell_codes.alloc(room * sizeof(uint16_t));
+        }
+        a.words = M.sell_words.as<uint32_t>();
+        a.cols = M.sell_cols.as<int32_t>();
+        a.codes = M.sell_codes.as<uint16_t>();
+        a.sptr = M.sell_ptr.as<int64_t>();
+        a.len = M.sell_len.as<uint16_t>();
+        a.nnz = totals.as<unsigned long long>();
+        a.maxlen = (int*)(totals.as<unsigned long long>() + 1);
+        launch_build<0>(b, a, grid, s);
+        unsigned long long t[2] = {0, 0};
+        QS_CUDA(cudaMemcpyAsync(t, totals.p, sizeof(t), cudaMemcpyDeviceToHost, s));
+        QS_CUDA(cudaStreamSynchronize(s));
+        note_launches(2);
+        M.nnz = (int64_t)t[0];
+        int maxlen = 0;
+        std::memcpy(&maxlen, &t[1], sizeof(int));
+        M.len_bits = 0;
+        while (((int64_t)1 << M.len_bits) < maxlen) ++M.len_bits;
+        M.has_sell = true;
     } else {
-        M.cols.alloc(std::max<int64_t>(1, M.nnz) * sizeof(int32_t));
-        M.codes.alloc(std::max<int64_t>(1, M.nnz) * sizeof(uint16_t));
-        a.cols = M.cols.as<int32_t>();
-        a.codes = M.codes.as<uint16_t>();
+        // rows may be longer than the sliced layout's 16-bit lengths: CSR, and
+        // the sliced copy when they are not
+        PoolBuf cnt32(b.n * sizeof(int32_t), s), cnt64(b.n * sizeof(int64_t), s);
+        M.rowptr.alloc((b.n + 1) * sizeof(int64_t));
+        a.counts = cnt32.as<int32_t>();
+        launch_build<1>(b, a, grid, s);
+        counts_to_i64<int32_t><<<grid, kThreads, 0, s>>>(cnt32.as<int32_t>(), cnt64.as<int64_t>(), b.n);
+        QS_CUDA(cudaGetLastError());
+        scan_i64(cnt64.as<int64_t>(), M.rowptr.as<int64_t>(), b.n, s);
+        int64_t last = 0, lastc = 0;
+        QS_CUDA(cudaMemcpyAsync(&last, M.rowptr.as<int64_t>() + b.n - 1, 8, cudaMemcpyDeviceToHost, s));
+        QS_CUDA(cudaMemcpyAsync(&lastc, cnt64.as<int64_t>() + b.n - 1, 8, cudaMemcpyDeviceToHost, s));
+        QS_CUDA(cudaStreamSynchronize(s));
+        M.nnz = last + lastc;
+        QS_CUDA(cudaMemcpy(M.rowptr.as<int64_t>() + b.n, &M.nnz, 8, cudaMemcpyHostToDevice));
+        if (packed) {
+            M.words.alloc(std::max<int64_t>(1, M.nnz) * sizeof(uint32_t));
+            a.words = M.words.as<uint32_t>();
+        } else {
+            M.cols.alloc(std::max<int64_t>(1, M.nnz) * sizeof(int32_t));
+            M.codes.alloc(std::max<int64_t>(1, M.nnz) * sizeof(uint16_t));
+            a.cols = M.cols.as<int32_t>();
+            a.codes = M.codes.as<uint16_t>();
+        }
+        a.rowptr = M.rowptr.as<int64_t>();
+        launch_build<2>(b, a, grid, s);
+        QS_CUDA(cudaStreamSynchronize(s));
+        note_launches(3);
+        // lanes per row: the power of two nearest a quarter of the mean row length
+        const double mean = b.n ? (double)M.nnz / (double)b.n : 0.0;
+        M.lanes = mean > 48 ? 16 : (mean > 12 ? 8 : 4);
+        build_sell(b, M, s);
     }
-    a.rowptr = M.rowptr.as<int64_t>();
-    if (wide) build_kernel<uint64_t, true><<<grid, kThreads, 0, s>>>(a);
-    else build_kernel<uint32_t, true><<<grid, kThreads, 0, s>>>(a);
-    QS_CUDA(cudaGetLastError());
-    QS_CUDA(cudaStreamSynchronize(s));
-    note_launches(4);
-    // lanes per row: the power of two nearest a quarter of the mean row length
-    double mean = b.n ? (double)M.nnz / (double)b.n : 0.0;
-    M.lanes = mean > 48 ? 16 : (mean > 12 ? 8 : 4);
-    build_sell(b, M, s);
     op.assembled = true;
 }
 
@@ -1493,8 +1575,7 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     if (M.has_sell) {
         SellArgs a{};
         a.sptr = M.sell_ptr.as<int64_t>();
-        a.perm = M.sell_perm.as<int32_t>();
-        a.len = M.sell_len.as<uint16_t>();
+            a.len = M.sell_len.as<uint16_t>();
         a.words = M.sell_words.as<uint32_t>();
         a.cols = M.sell_cols.as<int32_t>();
         a.codes = M.sell_codes.as<uint16_t>();
@@ -1784,7 +1865,6 @@ bool op_spmm_device(Op& op, const MatvecCall& c, int64_t nrhs, cudaStream_t s) {
         return false;
     SellArgs a{};
     a.sptr = M.sell_ptr.as<int64_t>();
-    a.perm = M.sell_perm.as<int32_t>();
     a.len = M.sell_len.as<uint16_t>();
     a.words = M.sell_words.as<uint32_t>();
     a.cols = M.sell_cols.as<int32_t>();
@@ -1851,24 +1931,27 @@ bool op_spmm_device(Op& op, const MatvecCall& c, int64_t nrhs, cudaStream_t s) {
 
 namespace {
 
-// Element values of the assembled CSR form: value k of row r is
+// Element values of the assembled form in CSR order: value k of row r is
 // table[code_k] / sqrt(stab_r) (the row scale the products apply after the
-// sum), column col_k.
-__global__ void export_kernel(const int64_t* __restrict__ rowptr, const uint32_t* __restrict__ words,
-                              const int32_t* __restrict__ cols, const uint16_t* __restrict__ codes, int packed,
-                              int cb, uint32_t cmask, const double2* __restrict__ table,
-                              const uint16_t* __restrict__ stab, int64_t n, int64_t* __restrict__ ocol,
-                              double2* __restrict__ oval) {
+// sum), column col_k.  The words are read from CSR, or from the sliced layout
+// (sptr) with a stride of one slice.
+__global__ void export_kernel(const int64_t* __restrict__ rowptr, const int64_t* __restrict__ sptr,
+                              const uint32_t* __restrict__ words, const int32_t* __restrict__ cols,
+                              const uint16_t* __restrict__ codes, int packed, int cb, uint32_t cmask,
+                              const double2* __restrict__ table, const uint16_t* __restrict__ stab, int64_t n,
+                              int64_t* __restrict__ ocol, double2* __restrict__ oval) {
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
         const double sc = stab ? 1.0 / sqrt((double)stab[r]) : 1.0;
-        for (int64_t k = rowptr[r]; k < rowptr[r + 1]; ++k) {
+        const int64_t j0 = sptr ? sptr[r / kSellSlice] + r % kSellSlice : rowptr[r];
+        const int64_t step = sptr ? kSellSlice : 1;
+        for (int64_t k = rowptr[r], j = j0; k < rowptr[r + 1]; ++k, j += step) {
             uint32_t col, code;
             if (packed) {
-                col = words[k] >> cb;
-                code = words[k] & cmask;
+                col = words[j] >> cb;
+                code = words[j] & cmask;
             } else {
-                col = (uint32_t)cols[k];
-                code = codes[k];
+                col = (uint32_t)cols[j];
+                code = codes[j];
             }
             const double2 v = table[code];
             ocol[k] = col;
@@ -1886,16 +1969,30 @@ void op_export_csr(Op& op, int64_t* rowptr, int64_t* cols, double* values, doubl
     const int64_t n = b.n;
     cudaStream_t s = op.stream;
     PoolBuf dcol((size_t)std::max<int64_t>(1, M.nnz) * sizeof(int64_t), s),
-        dval((size_t)std::max<int64_t>(1, M.nnz) * sizeof(double2), s);
+        dval((size_t)std::max<int64_t>(1, M.nnz) * sizeof(double2), s), drow;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
-    export_kernel<<<grid, 256, 0, s>>>(M.rowptr.as<int64_t>(), M.words.as<uint32_t>(), M.cols.as<int32_t>(),
-                                       M.codes.as<uint16_t>(), M.packed ? 1 : 0, M.code_bits,
-                                       M.code_bits >= 32 ? 0xffffffffu : ((1u << M.code_bits) - 1u),
+    const bool sell = M.has_sell;
+    const int64_t* rp = M.rowptr.as<int64_t>();
+    if (sell) {
+        // row pointers from the rows' lengths (the entry past the last row's 0)
+        PoolBuf len64((size_t)(n + 1) * sizeof(int64_t), s);
+        drow.alloc((size_t)(n + 1) * sizeof(int64_t), s);
+        QS_CUDA(cudaMemsetAsync(len64.p, 0, len64.bytes, s));
+        counts_to_i64<uint16_t><<<grid, 256, 0, s>>>(M.sell_len.as<uint16_t>(), len64.as<int64_t>(), n);
+        QS_CUDA(cudaGetLastError());
+        scan_i64(len64.as<int64_t>(), drow.as<int64_t>(), n + 1, s);
+        rp = drow.as<int64_t>();
+    }
+    export_kernel<<<grid, 256, 0, s>>>(rp, sell ? M.sell_ptr.as<int64_t>() : nullptr,
+                                       sell ? M.sell_words.as<uint32_t>() : M.words.as<uint32_t>(),
+                                       sell ? M.sell_cols.as<int32_t>() : M.cols.as<int32_t>(),
+                                       sell ? M.sell_codes.as<uint16_t>() : M.codes.as<uint16_t>(), M.packed ? 1 : 0,
+                                       M.code_bits, M.code_bits >= 32 ? 0xffffffffu : ((1u << M.code_bits) - 1u),
                                        M.table64.as<double2>(), b.symmetric ? b.d_stab.as<uint16_t>() : nullptr, n,
                                        dcol.as<int64_t>(), dval.as<double2>());
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    QS_CUDA(cudaMemcpyAsync(rowptr, M.rowptr.p, (size_t)(n + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    QS_CUDA(cudaMemcpyAsync(rowptr, rp, (size_t)(n + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (M.nnz) {
         QS_CUDA(cudaMemcpyAsync(cols, dcol.p, (size_t)M.nnz * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         QS_CUDA(cudaMemcpyAsync(values, dval.p, (size_t)M.nnz * sizeof(double2), cudaMemcpyDeviceToHost, s));

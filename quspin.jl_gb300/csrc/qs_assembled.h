@@ -133,6 +133,7 @@ __device__ __forceinline__ void sell_row(const uint32_t* __restrict__ words, con
 #endif
 
 struct Assembled {
+    // CSR form: only of operators with more than 65,535 programs
     DevBuf rowptr;     // int64, n + 1
     DevBuf words;      // uint32 (column << code_bits) | code, when packed
     DevBuf cols;       // int32 column per nonzero, when not packed
@@ -153,7 +154,6 @@ struct Assembled {
     DevBuf sell_words;  // uint32 packed (or int32 column + uint16 code pairs as uint32/uint16 arrays)
     DevBuf sell_cols, sell_codes;
     DevBuf sell_ptr;    // int64 start of each slice
-    DevBuf sell_perm;   // int32 row of each slice position (-1 past the end)
     DevBuf sell_len;    // uint16 length of each slice position's row
     int64_t nslices = 0;
     bool has_sell = false;

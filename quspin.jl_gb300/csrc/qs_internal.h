@@ -207,8 +207,9 @@ struct Op {
     // (complex double), and whether a sign depends on the state / a program
     // changes the particle number / runs by its characters
     DevBuf d_rowprogs, d_amp;
+    std::vector<uint32_t> prog_class;
     int nclass = 0;
-    bool any_zy = false, check_weight = false, any_chars = false, real_amp = true;
+    bool any_zy = false, check_weight = false, any_chars = false;
     DevBuf d_diag;                  // complex diagonal (user + extracted), 2*n doubles
     DevBuf d_diag32;                // single-precision copy
     DevBuf d_diag_re, d_diag32_re;  // real parts (read by real operators)

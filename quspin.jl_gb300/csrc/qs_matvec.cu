@@ -787,7 +787,6 @@ void prepare_row_programs(Op& op) {
     std::map<std::pair<double, double>, uint32_t> seen;
     std::vector<double> amp;
     op.any_zy = op.check_weight = op.any_chars = false;
-    op.real_amp = true;
     for (size_t k = 0; k < op.progs.size(); ++k) {
         const TermProg& p = op.progs[k];
         RowProg& r = rows[k];
@@ -815,13 +814,14 @@ void prepare_row_programs(Op& op) {
         }
         r.cls = it->second;
         if (r.zy) op.any_zy = true;
-        if (v.second != 0.0) op.real_amp = false;
         // the particle number: every flipped site raised or lowered, as many up as down
         if ((p.flip & ~(p.need0 | p.need1)) != 0 ||
             __builtin_popcountll(p.flip & p.need0) != __builtin_popcountll(p.flip & p.need1))
             op.check_weight = op.check_weight || b.nup >= 0;
     }
     op.nclass = (int)(amp.size() / 2);
+    op.prog_class.resize(rows.size());
+    for (size_t k = 0; k < rows.size(); ++k) op.prog_class[k] = rows[k].cls;
     op.d_rowprogs.alloc(std::max<size_t>(1, rows.size()) * sizeof(RowProg));
     op.d_amp.alloc(std::max<size_t>(2, amp.size()) * sizeof(double));
     if (!rows.empty())

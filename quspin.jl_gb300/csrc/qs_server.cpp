@@ -56,7 +56,7 @@ size_t op_bytes(const Op& o) {
            o.d_diag_df.bytes + o.d_x.bytes + o.d_y.bytes + o.d_x32.bytes + o.d_y32.bytes + M.rowptr.bytes +
            M.words.bytes + M.cols.bytes + M.codes.bytes + M.table64.bytes + M.table32.bytes + M.table_df.bytes +
            M.xsplit.bytes + M.rsq_df.bytes + M.sell_words.bytes + M.sell_cols.bytes + M.sell_codes.bytes +
-           M.sell_ptr.bytes + M.sell_perm.bytes + M.sell_len.bytes;
+           M.sell_ptr.bytes + M.sell_len.bytes + o.d_rowprogs.bytes + o.d_amp.bytes;
 }
 
 double binom(int n, int k) {
@@ -323,7 +323,7 @@ void builder_loop(Server& S) {
                 c->op = op_create(c->basis.get(), tv.data(), (int)tv.size(), nullptr,
                                   QS_CHECK_SYMM | QS_CHECK_HERM | QS_CHECK_PCON);
                 op_assemble(*c->op);
-                // the engine reads only the sliced layout: drop the row-compressed copy
+                // the engine reads only the sliced layout: drop a row-compressed form
                 Assembled& M = c->op->asm_;
                 M.rowptr.release();
                 M.words.release();

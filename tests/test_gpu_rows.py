@@ -1,4 +1,4 @@
-"""The row walk of the matrix-free product (live-program masks, orbit minimum by
+"""The row walk of the matrix-free product and the assembly (live-program masks, orbit minimum by
 windows, split rank tables) at the sizes where it can go wrong, against the
 oracle's representative-space product."""
 import os
@@ -84,3 +84,49 @@ def test_site_acted_on_twice(qs, ora):
     got = qs.QuantumLinearOperator(b, models.to_terms(qs, spec), check_herm=False).dot(x)
     want = ref.qlo_matvec(ora.consolidate_terms(spec), x)
     assert np.max(np.abs(got - want)) <= 1e-13 * max(1.0, float(np.abs(want).max()))
+
+
+# (the two-site chain's second-neighbour bond acts on one site twice: not assembled)
+@pytest.mark.parametrize("L,nup,sym,model", CASES[1:])
+def test_assembled_walk_against_matrix_free(qs, L, nup, sym, model):
+    """The assembly walks the same transitions: its product (table values, the same
+    order) agrees with the matrix-free one to rounding, and so does its export."""
+    spec = {"j1j2": lambda: models.j1j2(L, 1.0, 0.45), "tfim": lambda: models.tfim(L), "pairs": lambda: all_pairs(L),
+            "xyz": lambda: models.xyz_field(L)}[model]()
+    b = qs.SpinBasis1D(L, nup=nup, pauli=model == "tfim", **sym)
+    terms = models.to_terms(qs, spec)
+    x = models.seeded(b.Ns, complex_=True)
+    want = qs.QuantumLinearOperator(b, terms).dot(x)
+    H = qs.Hamiltonian(b, terms)
+    assert H.assembled
+    scale = max(1.0, float(np.abs(want).max()))
+    assert np.max(np.abs(H.dot(x) - want)) <= 1e-13 * scale
+    assert np.max(np.abs(H.tocsr() @ x - want)) <= 1e-13 * scale
+
+
+@pytest.mark.parametrize("L,nup,longest", [(24, 1, 5313), (11, None, 65536)])
+def test_assembly_of_many_programs(qs, L, nup, longest):
+    """More than 65,535 programs: assembled through CSR, kept in the sliced layout
+    where the rows fit its lengths (nup = 1) and in CSR where they do not."""
+    from itertools import combinations
+    rng = np.random.default_rng(11)
+    if nup:
+        c = [(float(v), *ij, *kl) for ij in combinations(range(1, L + 1), 2)
+             for kl in combinations([q for q in range(1, L + 1) if q not in ij], 2) for v in [rng.choice([0.25, 0.5])]]
+        spec = [("+-zz", c), ("-+zz", c)]
+    else:
+        spec = []
+        for nx in range(1, 9):
+            for nz in range(0, 9 - nx):
+                spec.append(("x" * nx + "z" * nz,
+                             [(0.5, *xs, *zs) for xs in combinations(range(1, L + 1), nx)
+                              for zs in combinations([q for q in range(1, L + 1) if q not in xs], nz)]))
+    b = qs.SpinBasis1D(L, nup=nup, pauli=True)
+    terms = models.to_terms(qs, spec)
+    H = qs.Hamiltonian(b, terms)
+    assert H.assembled and H.nnz >= longest * (b.Ns if nup is None else 1)
+    x = models.seeded(b.Ns)
+    want = qs.QuantumLinearOperator(b, terms).dot(x)
+    # rows of up to 1.3e5 terms of the same size: n eps of the sum of magnitudes
+    mag = H.nnz / b.Ns * 4 * np.abs(x).max()
+    assert np.max(np.abs(H.dot(x) - want)) <= 1e-13 * mag
