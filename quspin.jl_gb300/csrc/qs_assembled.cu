@@ -1992,12 +1992,12 @@ void op_export_csr(Op& op, int64_t* rowptr, int64_t* cols, double* values, doubl
                                        dcol.as<int64_t>(), dval.as<double2>());
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    QS_CUDA(cudaMemcpyAsync(rowptr, rp, (size_t)(n + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    copy_to_host(rowptr, rp, (size_t)(n + 1) * sizeof(int64_t), s);
     if (M.nnz) {
-        QS_CUDA(cudaMemcpyAsync(cols, dcol.p, (size_t)M.nnz * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        QS_CUDA(cudaMemcpyAsync(values, dval.p, (size_t)M.nnz * sizeof(double2), cudaMemcpyDeviceToHost, s));
+        copy_to_host(cols, dcol.p, (size_t)M.nnz * sizeof(int64_t), s);
+        copy_to_host(values, dval.p, (size_t)M.nnz * sizeof(double2), s);
     }
-    QS_CUDA(cudaMemcpyAsync(diag, op.d_diag.p, (size_t)n * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    copy_to_host(diag, op.d_diag.p, (size_t)n * sizeof(double2), s);
     QS_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -2067,8 +2067,12 @@ bool op_matvec_host_overlap(Op& op, const MatvecCall& c0, void* y_host, size_t e
         c.fx_ready = k > 0;   // the first range makes the integer copy of x for all
         op_spmv_device(op, c, op.stream);
         QS_CUDA(cudaEventRecord(op.range_done[k], op.stream));
+    }
+    touch_host(y_host, (size_t)n * eb);   // while the ranges compute
+    for (int k = 0; k < K; ++k) {
         QS_CUDA(cudaStreamWaitEvent(op.copy_stream, op.range_done[k], 0));
-        const int64_t r0 = c.slice0 * kSellSlice, r1 = std::min<int64_t>(n, c.slice1 * kSellSlice);
+        const int64_t r0 = M.nslices * k / K * kSellSlice;
+        const int64_t r1 = std::min<int64_t>(n, M.nslices * (k + 1) / K * kSellSlice);
         if (r1 > r0)
             QS_CUDA(cudaMemcpyAsync((char*)y_host + (size_t)r0 * eb, (const char*)c0.y + (size_t)r0 * eb,
                                     (size_t)(r1 - r0) * eb, cudaMemcpyDeviceToHost, op.copy_stream));

@@ -1755,7 +1755,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
         else embed_kernel<uint32_t><<<grid, 256, 0, s>>>(e);
         QS_CUDA(cudaGetLastError());
         note_launches(1);
-        if (!device) QS_CUDA(cudaMemcpyAsync(out, pout, (size_t)nout * sizeof(double2), cudaMemcpyDeviceToHost, s));
+        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
         QS_CUDA(cudaStreamSynchronize(s));
         return;
     }
@@ -1789,7 +1789,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
         }
         QS_CUDA(cudaGetLastError());
         note_launches(1);
-        if (!device) QS_CUDA(cudaMemcpyAsync(out, pout, (size_t)nout * sizeof(double2), cudaMemcpyDeviceToHost, s));
+        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
         QS_CUDA(cudaStreamSynchronize(s));
         return;
     }
@@ -1818,7 +1818,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
     else project_kernel<uint32_t><<<grid, 128, 0, s>>>(a);
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    if (!device) QS_CUDA(cudaMemcpyAsync(out, pout, (size_t)nout * sizeof(double2), cudaMemcpyDeviceToHost, s));
+    if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
     QS_CUDA(cudaStreamSynchronize(s));
 }
 

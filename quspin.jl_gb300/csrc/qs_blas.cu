@@ -559,6 +559,12 @@ void Blas::scale(void* dst, const void* src, cd a) {
     note_launches(1);
 }
 
+void scale_c128(void* dst, const void* src, cd a, int64_t n, cudaStream_t s) {
+    launch_axpby<double, true>(dst, src, a.real(), a.imag(), 0.0, n, s);
+    QS_CUDA(cudaGetLastError());
+    note_launches(1);
+}
+
 void Blas::axpy(void* y, const void* x, cd a) {
     if (vk_df(kind)) {
         if (kind == VKind::CDF64) axpby_df_kernel<true><<<nblocks(n), kThreads, 0, s>>>(y, x, split4(a), make_float2(1.f, 0.f), n);

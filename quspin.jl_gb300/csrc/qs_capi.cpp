@@ -134,6 +134,7 @@ int qs_basis_orbit_minima(const qs_basis* basis, uint64_t* out, int64_t n) {
             return;
         }
         if (b.wide) {
+            qs::touch_host(out, n * sizeof(uint64_t));
             QS_CUDA(cudaMemcpy(out, b.d_reps.p, n * sizeof(uint64_t), cudaMemcpyDeviceToHost));
         } else {
             std::vector<uint32_t> tmp(n);
@@ -152,6 +153,7 @@ int qs_basis_stabilizers(const qs_basis* basis, uint16_t* out, int64_t n) {
             for (int64_t i = 0; i < n; ++i) out[i] = 1;
             return;
         }
+        qs::touch_host(out, n * sizeof(uint16_t));
         QS_CUDA(cudaMemcpy(out, b.d_stab.p, n * sizeof(uint16_t), cudaMemcpyDeviceToHost));
     });
 }
@@ -365,7 +367,7 @@ int qs_op_matvec(qs_op* op, int32_t flags, const double* alpha, const void* x, i
             // next computes; otherwise one product and one read-back
             if (!qs::op_matvec_host_overlap(o, c, ys, yb)) {
                 qs::op_matvec_device(o, c, o.stream);
-                QS_CUDA(cudaMemcpyAsync(ys, o.d_y.p, n * yb, cudaMemcpyDeviceToHost, o.stream));
+                qs::copy_to_host(ys, o.d_y.p, n * yb, o.stream);
             }
             QS_CUDA(cudaStreamSynchronize(o.stream));
         }

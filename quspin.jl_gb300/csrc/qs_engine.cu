@@ -2100,7 +2100,7 @@ void Engine::store(int id, int col, double* out, bool device) {
     } else {
         PoolBuf st(bytes, s_);
         convert_vec(src, ks, st.p, k64, d.n, s_);
-        QS_CUDA(cudaMemcpyAsync(out, st.p, bytes, cudaMemcpyDeviceToHost, s_));
+        copy_to_host(out, st.p, bytes, s_);
     }
     ++launches_;
     QS_CUDA(cudaStreamSynchronize(s_));
@@ -2473,7 +2473,7 @@ void eigsh_batch(Op** ops, int nops, const qs_eigsh_opts& o, double* values, voi
             eigsh_batch(&one, 1, r, vals.data(), vec ? &vec : nullptr, &inf);
             for (int q = 0; q < k; ++q) values[(size_t)i * k + q] = vals[q];
             if (vectors && vectors[i] && !dev)
-                QS_CUDA(cudaMemcpy(vectors[i], vdev.p, vdev.bytes, cudaMemcpyDeviceToHost));
+                copy_to_host(vectors[i], vdev.p, vdev.bytes, op.stream);
             if (infos) {
                 infos[i].matvecs += inf.matvecs;
                 infos[i].restarts += inf.restarts;
@@ -2481,9 +2481,11 @@ void eigsh_batch(Op** ops, int nops, const qs_eigsh_opts& o, double* values, voi
             }
         } else {
             for (int q = 0; q < k; ++q) values[(size_t)i * k + q] = th[q];
-            if (vectors && vectors[i])
+            if (vectors && vectors[i]) {
+                if (!dev) touch_host(vectors[i], promoted[i].bytes);
                 QS_CUDA(cudaMemcpyAsync(vectors[i], promoted[i].p, promoted[i].bytes,
                                         dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, op.stream));
+            }
             if (infos) {
                 infos[i].matvecs += k;
                 infos[i].max_rel_residual = maxrel;
@@ -2620,13 +2622,16 @@ static void run_evo_slots(Engine& E, std::vector<int>& ids, std::vector<EvoTask>
         const double b = tasks[i].beta;
         if (device) {
             E.store(ids[i], 0, outs[i], true);
-            Blas B(VKind::C128, n, E.stream());
-            B.scale(outs[i], outs[i], cd(b, 0));
+            scale_c128(outs[i], outs[i], cd(b, 0), n, E.stream());
             QS_CUDA(cudaStreamSynchronize(E.stream()));
             return;
         }
-        E.store(ids[i], 0, outs[i], false);
-        for (int64_t q = 0; q < 2 * n; ++q) outs[i][q] *= b;
+        // scaled on the device, then one copy
+        PoolBuf col((size_t)n * 2 * sizeof(double), E.stream());
+        E.store(ids[i], 0, col.as<double>(), true);
+        scale_c128(col.p, col.p, cd(b, 0), n, E.stream());
+        copy_to_host(outs[i], col.p, col.bytes, E.stream());
+        QS_CUDA(cudaStreamSynchronize(E.stream()));
     };
     for (size_t i = 0; i < nt; ++i)
         if (fin[i]) emit(i);
@@ -2832,7 +2837,7 @@ void evolve_stepwise(Op& op, const double* v0, const std::vector<double>& offset
             }
             prev = offsets[i];
         }
-        QS_CUDA(cudaMemcpyAsync(out + (size_t)i * 2 * n, cur.p, bytes, cudaMemcpyDeviceToHost, st));
+        copy_to_host(out + (size_t)i * 2 * n, cur.p, bytes, st);
     }
     QS_CUDA(cudaStreamSynchronize(st));
     note_launches(E.launches());

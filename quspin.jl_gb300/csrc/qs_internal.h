@@ -81,6 +81,14 @@ void pool_trim();
 // Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister,
 // mapped under unified addressing), or null for any other pointer.
 void* mapped_host_address(void* p);
+// Writes one byte of every page of a caller's output back to itself, so that
+// the pages exist before a device copy lands in them.  A copy into untouched
+// pages faults them in one by one from the device: 17 ms for 21 MB on a GB300's
+// Grace host, against 1 ms for the touches and 0.17 ms for the copy (np.zeros
+// and malloc hand out such pages).
+void touch_host(void* p, size_t bytes);
+// Touches dst, then copies device memory into it on s.
+void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 struct PoolBuf {
     void* p = nullptr;

@@ -413,6 +413,7 @@ void eigs_general(Op& op, const qs_eigsh_opts& o, double* values, void* vectors,
         values[2 * q + 1] = theta[q].imag();
     }
     if (o.want_vectors && vectors) {
+        if (!dev) touch_host(vectors, (size_t)n * k * 16);
         QS_CUDA(cudaMemcpyAsync(vectors, X.p, (size_t)n * k * 16, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                 op.stream));
     }
@@ -610,6 +611,7 @@ void eigsh(Op& op, const qs_eigsh_opts& o, double* values, void* vectors, qs_eig
     for (int q = 0; q < k; ++q) values[q] = theta[q];
     if (o.want_vectors && vectors) {
         const void* src = single ? X64.p : X.p;
+        if (!dev) touch_host(vectors, (size_t)n * k * esz);
         QS_CUDA(cudaMemcpyAsync(vectors, src, (size_t)n * k * esz,
                                 dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, op.stream));
         QS_CUDA(cudaStreamSynchronize(op.stream));
@@ -751,7 +753,7 @@ void expm_multiply(Op& op, cd a, const double* v, double* out, double tol, int k
     convert_vec(d64.p, VKind::C128, dv.p, vk, n, op.stream);
     expmv_vector(c, dv.p, a, tol, krylov_dim, 0, dout.p);
     convert_vec(dout.p, vk, d64.p, VKind::C128, n, op.stream);
-    QS_CUDA(cudaMemcpyAsync(out, d64.p, n * 16, cudaMemcpyDeviceToHost, op.stream));
+    copy_to_host(out, d64.p, n * 16, op.stream);
     QS_CUDA(cudaStreamSynchronize(op.stream));
 }
 
@@ -791,7 +793,7 @@ void evolve(Op& op, const double* v0, double t0, const double* times, int nt, in
             src = st.p;
         }
         convert_vec(src, vk, d64.p, VKind::C128, n, op.stream);
-        QS_CUDA(cudaMemcpyAsync(out + (size_t)col * 2 * n, d64.p, n * 16, cudaMemcpyDeviceToHost, op.stream));
+        copy_to_host(out + (size_t)col * 2 * n, d64.p, n * 16, op.stream);
         QS_CUDA(cudaStreamSynchronize(op.stream));
     };
     if (nt == 0) return;

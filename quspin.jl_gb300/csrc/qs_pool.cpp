@@ -6,6 +6,7 @@
 // that event has completed.  cudaMalloc failing with out-of-memory frees the
 // whole cache and retries once.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <map>
 #include <mutex>
@@ -123,6 +124,20 @@ void* mapped_host_address(void* p) {
         return nullptr;
     }
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
+
+void touch_host(void* p, size_t bytes) {
+    static const size_t page = [] {
+        const long v = sysconf(_SC_PAGESIZE);
+        return v > 0 ? (size_t)v : (size_t)4096;
+    }();
+    volatile unsigned char* q = static_cast<volatile unsigned char*>(p);
+    for (size_t o = 0; o < bytes; o += page - ((uintptr_t)(q + o) & (page - 1))) q[o] = q[o];
+}
+
+void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    touch_host(dst, bytes);
+    QS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
 }
 
 void pool_trim() {

@@ -621,7 +621,7 @@ void basis_project_dense(Basis& b, bool pcon, int mode, const double* in, double
     }
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    if (!device) QS_CUDA(cudaMemcpyAsync(out, pout, (size_t)nout * ncols * 16, cudaMemcpyDeviceToHost, s));
+    if (!device) copy_to_host(out, pout, (size_t)nout * ncols * 16, s);
     QS_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -280,7 +280,7 @@ void lanczos_combine(LanczosSet& L, int s, const double* coeff, int ncoef, doubl
         o = tmp.as<double2>();
     }
     combine(column(L, s, 0), L.cv, L.n, used, Y.as<double2>(), ncoef, o, st);
-    if (!device) QS_CUDA(cudaMemcpyAsync(out, tmp.p, tmp.bytes, cudaMemcpyDeviceToHost, st));
+    if (!device) copy_to_host(out, tmp.p, tmp.bytes, st);
     QS_CUDA(cudaStreamSynchronize(st));
 }
 
@@ -380,6 +380,7 @@ void expm_columns(Op& op, const double* V, int ncol, const std::vector<cd>& scal
                     if (nr > 0) B.scale(src, src, cd(1.0 / nr, 0));
                 }
                 double* dst = out + ((size_t)i * ncol + c) * n * 2;   // out[:, c, i]
+                if (!device) touch_host(dst, col_bytes);
                 QS_CUDA(cudaMemcpyAsync(dst, src, col_bytes, device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                         st));
             }
@@ -435,7 +436,7 @@ void block_expm(const std::vector<Op*>& ops, bool pcon, const double* psi, const
     for (size_t q = 0; q < act.size(); ++q)
         basis_project(*act[q]->basis, pcon, 0, outs[q], o, true, true, nt);
     if (!device) {
-        QS_CUDA(cudaMemcpyAsync(out, o, (size_t)rows * nt * 16, cudaMemcpyDeviceToHost, st));
+        copy_to_host(out, o, (size_t)rows * nt * 16, st);
         QS_CUDA(cudaStreamSynchronize(st));
     }
 }
