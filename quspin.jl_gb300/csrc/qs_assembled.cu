@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kRowThreads) live_kernel(RowArgs a, int mode, 
                 __syncthreads();
             }
             const int nc = min(kRowChunk, a.nprog - c0);
-            for (int i = 0; i < nc; ++i) cnt += (s & sm.care[i]) == sm.value[i];
+            for (int i = 0; i < nc; ++i) cnt += (s & sm.test[i].care) == sm.test[i].value;
         }
         if (r >= a.n) cnt = 0;
         cnt = __reduce_max_sync(0xffffffffu, cnt);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kRowThreads) build_kernel(BuildArgs a) {
                 load_row_progs(sm, R, c0);
                 __syncthreads();
             }
-            row_hops<U>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
+            row_hops<U, true>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
                 if (kMode != 0 && R.check_weight && __popcll((unsigned long long)t) != R.nup) return;
                 U m = t;
                 int ec = 0, st = 1;

@@ -250,12 +250,12 @@ __device__ __noinline__ bool run_chars(const MvArgs& a, int k, U s, U& t, double
 
 // acc += w x with the character, sqrt(stab) of the column and the sign of a
 // transition of class cls (a program run by its characters brings its own w)
-template <bool kCM, bool kCV, typename T>
+template <bool kCM, bool kCV, typename T, bool kPlain>
 __device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab, uint32_t cls, int ec, int st, int sign,
                                                T wr, T wi, int64_t idx, T& acc_r, T& acc_i) {
-    if (cls == kCharsClass) {
+    if (!kPlain && cls == kCharsClass) {
         times_chi<kCM, T>(a, ec, wr, wi);
-    } else if (a.table) {
+    } else if (kPlain || a.table) {
         const int i = (int)cls * a.nelem + (a.nelem == 1 ? 0 : ec);
         if (kCM) {
             const typename V2<T>::t v = ((const typename V2<T>::t*)tab)[i];
@@ -268,7 +268,7 @@ __device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab,
         class_amp<T>(a, cls, wr, wi);
         times_chi<kCM, T>(a, ec, wr, wi);
     }
-    if (sign) {
+    if (!kPlain && sign) {
         wr = -wr;
         wi = -wi;
     }
@@ -337,7 +337,10 @@ QS_HD size_t mv_table_bytes(int entries, bool cm, size_t real) {
     return ((size_t)entries * real * (cm ? 2 : 1) + 15) / 16 * 16;
 }
 
-template <typename U, int kMode, bool kCM, bool kCV, typename T>
+// kPlain: every program by its masks with a state-independent sign, the values
+// staged and the particle number kept: what exchange couplings and transverse
+// fields need, without the flags' tests on every transition.
+template <typename U, int kMode, bool kCM, bool kCV, typename T, bool kPlain>
 __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
     constexpr bool kSym = kMode >= 2;
     constexpr bool k32 = sizeof(U) == 4;
@@ -373,10 +376,10 @@ __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
                 load_row_progs(sm, R, c0);
                 __syncthreads();
             }
-            row_hops<U>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
+            row_hops<U, !kPlain>(sm, R, min(kRowChunk, R.nprog - c0), valid, s, [&](int i, U t, int sign) {
                 const uint32_t cls = sm.cls[i];
                 T wr = 0, wi = 0;
-                if (a.any_chars && cls == kCharsClass) {
+                if (!kPlain && a.any_chars && cls == kCharsClass) {
                     U tc;
                     double dr, di;
                     if (!run_chars<U>(a, c0 + i, s, tc, dr, di)) return;
@@ -384,13 +387,13 @@ __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
                     wr = (T)dr;
                     wi = (T)di;
                 }
-                if (kMode != 0 && R.check_weight && __popcll((unsigned long long)t) != a.nup) return;
+                if (!kPlain && kMode != 0 && R.check_weight && __popcll((unsigned long long)t) != a.nup) return;
                 U m = t;
                 int ec = 0, st = 1;
                 if (kSym) row_orbit<U>(R, g, t, m, ec, st);
                 const int64_t idx = row_column<U, kMode>(R, spl, rtab, m);
                 if (kSym && idx < 0) return;
-                add_transition<kCM, kCV, T>(a, dyn, cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
+                add_transition<kCM, kCV, T, kPlain>(a, dyn, cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
             });
         }
         if (valid) store_row<kSym, kCM, kCV, T>(a, r, acc_r, acc_i);
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(kMvThreads) matvec_warp_rank_kernel(MvArgs a) 
             const int64_t idx = rank_warp<U>((const U*)R.reps, a.n, spl, (int)R.nsplit, R.stride, m, alive);
             if (!alive || idx < 0) continue;
             const int sign = __popcll((unsigned long long)(s & (U)p.zy)) & 1;
-            add_transition<kCM, kCV, T>(a, dyn, p.cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
+            add_transition<kCM, kCV, T, false>(a, dyn, p.cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
         }
         if (rv) store_row<true, kCM, kCV, T>(a, r, acc_r, acc_i);
     }
@@ -701,9 +704,20 @@ void launch_mode(const MvArgs& a, bool cm, bool cv, cudaStream_t s) {
     const bool ranks = sizeof(U) == 4 && (kMode == 1 || kMode == 3);
     const size_t dyn = (a.table ? mv_table_bytes(a.nclass * a.nelem, cm, sizeof(T)) : 0) +
                        (ranks ? (size_t)a.row.rank.size * sizeof(uint32_t) : 0);
-    if (cm) launch_rows(matvec_kernel<U, kMode, true, true, T>, grid, threads, dyn, s, a);
-    else if (cv) launch_rows(matvec_kernel<U, kMode, false, true, T>, grid, threads, dyn, s, a);
-    else launch_rows(matvec_kernel<U, kMode, false, false, T>, grid, threads, dyn, s, a);
+#define QS_ROWS(P_)                                                                                       \
+    do {                                                                                                   \
+        if (cm) launch_rows(matvec_kernel<U, kMode, true, true, T, P_>, grid, threads, dyn, s, a);         \
+        else if (cv) launch_rows(matvec_kernel<U, kMode, false, true, T, P_>, grid, threads, dyn, s, a);   \
+        else launch_rows(matvec_kernel<U, kMode, false, false, T, P_>, grid, threads, dyn, s, a);          \
+    } while (0)
+    if constexpr (sizeof(U) == 4 && (kMode == 1 || kMode == 3)) {
+        if (a.table && !a.any_chars && !a.row.any_zy && !a.row.check_weight) {
+            QS_ROWS(true);
+            return;
+        }
+    }
+    QS_ROWS(false);
+#undef QS_ROWS
 }
 
 // QS_RANK_MODE picks the rank lookup of a symmetric sector's generated states

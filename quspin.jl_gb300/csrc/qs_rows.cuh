@@ -49,8 +49,13 @@ struct RowArgs {
 RowArgs op_row_args(const Op& op, bool bwd);
 
 template <typename U>
+struct RowTest {
+    U care, value;
+};
+template <typename U>
 struct RowSmem {
-    U care[kRowChunk], value[kRowChunk], flip[kRowChunk], zy[kRowChunk];
+    RowTest<U> test[kRowChunk];   // one 8- or 16-byte read per test
+    U flip[kRowChunk], zy[kRowChunk];
     uint32_t cls[kRowChunk];
     uint32_t live[kRowChunk / 32][kRowThreads];
 };
@@ -61,8 +66,7 @@ __device__ __forceinline__ void load_row_progs(RowSmem<U>& sm, const RowArgs& a,
     const int nc = min(kRowChunk, a.nprog - c0);
     for (int i = threadIdx.x; i < nc; i += blockDim.x) {
         const RowProg p = a.progs[c0 + i];
-        sm.care[i] = (U)p.care;
-        sm.value[i] = (U)p.value;
+        sm.test[i] = RowTest<U>{(U)p.care, (U)p.value};
         sm.flip[i] = (U)p.flip;
         sm.zy[i] = (U)p.zy;
         sm.cls[i] = p.cls;
@@ -82,17 +86,19 @@ __device__ __forceinline__ void load_row_progs(RowSmem<U>& sm, const RowArgs& a,
 struct WinBase {
     uint32_t hi, lo;
     uint32_t mn, mx;
-    int gmn, gmx;   // groups of eight windows that hold them first
+    int gmn, gmx;   // groups of eight windows that hold them first (kJ)
 };
 
+// t's L bits repeated from the top of hi, through lo
 __device__ __forceinline__ void win_periodic(uint32_t t, int L, uint32_t& hi, uint32_t& lo) {
-    unsigned long long e = (unsigned long long)t << (64 - L);
-    for (int w = L; w < 64; w <<= 1) e |= e >> w;
-    hi = (uint32_t)(e >> 32);
-    lo = (uint32_t)e;
+    hi = t << (32 - L);
+    for (int w = L; w < 32; w <<= 1) hi |= hi >> w;
+    // the string's bit 32 + i is its bit 32 - L + i
+    lo = hi << (32 - L);
+    for (int w = L; w < 32; w <<= 1) lo |= lo >> w;
 }
 
-template <bool kFlip>
+template <bool kFlip, bool kJ>
 __device__ __forceinline__ void win_scan(WinBase& b, int L) {
     b.mn = 0xffffffffu;
     b.mx = 0u;
@@ -103,26 +109,83 @@ __device__ __forceinline__ void win_scan(WinBase& b, int L) {
         uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) w[i] = __funnelshift_l(b.lo, b.hi, 8 * g + i);
-        const uint32_t m = __vimin3_u32(__vimin3_u32(w[0], w[1], w[2]), __vimin3_u32(w[3], w[4], w[5]), min(w[6], w[7]));
-        if (m < b.mn) b.gmn = g;
-        b.mn = min(b.mn, m);
-        if (kFlip) {
-            const uint32_t x = __vimax3_u32(__vimax3_u32(w[0], w[1], w[2]), __vimax3_u32(w[3], w[4], w[5]), max(w[6], w[7]));
+        if (kJ) {
+            const uint32_t m =
+                __vimin3_u32(__vimin3_u32(w[0], w[1], w[2]), __vimin3_u32(w[3], w[4], w[5]), min(w[6], w[7]));
+            if (m < b.mn) b.gmn = g;
+            b.mn = min(b.mn, m);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) b.mn = __vimin3_u32(b.mn, w[i], w[i + 1]);
+        }
+        if (kFlip && kJ) {
+            const uint32_t x =
+                __vimax3_u32(__vimax3_u32(w[0], w[1], w[2]), __vimax3_u32(w[3], w[4], w[5]), max(w[6], w[7]));
             if (x > b.mx) b.gmx = g;
             b.mx = max(b.mx, x);
+        } else if (kFlip) {
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) b.mx = __vimax3_u32(b.mx, w[i], w[i + 1]);
         }
     }
 }
 
-// elem = (r * 2 + f) * nT + j as orbit_min_fast numbers the elements (j = 0 when
-// the characters do not depend on it), the first in that order among the
-// elements that reach the minimum; stab = their number.
-__device__ __forceinline__ void orbit_min_win(const FastGroup& G, uint32_t t, uint32_t& best, int& elem, int& stab) {
+// elem = (r * 2 + f) * nT + j as orbit_min_fast numbers the elements (j = 0
+// without kJ: the characters do not depend on it), the first in that order
+// among the elements that reach the minimum; stab = their number.
+template <bool kFlip, bool kJ>
+__device__ __forceinline__ void orbit_min_bases(const FastGroup& G, uint32_t t, uint32_t& best, int& elem, int& stab) {
     const int L = G.L;
-    const uint32_t lm = (uint32_t)G.lmask;
+    WinBase b[2];
+    win_periodic(t, L, b[0].hi, b[0].lo);
+    win_scan<kFlip, kJ>(b[0], L);
+    uint32_t w = b[0].mn;
+    int q = 0, g = b[0].gmn, n = 1;
+    auto take = [&](uint32_t c, int code, int grp) {
+        if (c == w) ++n;
+        if (c < w) {
+            w = c;
+            q = code;
+            if (kJ) g = grp;
+            n = 1;
+        }
+    };
+    if (kFlip) take(~b[0].mx, 1, b[0].gmx);
+    if (G.has_refl) {
+        win_periodic(__brev(t) >> (32 - L), L, b[1].hi, b[1].lo);
+        win_scan<kFlip, kJ>(b[1], L);
+        take(b[1].mn, 2, b[1].gmn);
+        if (kFlip) take(~b[1].mx, 3, b[1].gmx);
+    }
+    best = w >> (32 - L);
+    // rotations that fix the state (the same number from every base)
+    bool sym = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (i < G.nper) sym |= __funnelshift_l(b[0].lo, b[0].hi, G.per[i]) == b[0].hi;
+    if (sym) {
+        int c = 1;
+        for (int j = 1; j < L; ++j) c += __funnelshift_l(b[0].lo, b[0].hi, j) == b[0].hi;
+        n *= c;
+    }
+    stab = n;
+    elem = q * G.nT;
+    if (kJ) {
+        const uint32_t hi = (q & 2) ? b[1].hi : b[0].hi, lo = (q & 2) ? b[1].lo : b[0].lo;
+        const uint32_t target = (q & 1) ? ~w : w;
+        int j = 0;
+#pragma unroll
+        for (int i = 7; i >= 0; --i)
+            if (__funnelshift_l(lo, hi, 8 * g + i) == target) j = i;
+        elem += 8 * g + j;
+    }
+}
+
+__device__ __forceinline__ void orbit_min_win(const FastGroup& G, uint32_t t, uint32_t& best, int& elem, int& stab) {
     if (G.win == 2) {   // no translations
-        const uint32_t tr = __brev(t) >> (32 - L);
-        uint32_t c[4] = {t, ~t & lm, tr, ~tr & lm};
+        const uint32_t lm = (uint32_t)G.lmask;
+        const uint32_t tr = __brev(t) >> (32 - G.L);
+        const uint32_t c[4] = {t, ~t & lm, tr, ~tr & lm};
         best = t;
         elem = 0;
         stab = 1;
@@ -139,50 +202,12 @@ __device__ __forceinline__ void orbit_min_win(const FastGroup& G, uint32_t t, ui
         }
         return;
     }
-    WinBase b[2];
-    win_periodic(t, L, b[0].hi, b[0].lo);
-    if (G.has_flip) win_scan<true>(b[0], L);
-    else win_scan<false>(b[0], L);
-    uint32_t w = b[0].mn;
-    int q = 0, g = b[0].gmn, n = 1;
-    auto take = [&](uint32_t c, int code, int grp) {
-        if (c < w) {
-            w = c;
-            q = code;
-            g = grp;
-            n = 1;
-        } else if (c == w) {
-            ++n;
-        }
-    };
-    if (G.has_flip) take(~b[0].mx, 1, b[0].gmx);
-    if (G.has_refl) {
-        win_periodic(__brev(t) >> (32 - L), L, b[1].hi, b[1].lo);
-        if (G.has_flip) win_scan<true>(b[1], L);
-        else win_scan<false>(b[1], L);
-        take(b[1].mn, 2, b[1].gmn);
-        if (G.has_flip) take(~b[1].mx, 3, b[1].gmx);
-    }
-    best = w >> (32 - L);
-    // rotations that fix the state (the same number from every base)
-    bool sym = false;
-    for (int i = 0; i < G.nper; ++i) sym |= __funnelshift_l(b[0].lo, b[0].hi, G.per[i]) == b[0].hi;
-    if (sym) {
-        int c = 1;
-        for (int j = 1; j < L; ++j) c += __funnelshift_l(b[0].lo, b[0].hi, j) == b[0].hi;
-        n *= c;
-    }
-    stab = n;
-    elem = q * G.nT;
     if (G.need_j) {
-        const uint32_t hi = (q & 2) ? b[1].hi : b[0].hi, lo = (q & 2) ? b[1].lo : b[0].lo;
-        const uint32_t target = (q & 1) ? ~w : w;
-        int j = 8 * g;
-#pragma unroll
-        for (int i = 7; i >= 1; --i)
-            if (__funnelshift_l(lo, hi, 8 * g + i) == target) j = 8 * g + i;
-        if (__funnelshift_l(lo, hi, 8 * g) == target) j = 8 * g;
-        elem += j;
+        if (G.has_flip) orbit_min_bases<true, true>(G, t, best, elem, stab);
+        else orbit_min_bases<false, true>(G, t, best, elem, stab);
+    } else {
+        if (G.has_flip) orbit_min_bases<true, false>(G, t, best, elem, stab);
+        else orbit_min_bases<false, false>(G, t, best, elem, stab);
     }
 }
 
@@ -234,8 +259,9 @@ __device__ __forceinline__ int64_t row_column(const RowArgs& a, const U* spl, co
 }
 
 // Walks the live programs of the chunk [c0, c0 + nc) on state s: one call of
-// hop(i, t, sign) per live program i of the chunk, ascending.
-template <typename U, class Hop>
+// hop(i, t, sign) per live program i of the chunk, ascending.  kSign: some sign
+// depends on the state.
+template <typename U, bool kSign, class Hop>
 __device__ __forceinline__ void row_hops(RowSmem<U>& sm, const RowArgs& a, int nc, bool valid, U s, Hop hop) {
     const int nw = (nc + 31) >> 5;
     for (int w = 0; w < nw; ++w) {
@@ -243,11 +269,15 @@ __device__ __forceinline__ void row_hops(RowSmem<U>& sm, const RowArgs& a, int n
         const int k1 = min(32, nc - 32 * w);
         if (k1 == 32) {
 #pragma unroll 8
-            for (int i = 0; i < 32; ++i)
-                if ((s & sm.care[32 * w + i]) == sm.value[32 * w + i]) bits |= 1u << i;
+            for (int i = 0; i < 32; ++i) {
+                const RowTest<U> q = sm.test[32 * w + i];
+                if ((s & q.care) == q.value) bits |= 1u << i;
+            }
         } else {
-            for (int i = 0; i < k1; ++i)
-                if ((s & sm.care[32 * w + i]) == sm.value[32 * w + i]) bits |= 1u << i;
+            for (int i = 0; i < k1; ++i) {
+                const RowTest<U> q = sm.test[32 * w + i];
+                if ((s & q.care) == q.value) bits |= 1u << i;
+            }
         }
         sm.live[w][threadIdx.x] = valid ? bits : 0u;
     }
@@ -259,7 +289,7 @@ __device__ __forceinline__ void row_hops(RowSmem<U>& sm, const RowArgs& a, int n
         const int i = 32 * w + __ffs((int)cur) - 1;
         cur &= cur - 1u;
         int sign = 0;
-        if (a.any_zy)
+        if (kSign && a.any_zy)
             sign = (sizeof(U) == 8 ? __popcll((unsigned long long)(s & sm.zy[i])) : __popc((unsigned)(s & sm.zy[i]))) & 1;
         hop(i, (U)(s ^ sm.flip[i]), sign);
     }
