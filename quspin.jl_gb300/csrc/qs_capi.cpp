@@ -367,7 +367,8 @@ int qs_op_matvec(qs_op* op, int32_t flags, const double* alpha, const void* x, i
             // next computes; otherwise one product and one read-back
             if (!qs::op_matvec_host_overlap(o, c, ys, yb)) {
                 qs::op_matvec_device(o, c, o.stream);
-                qs::copy_to_host(ys, o.d_y.p, n * yb, o.stream);
+                if (beta_zero) qs::touch_host(ys, n * yb);   // (with beta the caller's y is already there)
+                QS_CUDA(cudaMemcpyAsync(ys, o.d_y.p, n * yb, cudaMemcpyDeviceToHost, o.stream));
             }
             QS_CUDA(cudaStreamSynchronize(o.stream));
         }
