@@ -973,7 +973,7 @@ def profile_range(kind):
                 "matrixfree": "fp64"}[kind]
         x = np.random.default_rng(20261203).standard_normal(b.Ns)
         # device buffers (what the bench times): one launch is one full-range
-        # product; the warm-up products time the kernel variants first
+        # product
         import ctypes
         from qsgpu import _lib
         lib = _lib.load()

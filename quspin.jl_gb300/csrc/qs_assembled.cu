@@ -1239,42 +1239,38 @@ __global__ void __launch_bounds__(kThreads, MINB) sell_fx_kernel(SellArgs a, FxA
     }
 }
 
-// the fixed-point product's variants (gathers in flight, resident blocks):
+// the fixed-point product's two shapes (gathers in flight, resident blocks):
 // complex vectors and four classes hold more accumulators, so fewer blocks
 template <bool kCV, bool kPacked, int NC>
 void launch_fx(int v, int grid, cudaStream_t s, const SellArgs& a, const FxArgs& f) {
     constexpr int B0 = kCV ? 4 : (NC <= 2 ? 8 : 6);
-    constexpr int B1 = (kCV || NC > 2) ? 4 : 6;
-    switch (v) {
-        case 0: sell_fx_kernel<kCV, kPacked, NC, 1, B0, false><<<grid, kThreads, 0, s>>>(a, f); break;
-        case 1: sell_fx_kernel<kCV, kPacked, NC, 2, B1, false><<<grid, kThreads, 0, s>>>(a, f); break;
-        case 2: sell_fx_kernel<kCV, kPacked, NC, 4, 4, false><<<grid, kThreads, 0, s>>>(a, f); break;
-        case 3: sell_fx_kernel<kCV, kPacked, NC, 1, B0, true><<<grid, kThreads, 0, s>>>(a, f); break;
-        case 4: sell_fx_kernel<kCV, kPacked, NC, 2, B1, true><<<grid, kThreads, 0, s>>>(a, f); break;
-        default: sell_fx_kernel<kCV, kPacked, NC, 4, 4, true><<<grid, kThreads, 0, s>>>(a, f); break;
-    }
+    if (v == 0) sell_fx_kernel<kCV, kPacked, NC, 1, B0, false><<<grid, kThreads, 0, s>>>(a, f);
+    else sell_fx_kernel<kCV, kPacked, NC, 4, 4, true><<<grid, kThreads, 0, s>>>(a, f);
 }
 
-// six sliced-ELL variants: three (gathers in flight, blocks per SM) shapes,
-// each with plain loads and with the evict-first / evict-last hints
-constexpr int kSellVariants = 6;
-
-// QS_TUNE_VERBOSE=1 prints the variant timings of each tuning to stderr
-bool tune_verbose() {
-    static const bool on = [] {
-        const char* e = std::getenv("QS_TUNE_VERBOSE");
-        return e && e[0] && e[0] != '0';
-    }();
-    return on;
-}
-
-// QS_SELL_VARIANT=v (0 .. kSellVariants - 1) runs variant v instead of the
-// timed choice (read on every product; the tests run every variant with it)
-int forced_variant() {
+// Two shapes of every sliced-ELL product: 0 narrow (one gather in flight a
+// thread, eight blocks an SM), 1 wide (four gathers, four blocks), both with the
+// word stream evict-first and the x gathers evict-last (the fixed-point form's
+// narrow shape without).  Same bits; chosen by the rows and their mean length:
+//  - wide for rows of 16 transitions or more: 4.7 M rows of 33, FP64 0.350 ms
+//    against 0.366, FP32 0.203 / 0.222, double-float 0.301 / 0.328; 101,340 rows
+//    of 27, FP64 13.2 / 15.9 us; 208,012 complex rows 62 / 60;
+//  - narrow for FP64 products of complex matrices from 100,000 rows on (400,664
+//    rows of 26: 90.6 against 95.5 us; 742,900: 193 / 206; 32,065 rows 17.3 /
+//    15.2): FP64-pipe bound, four multiply-adds a transition;
+//  - narrow for short rows from a million on, whose four gathers leave a warp
+//    mostly remainders: 10.4 M rows of 13.5, FP64 0.396 / 0.428, FP32 0.188 /
+//    0.258 ms; 705,432 rows of 11.5 are equal, 48,620 rows 9.2 / 7.7 us;
+//  - fixed point: narrow from 200,000 rows on (4.7 M rows 0.251 / 0.297 ms,
+//    361,270 rows equal), wide below (101,340 rows 12.5 / 11.1 us).
+int sell_variant(bool fixed_point, bool complex64, int64_t n, int64_t nnz) {
+    // QS_SELL_VARIANT=v runs shape v mod 2 (read on every product; the tests
+    // run both with it)
     const char* e = std::getenv("QS_SELL_VARIANT");
-    if (!e || !e[0]) return -1;
-    const int v = std::atoi(e);
-    return (v >= 0 && v < kSellVariants) ? v : -1;
+    if (e && e[0] >= '0' && e[0] <= '9') return std::atoi(e) & 1;
+    if (fixed_point) return n < 200000;
+    if (complex64 && n >= 100000) return 0;
+    return !(n >= 1000000 && nnz < 16 * n);
 }
 
 int grid_rows(int64_t threads_needed) {
@@ -1600,18 +1596,10 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
         a.y = c.y;
         const bool cm = op.complex_mat, cv = c.y_complex;
         const int grid = grid_rows(std::max<int64_t>(1, a.nslices - a.slice0) * kSlice);
-        // variants: (gathers in flight per thread, resident blocks per SM) x
-        // (plain loads, or the word stream evict-first and x evict-last)
-#define QS_VARIANTS(LAUNCH, v)                         \
-    do {                                               \
-        switch (v) {                                   \
-            case 0: LAUNCH(1, 8, false); break;        \
-            case 1: LAUNCH(2, 6, false); break;        \
-            case 2: LAUNCH(4, 4, false); break;        \
-            case 3: LAUNCH(1, 8, true); break;         \
-            case 4: LAUNCH(2, 6, true); break;         \
-            default: LAUNCH(4, 4, true); break;        \
-        }                                              \
+#define QS_VARIANTS(LAUNCH, v)            \
+    do {                                  \
+        if ((v) == 0) LAUNCH(1, 8, true); \
+        else LAUNCH(4, 4, true);          \
     } while (0)
 #define QS_SHAPES(K, U_, B_, H_, ...)                                                        \
     do {                                                                                     \
@@ -1625,11 +1613,9 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
             else K<false, false, false, U_, B_, H_><<<grid, kThreads, 0, s>>>(__VA_ARGS__);        \
         }                                                                                    \
     } while (0)
-        int kind;
         std::function<void(int)> launch;
         const float4* td = M.table_df.as<float4>();
         if (c.df_io) {
-            kind = 3;
             const float4* dd = op.d_diag_df.as<float4>();
             const float2* rq = M.rsq_df.as<float2>();
             launch = [&, td, dd, rq](int v) {
@@ -1638,7 +1624,6 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
 #undef L_DFIO
             };
         } else if (c.fx && !c.single && M.fx_classes > 0) {
-            kind = 4;
             a.table = M.table64.p;
             a.diag = op.d_diag.p;
             a.diag_re = op.d_diag_re.p;
@@ -1676,7 +1661,6 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
                 }
             };
         } else if (c.df && !c.single) {
-            kind = 2;
             a.table = M.table64.p;
             a.diag = op.d_diag.p;
             a.diag_re = op.d_diag_re.p;
@@ -1692,7 +1676,6 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
 #undef L_DF
             };
         } else if (c.single) {
-            kind = 1;
             a.table = M.table32.p;
             a.diag = op.d_diag32.p;
             a.diag_re = op.d_diag32_re.p;
@@ -1713,7 +1696,6 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
 #undef L_32
             };
         } else {
-            kind = 0;
             a.table = M.table64.p;
             a.diag = op.d_diag.p;
             a.diag_re = op.d_diag_re.p;
@@ -1736,47 +1718,8 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
         }
 #undef QS_SHAPES
 #undef QS_VARIANTS
-        int& var = op.asm_.sell_variant[kind];
-        if (var < 0 && !c.no_tune && forced_variant() < 0) {
-            // choose the variant by timing, when repeating the product is harmless
-            // (beta = 0) and the stream is not being captured into a graph
-            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            QS_CUDA(cudaStreamIsCapturing(s, &cap));
-            if (a.beta_zero && cap == cudaStreamCaptureStatusNone) {
-                cudaEvent_t e0, e1;
-                QS_CUDA(cudaEventCreate(&e0));
-                QS_CUDA(cudaEventCreate(&e1));
-                float best = 1e30f;
-                int bv = 2;
-                float ms_v[kSellVariants] = {};
-                for (int v = 0; v < kSellVariants; ++v) {
-                    launch(v);
-                    QS_CUDA(cudaGetLastError());
-                    QS_CUDA(cudaEventRecord(e0, s));
-                    for (int r = 0; r < 3; ++r) launch(v);
-                    QS_CUDA(cudaEventRecord(e1, s));
-                    QS_CUDA(cudaEventSynchronize(e1));
-                    float ms = 0;
-                    QS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                    ms_v[v] = ms / 3;
-                    if (ms < best) {
-                        best = ms;
-                        bv = v;
-                    }
-                }
-                cudaEventDestroy(e0);
-                cudaEventDestroy(e1);
-                note_launches(4 * kSellVariants);
-                if (tune_verbose()) {
-                    std::fprintf(stderr, "qsgpu: sliced-ELL product kind %d, n=%lld: variant ms", kind, (long long)b.n);
-                    for (int v = 0; v < kSellVariants; ++v) std::fprintf(stderr, " %d:%.4f", v, ms_v[v]);
-                    std::fprintf(stderr, " -> %d\n", bv);
-                }
-                var = bv;
-            }
-        }
-        const int fv = forced_variant();
-        launch(fv >= 0 ? fv : (var < 0 ? 2 : var));
+        launch(sell_variant(c.fx && !c.single && M.fx_classes > 0 && !c.df_io, cm && !c.single && !c.df && !c.df_io, b.n,
+                            M.nnz));
         QS_CUDA(cudaGetLastError());
         note_launches(1);
         return;
@@ -2051,8 +1994,6 @@ bool op_matvec_host_overlap(Op& op, const MatvecCall& c0, void* y_host, size_t e
     if (!op.commuting || !op.assembled || !M.has_sell || (T && !op.hermitian) || (c0.df && !fx) || c0.df_io)
         return false;
     if (!(c0.beta.re == 0.0 && c0.beta.im == 0.0)) return false;   // y is not read
-    // the first product of a kind times the kernel variants on the full range
-    if (M.sell_variant[fx ? 4 : (c0.single ? 1 : 0)] < 0) return false;
     constexpr int K = 4;
     if (M.nslices < 4 * K) return false;
     if (!op.copy_stream) {

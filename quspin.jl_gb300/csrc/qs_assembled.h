@@ -166,11 +166,6 @@ struct Assembled {
     DevBuf fx_amp;      // double per class: A_c
     DevBuf fx_sq;       // double sqrt(i), i = 0 .. kMaxGroup
     DevBuf fx_max;      // uint64: max |x_j sqrt(stab_j)| of the current product (bit pattern), then per-block maxima
-    // sliced-ELL kernel variant (gathers in flight x resident blocks) per
-    // product kind (FP64, FP32, double-float with FP64 vectors, double-float
-    // vectors, fixed-point row sums), chosen by timing on the first product
-    // that allows it (-1: not yet)
-    int sell_variant[5] = {-1, -1, -1, -1, -1};
 };
 
 }  // namespace qs

@@ -81,13 +81,13 @@ void pool_trim();
 // Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister,
 // mapped under unified addressing), or null for any other pointer.
 void* mapped_host_address(void* p);
-// Writes one byte of every page of a caller's output back to itself, so that
-// the pages exist before a device copy lands in them.  A copy into untouched
-// pages faults them in one by one from the device: 17 ms for 21 MB on a GB300's
-// Grace host, against 1 ms for the touches and 0.17 ms for the copy (np.zeros
-// and malloc hand out such pages).
+// Writes a zero into every page of a caller's output that is about to be
+// overwritten whole, so that the pages exist before a device copy lands in them.  A copy into heap pages that
+// no one has touched faults them in one by one from the device: 17 ms for 21 MB
+// on a GB300's Grace host, against 1 ms for the touches and 0.17 ms for the
+// copy (malloc hands out such pages after it has trimmed its heap).
 void touch_host(void* p, size_t bytes);
-// Touches dst, then copies device memory into it on s.
+// touch_host(dst), then the copy of device memory into it on s.
 void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 struct PoolBuf {
@@ -273,7 +273,6 @@ struct MatvecCall {
     bool df_io = false;             // double-float vectors in and out, alpha = 1, beta = 0
     bool fx = false;                // FP64 vectors, exact fixed-point row sums where the operator allows
     bool fx_ready = false;          // the scaled integer copy of x is already made (later row ranges)
-    bool no_tune = false;           // never time kernel variants inside this call
     int64_t slice0 = 0, slice1 = -1; // sliced-ELL slices [slice0, slice1) only (-1: to the end)
 };
 void op_prepare_device(Op& op);

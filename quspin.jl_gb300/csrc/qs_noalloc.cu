@@ -88,7 +88,6 @@ void op_matvec_noalloc(Op& op, int flags, cplx alpha, const void* x, int x_dtype
                                          std::to_string(vb) + " bytes (use qs_op_matvec)");
     unsigned char* stage = stage_address();
     MatvecCall c;
-    c.no_tune = true;   // variant timing would create events
     // the same flag meaning as qs_op_matvec: double-float products and
     // fixed-point row sums use tables and scratch that assembly allocated
     c.flags = flags & (QS_TRANSPOSE | QS_CONJUGATE);

@@ -529,7 +529,6 @@ void engine_loop(Server& S) {
             c.x = xq;
             c.y = Ax.p;
             c.x_complex = c.y_complex = q.cv;
-            c.no_tune = true;   // the operator may be stepping on the other lane
             op_matvec_device(op, c, s1);
             th[i] = B.dot(xq, Ax.p).real();
             B.axpy(Ax.p, xq, cd(-th[i], 0));
