@@ -2106,6 +2106,15 @@ void Engine::store(int id, int col, double* out, bool device) {
     QS_CUDA(cudaStreamSynchronize(s_));
 }
 
+void Engine::copy_column(int src, int scol, int dst, int dcol) {
+    const SlotDev &a = slots_[src].d, &b = slots_[dst].d;
+    if (a.n != b.n || a.cv != b.cv || scol < 0 || scol > a.m || dcol < 0 || dcol > b.m)
+        throw Error(QS_ERR_ARGUMENT, "column copy between slots of different shapes");
+    const size_t bytes = (size_t)a.n * store_bytes(st_, a.cv);
+    QS_CUDA(cudaMemcpyAsync((char*)b.V + dcol * bytes, (const char*)a.V + scol * bytes, bytes, cudaMemcpyDeviceToDevice,
+                            s_));
+}
+
 std::vector<double> Engine::normalize(const std::vector<int>& ids, int col, bool scale) {
     std::vector<int> saved(ids.size());
     for (size_t q = 0; q < ids.size(); ++q) {
@@ -2497,8 +2506,10 @@ void eigsh_batch(Op** ops, int nops, const qs_eigsh_opts& o, double* values, voi
 }
 
 // ================================================================ Krylov exponential
-void krylov_project(const std::vector<cd>& H, int m, bool hermitian, cd scale, int& c, std::vector<cd>& coef,
-                    double& terminal) {
+void KrylovFact::init(std::vector<cd> rec, int m_, bool herm) {
+    H = std::move(rec);
+    m = m_;
+    hermitian = herm;
     const int ld = m + 1;
     auto h = [&](int i, int j) { return H[(size_t)j * ld + i]; };
     // completed steps: the reference stops when the new norm is below
@@ -2519,25 +2530,32 @@ void krylov_project(const std::vector<cd>& H, int m, bool hermitian, cd scale, i
         }
     }
     terminal = std::abs(h(c, c - 1));
-    coef.assign(c, cd(0, 0));
     if (hermitian) {
-        std::vector<double> T((size_t)c * c, 0.0), w, U;
+        std::vector<double> T((size_t)c * c, 0.0);
         for (int i = 0; i < c; ++i) {
             T[(size_t)i * c + i] = h(i, i).real();
             if (i + 1 < c) T[(size_t)i * c + i + 1] = T[(size_t)(i + 1) * c + i] = h(i + 1, i).real();
         }
         sym_eig(c, T, w, U);
+    }
+}
+
+void KrylovFact::coef(cd scale, std::vector<cd>& out) const {
+    out.assign(c, cd(0, 0));
+    if (hermitian) {
+        std::vector<cd> g(c);
+        for (int q = 0; q < c; ++q) g[q] = std::exp(scale * w[q]) * U[q];
         for (int r = 0; r < c; ++r) {
             cd acc(0, 0);
-            for (int q = 0; q < c; ++q) acc += U[(size_t)r * c + q] * (std::exp(scale * w[q]) * U[q]);
-            coef[r] = acc;
+            for (int q = 0; q < c; ++q) acc += U[(size_t)r * c + q] * g[q];
+            out[r] = acc;
         }
     } else {
         std::vector<cd> A((size_t)c * c), E;
         for (int i = 0; i < c; ++i)
-            for (int j = 0; j < c; ++j) A[(size_t)i * c + j] = scale * h(i, j);
+            for (int j = 0; j < c; ++j) A[(size_t)i * c + j] = scale * H[(size_t)j * (m + 1) + i];
         expm_complex(c, A, E);
-        for (int r = 0; r < c; ++r) coef[r] = E[(size_t)r * c];
+        for (int r = 0; r < c; ++r) out[r] = E[(size_t)r * c];
     }
 }
 
@@ -2560,25 +2578,40 @@ void EvoTask::init(int m_, int64_t n_, bool herm, cd scale, double tol, double b
 }
 
 void EvoTask::on_hold(const std::vector<cd>& Hrec, int id, RotReq& rot) {
-    H = Hrec;
-    project(id, rot);
+    fact.init(Hrec, m, hermitian);
+    project(fact, id, rot);
 }
 
-void EvoTask::project(int id, RotReq& rot) {
-    const Seg sg = segs.front();
-    int c;
+void EvoTask::project(const KrylovFact& F, int id, RotReq& rot) {
     std::vector<cd> coef;
-    double terminal;
-    krylov_project(H, m, hermitian, sg.scale, c, coef, terminal);
+    while (true) {
+        const Seg sg = segs.front();
+        F.coef(sg.scale, coef);
+        const bool est_on = F.c == m && m < n;
+        err = est_on ? std::abs(sg.scale) * F.terminal * beta * std::abs(coef[F.c - 1]) : 0.0;
+        // the candidate's norm is at most beta times the sum of its coefficients'
+        // magnitudes (unit columns): a step whose error is past the bound for
+        // that norm fails without being formed
+        double top = 0.0;
+        for (const cd& v : coef) top += std::abs(v);
+        if (err <= sg.tol * std::max(1.0, 1.001 * beta * top) || sg.depth >= 14) break;
+        split_front();
+    }
     rot = RotReq();
     rot.id = id;
-    rot.nin = c;
+    rot.nin = F.c;
     rot.p = 1;
     rot.out0 = m;   // the candidate goes to column m; column 0 keeps the segment's start
-    rot.Y.resize(c);
-    for (int i = 0; i < c; ++i) rot.Y[i] = coef[i] * beta;
-    const bool est_on = c == m && m < n;
-    err = est_on ? std::abs(sg.scale) * terminal * beta * std::abs(coef[c - 1]) : 0.0;
+    rot.Y.resize(F.c);
+    for (int i = 0; i < F.c; ++i) rot.Y[i] = coef[i] * beta;
+}
+
+void EvoTask::split_front() {
+    const Seg sg = segs.front();
+    segs.pop_front();
+    segs.push_front(Seg{sg.scale / 2.0, sg.tol / 2, sg.depth + 1});
+    segs.push_front(Seg{sg.scale / 2.0, sg.tol / 2, sg.depth + 1});
+    ++halvings;
 }
 
 int EvoTask::after_norm(double nr, int id, RotReq& copy) {
@@ -2593,66 +2626,119 @@ int EvoTask::after_norm(double nr, int id, RotReq& copy) {
         return 1;
     }
     if (sg.depth >= 14) return -1;
-    segs.pop_front();
-    segs.push_front(Seg{sg.scale / 2.0, sg.tol / 2, sg.depth + 1});
-    segs.push_front(Seg{sg.scale / 2.0, sg.tol / 2, sg.depth + 1});
-    ++halvings;
+    split_front();
     return 0;
 }
 
-// Runs EvoTasks on their slots until all are done; out_cols[i] receives
-// beta * column 0 (host, Ns complex) of task i.
-// Runs the EvoTasks of the listed slots to completion and writes beta * the
-// accepted state of each to outs (host, or device with `device`).  Slots may
-// have different Krylov sizes (different operators).
-static void run_evo_slots(Engine& E, std::vector<int>& ids, std::vector<EvoTask>& tasks,
-                          const std::vector<double*>& outs, bool device = false) {
+// Runs the EvoTasks to completion and writes beta * the final state of each to
+// outs (host, or device with `device`).  ids[i]: a slot of task i's own; the
+// slots may have different Krylov sizes (different operators).
+//
+// Tasks whose states are the same share them: a state is known by the slot
+// that holds it in column 0, one factorisation from it serves every task that
+// is there, and tasks part only where they accept different steps (each new
+// state moves to the own slot of one of its tasks).  The engine is
+// deterministic, so a shared state is the state each task would have computed,
+// bit for bit: on an even grid of ten times most first steps are common, and
+// the evolution of 96,909 rows to t = 2 takes 28 factorisations instead of 46.
+// roots (with facts): the slot whose factorised column 0 task i starts from;
+// without, task i's start is in column 0 of its own slot.
+static void run_evo_slots(Engine& E, const std::vector<int>& ids, std::vector<EvoTask>& tasks,
+                          const std::vector<double*>& outs, bool device = false,
+                          const std::vector<int>& roots = {}, const std::map<int, const KrylovFact*>& root_facts = {}) {
     const size_t nt = tasks.size();
     std::vector<char> fin(nt, 0);
+    std::vector<int> at(nt);   // the slot that holds task i's state
     size_t left = 0;
-    for (size_t i = 0; i < nt; ++i) {
-        if (tasks[i].done()) fin[i] = 1;
-        else {
-            E.start(ids[i], 0);
-            ++left;
-        }
-    }
+    for (size_t i = 0; i < nt; ++i) at[i] = roots.empty() ? ids[i] : roots[i];
     auto emit = [&](size_t i) {
         const int64_t n = tasks[i].n;
-        const double b = tasks[i].beta;
+        const cd b(tasks[i].beta, 0);
         if (device) {
-            E.store(ids[i], 0, outs[i], true);
-            scale_c128(outs[i], outs[i], cd(b, 0), n, E.stream());
+            E.store(at[i], 0, outs[i], true);
+            scale_c128(outs[i], outs[i], b, n, E.stream());
             QS_CUDA(cudaStreamSynchronize(E.stream()));
             return;
         }
         // scaled on the device, then one copy
         PoolBuf col((size_t)n * 2 * sizeof(double), E.stream());
-        E.store(ids[i], 0, col.as<double>(), true);
-        scale_c128(col.p, col.p, cd(b, 0), n, E.stream());
+        E.store(at[i], 0, col.as<double>(), true);
+        scale_c128(col.p, col.p, b, n, E.stream());
         copy_to_host(outs[i], col.p, col.bytes, E.stream());
         QS_CUDA(cudaStreamSynchronize(E.stream()));
     };
-    for (size_t i = 0; i < nt; ++i)
-        if (fin[i]) emit(i);
-    while (left > 0) {
-        const int steps = E.steps_to_event();
-        if (steps <= 0) throw Error(QS_ERR_CUDA, "Krylov exponential lost its stepping slots");
-        E.run(steps);
-        std::vector<size_t> hold;
-        std::vector<int> hold_ids;
+    for (size_t i = 0; i < nt; ++i) {
+        if (!tasks[i].done()) {
+            ++left;
+            continue;
+        }
+        emit(i);
+        fin[i] = 1;
+    }
+    if (roots.empty())
         for (size_t i = 0; i < nt; ++i)
-            if (!fin[i] && E.slot(ids[i]).state == kSlotHold) {
-                hold.push_back(i);
-                hold_ids.push_back(ids[i]);
+            if (!fin[i]) E.start(at[i], 0);
+    bool first = !roots.empty();   // the roots' factorisations are ready
+    while (left > 0) {
+        // the states whose factorisation is ready, with their tasks
+        std::map<int, std::vector<size_t>> held;
+        std::map<int, KrylovFact> facts;
+        if (first) {
+            for (size_t i = 0; i < nt; ++i)
+                if (!fin[i]) held[at[i]].push_back(i);
+        } else {
+            const int steps = E.steps_to_event();
+            if (steps <= 0) throw Error(QS_ERR_CUDA, "Krylov exponential lost its stepping slots");
+            E.run(steps);
+            for (size_t i = 0; i < nt; ++i)
+                if (!fin[i] && E.slot(at[i]).state == kSlotHold) held[at[i]].push_back(i);
+            std::vector<int> hid;
+            for (const auto& kv : held) hid.push_back(kv.first);
+            std::vector<std::vector<cd>> H;
+            E.records(hid, H);
+            for (size_t q = 0; q < hid.size(); ++q) {
+                const EvoTask& t = tasks[held[hid[q]].front()];
+                facts[hid[q]].init(std::move(H[q]), t.m, t.hermitian);
             }
-        std::vector<std::vector<cd>> H;
-        E.records(hold_ids, H);
-        std::vector<RotReq> rot(hold.size());
-        for (size_t q = 0; q < hold.size(); ++q) tasks[hold[q]].on_hold(H[q], ids[hold[q]], rot[q]);
-        std::vector<size_t> proj = hold, done_now, restart;
-        // project, measure, decide; rejected slots project their half step from
-        // the same basis until every slot is accepted
+        }
+        struct Taken {
+            cd scale;
+            double nr;
+            int slot;
+        };
+        std::map<int, std::vector<Taken>> taken;   // the new states of each slot so far
+        std::map<int, size_t> next;                // the member whose step is being decided
+        std::vector<size_t> proj;
+        std::vector<RotReq> rot;
+        // the next step to form in slot s (column m), joining states that exist
+        auto propose = [&](int s) {
+            const std::vector<size_t>& M = held[s];
+            const KrylovFact& F = first ? *root_facts.at(s) : facts[s];
+            while (next[s] < M.size()) {
+                const size_t i = M[next[s]];
+                RotReq R;
+                tasks[i].project(F, s, R);
+                const Taken* same = nullptr;
+                for (const Taken& t : taken[s])
+                    if (t.scale == tasks[i].segs.front().scale) same = &t;
+                if (!same) {
+                    proj.push_back(i);
+                    rot.push_back(std::move(R));
+                    return;
+                }
+                RotReq unused;
+                const int r = tasks[i].after_norm(same->nr, s, unused);
+                if (r < 0)
+                    throw Error(QS_ERR_NOT_CONVERGED, "Krylov exponential action did not converge; increase krylov_dim");
+                if (r == 1) {
+                    at[i] = same->slot;
+                    ++next[s];
+                }
+            }
+        };
+        for (const auto& kv : held) propose(kv.first);
+        // project, measure, decide; rejected steps project their half from the
+        // same basis until every task's step is accepted
         while (!proj.empty()) {
             E.rotate(rot);
             // the candidates sit in column m of each slot: one normalisation per Krylov size
@@ -2661,40 +2747,72 @@ static void run_evo_slots(Engine& E, std::vector<int>& ids, std::vector<EvoTask>
             for (size_t q = 0; q < proj.size(); ++q) by_m[tasks[proj[q]].m].push_back(q);
             for (const auto& kv : by_m) {
                 std::vector<int> pid;
-                for (size_t q : kv.second) pid.push_back(ids[proj[q]]);
+                for (size_t q : kv.second) pid.push_back(rot[q].id);
                 const std::vector<double> g = E.normalize(pid, kv.first);
                 for (size_t t = 0; t < kv.second.size(); ++t) nr[kv.second[t]] = g[t];
             }
-            std::vector<RotReq> copies, next_rot;
-            std::vector<size_t> next;
+            std::vector<RotReq> copies;
+            std::vector<int> again;
             for (size_t q = 0; q < proj.size(); ++q) {
                 const size_t i = proj[q];
+                const int s = rot[q].id;
+                const cd scale = tasks[i].segs.front().scale;
                 RotReq cp;
-                const int r = tasks[i].after_norm(nr[q], ids[i], cp);
+                const int r = tasks[i].after_norm(nr[q], s, cp);
                 if (r < 0)
                     throw Error(QS_ERR_NOT_CONVERGED, "Krylov exponential action did not converge; increase krylov_dim");
                 if (r == 1) {
-                    copies.push_back(std::move(cp));
-                    (tasks[i].done() ? done_now : restart).push_back(i);
-                } else {
-                    RotReq R;
-                    tasks[i].project(ids[i], R);
-                    next_rot.push_back(std::move(R));
-                    next.push_back(i);
+                    // the new state goes to a slot of the same operator that holds
+                    // no unfinished task's state: there is one while another
+                    // member is undecided, as a group has at least as many
+                    // slots as states.  The last member may find none: its
+                    // state replaces the old one.
+                    int dst = -1;
+                    auto is_free = [&](int id) {
+                        if (&E.op(id) != &E.op(s) || E.slot(id).m != E.slot(s).m) return false;
+                        for (size_t k = 0; k < nt; ++k)
+                            if (!fin[k] && at[k] == id) return false;
+                        return true;
+                    };
+                    for (size_t k = 0; k < nt && dst < 0; ++k)
+                        if (is_free(ids[k])) dst = ids[k];
+                    if (dst < 0) {
+                        dst = s;
+                        copies.push_back(std::move(cp));
+                    } else {
+                        E.copy_column(s, tasks[i].m, dst, 0);
+                    }
+                    taken[s].push_back(Taken{scale, nr[q], dst});
+                    at[i] = dst;
+                    ++next[s];
                 }
+                again.push_back(s);
             }
             E.rotate(copies);
-            rot.swap(next_rot);
-            proj.swap(next);
+            proj.clear();
+            rot.clear();
+            for (int s : again) propose(s);
         }
-        for (size_t i : done_now) {
-            emit(i);
-            fin[i] = 1;
-            --left;
-            E.remove(ids[i]);
-        }
-        for (size_t i : restart) E.start(ids[i], 0);
+        // finished tasks, then a factorisation from every state that is left;
+        // slots without one wait (removing them would rebuild the block maps
+        // and recapture the step graph)
+        std::vector<int> used;
+        for (const auto& kv : held)
+            for (size_t i : kv.second) {
+                if (tasks[i].done()) {
+                    emit(i);
+                    fin[i] = 1;
+                    --left;
+                } else {
+                    used.push_back(at[i]);
+                }
+            }
+        for (const auto& kv : held) E.slot_mut(kv.first).state = kSlotIdle;
+        for (int s : used)
+            if (E.slot(s).state != kSlotStep) E.start(s, 0);
+        first = false;
     }
+    for (int id : ids) E.remove(id);
 }
 
 void evolve_engine(Op& op, const double* v0, const std::vector<cd>& scales, double tol, int krylov_dim, int precision,
@@ -2720,38 +2838,49 @@ void evolve_engine(Op& op, const double* v0, const std::vector<cd>& scales, doub
     }
     E.start(f, 0);
     E.run(m);
-    std::vector<cd> H;
-    E.record(f, H);
+    KrylovFact F;
+    {
+        std::vector<cd> H;
+        E.record(f, H);
+        F.init(std::move(H), m, herm);
+    }
     std::vector<int> failing;
     for (int i = 0; i < nt; ++i) {
         if (scales[i] == cd(0, 0)) {
             copy_v0(i);
             continue;
         }
-        int c;
         std::vector<cd> coef;
-        double terminal;
-        krylov_project(H, m, herm, scales[i], c, coef, terminal);
+        F.coef(scales[i], coef);
+        const bool est_on = F.c == m && m < n;
+        const double est = est_on ? std::abs(scales[i]) * F.terminal * beta * std::abs(coef[F.c - 1]) : 0.0;
+        double top = 0.0;
+        for (const cd& v : coef) top += std::abs(v);
+        if (est > tol * std::max(1.0, 1.001 * beta * top)) {   // past the bound for any norm it can have
+            failing.push_back(i);
+            continue;
+        }
         RotReq R;
         R.id = f;
-        R.nin = c;
+        R.nin = F.c;
         R.p = 1;
         R.out0 = m;
-        R.Y.resize(c);
-        for (int r = 0; r < c; ++r) R.Y[r] = coef[r] * beta;
+        R.Y.resize(F.c);
+        for (int r = 0; r < F.c; ++r) R.Y[r] = coef[r] * beta;
         E.rotate({R});
         const double nr = E.normalize({f}, m, false)[0];
-        const bool est_on = c == m && m < n;
-        const double est = est_on ? std::abs(scales[i]) * terminal * beta * std::abs(coef[c - 1]) : 0.0;
         if (est > tol * std::max(1.0, nr)) failing.push_back(i);
         else E.store(f, m, out + (size_t)i * 2 * n, false);
     }
-    E.remove(f);
     // the failing times: the recursion from v0, concurrently, in waves that fit in memory
     if (!failing.empty()) {
         size_t fr = 0, tot = 0;
         QS_CUDA(cudaMemGetInfo(&fr, &tot));
         const size_t per = Engine::slot_bytes(n, m, true, 1, E.store());
+        // their first steps start from the factorisation at hand where its slot
+        // leaves room for others
+        const bool share = per <= fr / 4;
+        if (!share) E.remove(f);
         const int wave = (int)std::max<size_t>(1, std::min<size_t>(failing.size(), (fr / 2) / std::max<size_t>(per, 1)));
         for (size_t w0 = 0; w0 < failing.size(); w0 += wave) {
             const size_t w1 = std::min(failing.size(), w0 + wave);
@@ -2761,18 +2890,19 @@ void evolve_engine(Op& op, const double* v0, const std::vector<cd>& scales, doub
             for (size_t q = w0; q < w1; ++q) {
                 const int i = failing[q];
                 const int id = E.add(op, m, true, 1, orth);
-                E.load(id, 0, v0, false);
+                if (!share) E.load(id, 0, v0, false);
                 ids.push_back(id);
                 outs.push_back(out + (size_t)i * 2 * n);
             }
-            std::vector<double> b0 = E.normalize(ids);
+            const std::vector<double> b0 = share ? std::vector<double>(ids.size(), beta) : E.normalize(ids);
             for (size_t q = w0; q < w1; ++q) {
                 EvoTask t;
                 // the recursion's first attempt is the shared factorisation, which failed
                 t.init(m, n, herm, scales[failing[q]], tol, b0[q - w0], true);
                 tasks.push_back(t);
             }
-            run_evo_slots(E, ids, tasks, outs);
+            if (share) run_evo_slots(E, ids, tasks, outs, false, std::vector<int>(ids.size(), f), {{f, &F}});
+            else run_evo_slots(E, ids, tasks, outs);
         }
     }
     if (normalise)
@@ -2890,8 +3020,12 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
             act.push_back(b);
             act_ids.push_back(f[b]);
         }
-    std::vector<std::vector<cd>> H;
-    E.records(act_ids, H);
+    std::vector<KrylovFact> facts(act.size());
+    {
+        std::vector<std::vector<cd>> H;
+        E.records(act_ids, H);
+        for (size_t q = 0; q < act.size(); ++q) facts[q].init(std::move(H[q]), m[act[q]], herm[act[q]]);
+    }
     // every time of every block from its shared factorisation: one rotation
     // launch and one normalisation per Krylov size for all blocks at a time
     std::vector<std::pair<size_t, int>> failing;
@@ -2906,21 +3040,20 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
                 copy_v0(b, i);
                 continue;
             }
-            int c;
+            const KrylovFact& F = facts[q];
             std::vector<cd> coef;
-            double terminal;
-            krylov_project(H[q], m[b], herm[b], scales[i], c, coef, terminal);
+            F.coef(scales[i], coef);
             RotReq R;
             R.id = f[b];
-            R.nin = c;
+            R.nin = F.c;
             R.p = 1;
             R.out0 = m[b];
-            R.Y.resize(c);
-            for (int r = 0; r < c; ++r) R.Y[r] = coef[r] * beta[b];
+            R.Y.resize(F.c);
+            for (int r = 0; r < F.c; ++r) R.Y[r] = coef[r] * beta[b];
             rot.push_back(std::move(R));
             who.push_back(b);
-            cs.push_back(c);
-            terms.push_back(std::abs(scales[i]) * terminal * beta[b] * std::abs(coef[c - 1]));
+            cs.push_back(F.c);
+            terms.push_back(std::abs(scales[i]) * F.terminal * beta[b] * std::abs(coef[F.c - 1]));
         }
         if (rot.empty()) continue;
         E.rotate(rot);
@@ -2941,11 +3074,22 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
             else E.store(f[b], m[b], outs[b] + (size_t)i * 2 * n[b], true);
         }
     }
-    for (size_t b : act) E.remove(f[b]);
     // phase 2: the failing (block, time) pairs run the reference's recursion
-    // from their start vectors, concurrently, in waves that fit in memory
+    // from their start vectors, concurrently, in waves that fit in memory; the
+    // blocks' factorisations serve their first steps where they leave room
     size_t fr = 0, tot = 0;
     QS_CUDA(cudaMemGetInfo(&fr, &tot));
+    size_t held = 0;
+    std::map<int, const KrylovFact*> root_facts;
+    for (size_t q = 0; q < act.size(); ++q) {
+        held += Engine::slot_bytes(n[act[q]], m[act[q]], true, 1, E.store());
+        root_facts[f[act[q]]] = &facts[q];
+    }
+    const bool share = held <= fr / 4;
+    for (size_t b : act) {
+        if (share) E.slot_mut(f[b]).state = kSlotIdle;
+        else E.remove(f[b]);
+    }
     for (size_t w0 = 0; w0 < failing.size();) {
         std::vector<int> ids;
         std::vector<EvoTask> tasks;
@@ -2958,19 +3102,28 @@ void evolve_blocks(const std::vector<Op*>& ops, const std::vector<const double*>
             if (w1 > w0 && used + per > fr / 2) break;
             used += per;
             const int id = E.add(*ops[b], m[b], true, 1, herm[b] ? 2 : 0);
-            E.load(id, 0, v0s[b], true);
+            if (!share) E.load(id, 0, v0s[b], true);
             ids.push_back(id);
             wouts.push_back(outs[b] + (size_t)failing[w1].second * 2 * n[b]);
             blk.push_back(b);
         }
-        const std::vector<double> b0 = E.normalize(ids);
+        std::vector<double> b0;
+        std::vector<int> roots;
+        if (share) {
+            for (size_t b : blk) {
+                b0.push_back(beta[b]);
+                roots.push_back(f[b]);
+            }
+        } else {
+            b0 = E.normalize(ids);
+        }
         for (size_t q = 0; q < ids.size(); ++q) {
             EvoTask t;
             // the recursion's first attempt is the shared factorisation, which failed
             t.init(m[blk[q]], n[blk[q]], herm[blk[q]], scales[failing[w0 + q].second], tol, b0[q], true);
             tasks.push_back(t);
         }
-        run_evo_slots(E, ids, tasks, wouts, true);
+        run_evo_slots(E, ids, tasks, wouts, true, roots, root_facts);
         w0 = w1;
     }
     QS_CUDA(cudaStreamSynchronize(st));

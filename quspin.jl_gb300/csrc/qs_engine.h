@@ -128,6 +128,8 @@ class Engine {
     void load(int id, int col, const double* v, bool device);
     // FP64 copy of a column (host or device destination)
     void store(int id, int col, double* out, bool device);
+    // column dcol of slot dst <- column scol of slot src (same rows and kind)
+    void copy_column(int src, int scol, int dst, int dcol);
     // column col /= ||column col|| for the listed slots (scale = false: only
     // measure); returns the norms
     std::vector<double> normalize(const std::vector<int>& ids, int col = 0, bool scale = true);
@@ -222,14 +224,21 @@ struct EigTask {
 // Element bytes of a vector in storage st (cv: complex).
 inline size_t store_bytes(Store st, bool cv) { return (st == Store::F32 ? 4 : 8) * (cv ? 2 : 1); }
 
-// Krylov projection of a filled record H ((m + 1) x m, column-major):
-// the completed size c (the reference's breakdown test, tn <= 100 eps
-// max(1, ||H||_F) on the matrix built so far), coef = exp(s H_c) e_1 (for a
-// Hermitian recurrence through the eigen-decomposition of the real
-// tridiagonal, as the reference does, else Pade), and the terminal norm
-// H(c, c - 1).  src/operators.jl:1655-1756.
-void krylov_project(const std::vector<cd>& H, int m, bool hermitian, cd scale, int& c, std::vector<cd>& coef,
-                    double& terminal);
+// A filled record H ((m + 1) x m, column-major): the completed size c (the
+// reference's breakdown test, tn <= 100 eps max(1, ||H||_F) on the matrix built
+// so far), the terminal norm H(c, c - 1), and, for a Hermitian recurrence, the
+// eigen-decomposition of the real tridiagonal, which serves every scale.
+// coef(scale) = exp(scale H_c) e_1 (through it, as the reference does, else
+// Pade).  src/operators.jl:1655-1756.
+struct KrylovFact {
+    int m = 0, c = 0;
+    bool hermitian = true;
+    double terminal = 0;
+    std::vector<cd> H;
+    std::vector<double> w, U;
+    void init(std::vector<cd> rec, int m_, bool herm);
+    void coef(cd scale, std::vector<cd>& out) const;
+};
 
 // The reference's _krylov_expmv_vector (src/operators.jl:1758-1803) on one
 // slot: the recursion is a queue of segments (scale, tol, depth) applied in
@@ -250,7 +259,7 @@ struct EvoTask {
     std::deque<Seg> segs;
     double beta = 0, err = 0;
     int halvings = 0;
-    std::vector<cd> H;   // record of the factorisation of column 0's state
+    KrylovFact fact;     // the factorisation of column 0's state (on_hold)
     // split: the full-scale attempt is known to fail (it was the shared
     // factorisation), so start from the two half steps it would produce
     void init(int m_, int64_t n_, bool herm, cd scale, double tol, double beta0, bool split = false);
@@ -259,8 +268,11 @@ struct EvoTask {
     // segment (project).
     void on_hold(const std::vector<cd>& Hrec, int id, RotReq& rot);
     // The candidate beta V_c exp(s H_c) e_1 of the front segment goes to
-    // column m (rot); the error estimate is kept.
-    void project(int id, RotReq& rot);
+    // column m (rot); the error estimate is kept.  Segments that fail whatever
+    // the candidate's norm are halved first.
+    void project(const KrylovFact& F, int id, RotReq& rot);
+    void project(int id, RotReq& rot) { project(fact, id, rot); }
+    void split_front();
     // With the candidate's norm: 1 accepted (copy column m to column 0 through
     // `copy`, beta = nr; a new factorisation is due unless done()), 0 rejected
     // and split (call project again: same basis), -1 depth limit reached.
