@@ -2,9 +2,9 @@
 // each on its own assembled operator and its own vectors, advanced together.
 //
 // One Lanczos/Arnoldi step of every stepping slot is a fixed sequence of ten
-// launches (SpMV; dots + reduce; the update with the norm and the second
-// pass's dots fused; the conditional second Gram-Schmidt update; scale;
-// advance; seven when every slot runs the three-term recurrence), each
+// launches (SpMV; dots + reduce; the update with the norm + reduce; the second
+// Gram-Schmidt pass where a step asks for it: dots + reduce, update + reduce;
+// scale; six when every slot runs the three-term recurrence), each
 // covering all slots through a block -> slot map.  The step
 // counters live on the device, so the sequence is captured once in a CUDA
 // graph and replayed; the host only meets the device when a slot has filled
@@ -66,14 +66,17 @@ struct SlotDev {
     void* y;                // rotation coefficients, rot_in x p column-major (storage format)
     // [0] squared norm of the new direction, [1] its inverse norm, [2] norm of
     // a normalised column, [3] ||w||^2 before orthogonalisation, [4] 1 when the
-    // second Gram-Schmidt pass runs in this step
+    // second Gram-Schmidt pass runs in this step, [6] 1 when the newest column
+    // waits for its scaling
     double* nrm;
     int32_t m, j, state;
+    int32_t j0;             // the column this run of steps started from
     // orthogonalisation of a step: 0 classical Gram-Schmidt twice (CGS2);
     // 1 CGS with the DGKS correction only when ||w'|| < 0.717 ||w|| (ARPACK's
     // dsaitr test); 2 Lanczos three-term recurrence (Hermitian operators,
     // the reference's Krylov exponential)
     int32_t orth;
+    int32_t shift;          // steps take the known part of the recurrence out in the product (Shift)
     // rotation: V[:, out0 + c] = sum_{i < rot_in} V[:, i] Y[i, c] for c < p, then
     // V[:, cdst] = V[:, carry] when carry >= 0
     int32_t rot_in, p, out0, carry, cdst;
@@ -190,7 +193,7 @@ class Engine {
     // most vectors any slot dots against in a step (1 for three-term slots,
     // m for Gram-Schmidt ones) and whether any slot takes a second pass
     int dmax_ = 1;
-    bool cgs_ = false;
+    bool cgs_ = false, shift_ = false;
     int step_launches_ = 10;
     size_t cap_partial_ = 0, cap_rmap_ = 0, cap_smap_ = 0;
     bool dirty_ = true, maps_dirty_ = true;
