@@ -2011,21 +2011,27 @@ void grid_barrier_check(int phantom, double limit_ms, int blocks) {
 }
 
 // Which stepping slots take the cluster step, and with how many CTAs: by the
-// slot's own size only, so that a slot's result is the same alone and in any
-// batch.  Measured on GB300 against the graph replay: eight CTAs per slot
-// 1.3-2.2x faster for slots of 700 to 9,300 rows; sixteen CTAs for 8,400 to
-// 29,000 rows (1.9x at 8,400, 1.23x at 29,000 rows alone, even for the 22
-// sectors of J1-J2 L=22 at 32,000 rows); larger slots are faster on the graph
-// replay (0.6-0.7x for the 26 sectors of L=24 at 104,000 rows), whose kernels
-// spread a slot over the whole GPU.
-constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 32768;
+// slot and the storage, so that a slot's result is the same alone and in any
+// batch.  Up to 8,192 rows eight CTAs win everywhere (2,703 rows, ground state:
+// 3.4 against 4.5 ms on the graph replay).  Above, sixteen CTAs save the launch
+// gaps of ten kernels a step but have 16 SMs' FP64 rate, where the graph spreads a
+// slot over all of them; so the limit is where the work of a row overtakes the
+// gaps (ground states on GB300, cluster / graph in ms):
+//   real matrix:  14,310 rows 3.4/3.8, 19,448 rows 3.6/3.8, 24,310 rows 4.05/3.83,
+//                 28,968 rows 6.5/4.6; evolution 16,384 rows 6.6/7.6, 32,768 9.2/8.5
+//   complex, FP64 (four multiply-adds an entry on the FP64 pipe):
+//                 8,398 rows 6.5/6.2, 9,225 rows 8.1/7.6, 16,796 rows 9.8/6.2
+//   complex, double-float: 9,225 rows 5.3/6.3, 14,000 rows 3.9/4.1, 16,796 rows
+//                 5.8/5.2; FP32: 3.9/4.5, 2.4/2.5, 3.8/3.6
+constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 20480, kClusterRowsComplex = 14336;
 
 int Engine::cluster_size_for(const SlotDev& d) const {
     const char* e = std::getenv("QS_CLUSTER_STEP");
     if (e && e[0] == '0') return 0;
     if (!(e && e[0] == '1') && persistent_wanted()) return 0;
     if (d.n <= kClusterRows8) return 8;
-    if (d.n <= kClusterRows16 || (e && e[0] == '1')) return cluster16_ok() ? 16 : 8;
+    const int64_t limit = !d.cm ? kClusterRows16 : st_ == Store::F64 ? kClusterRows8 : kClusterRowsComplex;
+    if (d.n <= limit || (e && e[0] == '1')) return cluster16_ok() ? 16 : 8;
     return 0;
 }
 
