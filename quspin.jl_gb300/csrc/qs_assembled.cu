@@ -1404,12 +1404,11 @@ void op_assemble(Op& op) {
     M.ncodes = (int)ncodes;
     M.code_bits = code_bits;
     M.packed = packed;
-    M.table64.alloc(ncodes * sizeof(cd));
-    QS_CUDA(cudaMemcpy(M.table64.p, table.data(), ncodes * sizeof(cd), cudaMemcpyHostToDevice));
+    BufPack tables;
+    tables.add(M.table64, ncodes * sizeof(cd), table.data());
     std::vector<std::complex<float>> t32(ncodes);
     for (int64_t i = 0; i < ncodes; ++i) t32[i] = std::complex<float>((float)table[i].real(), (float)table[i].imag());
-    M.table32.alloc(ncodes * sizeof(std::complex<float>));
-    QS_CUDA(cudaMemcpy(M.table32.p, t32.data(), ncodes * sizeof(std::complex<float>), cudaMemcpyHostToDevice));
+    tables.add(M.table32, ncodes * sizeof(std::complex<float>), t32.data());
     std::vector<float> tdf(4 * ncodes);
     for (int64_t i = 0; i < ncodes; ++i) {
         double re = table[i].real(), im = table[i].imag();
@@ -1419,8 +1418,7 @@ void op_assemble(Op& op) {
         tdf[4 * i + 2] = ih;
         tdf[4 * i + 3] = (float)(im - (double)ih);
     }
-    M.table_df.alloc(ncodes * 4 * sizeof(float));
-    QS_CUDA(cudaMemcpy(M.table_df.p, tdf.data(), ncodes * 4 * sizeof(float), cudaMemcpyHostToDevice));
+    tables.add(M.table_df, ncodes * 4 * sizeof(float), tdf.data());
     {
         // fixed-point row sums: value(code) = +-amp[class] * D[d], with class =
         // a * nC + c real and at most four of them
@@ -1441,22 +1439,19 @@ void op_assemble(Op& op) {
                 cls[code] = (uint32_t)((((code >> 1) / nD) << 1) | (code & 1));
             std::vector<double> sq(kMaxGroup + 1);
             for (int i = 0; i <= kMaxGroup; ++i) sq[i] = std::sqrt((double)i);
-            M.fx_cls.alloc(cls.size() * sizeof(uint32_t));
-            QS_CUDA(cudaMemcpy(M.fx_cls.p, cls.data(), cls.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-            M.fx_amp.alloc(4 * sizeof(double));
-            QS_CUDA(cudaMemcpy(M.fx_amp.p, amp.data(), 4 * sizeof(double), cudaMemcpyHostToDevice));
-            M.fx_sq.alloc(sq.size() * sizeof(double));
-            QS_CUDA(cudaMemcpy(M.fx_sq.p, sq.data(), sq.size() * sizeof(double), cudaMemcpyHostToDevice));
-            M.fx_max.alloc((1 + kFxParts) * sizeof(unsigned long long));
+            tables.add(M.fx_cls, cls.size() * sizeof(uint32_t), cls.data());
+            tables.add(M.fx_amp, 4 * sizeof(double), amp.data());
+            tables.add(M.fx_sq, sq.size() * sizeof(double), sq.data());
+            tables.add(M.fx_max, (1 + kFxParts) * sizeof(unsigned long long));
             M.fx_classes = ncls;
         }
     }
     {
         std::vector<float> rq(2 * (kMaxGroup + 1), 0.f);
         for (int i = 1; i <= kMaxGroup; ++i) df_split_host(1.0 / std::sqrt((double)i), rq[2 * i], rq[2 * i + 1]);
-        M.rsq_df.alloc(rq.size() * sizeof(float));
-        QS_CUDA(cudaMemcpy(M.rsq_df.p, rq.data(), rq.size() * sizeof(float), cudaMemcpyHostToDevice));
+        tables.add(M.rsq_df, rq.size() * sizeof(float), rq.data());
     }
+    tables.place(M.tables);
     M.xsplit.alloc((size_t)b.n * 4 * sizeof(float));
 
     cudaStream_t s = op.stream;

@@ -138,6 +138,7 @@ struct Assembled {
     DevBuf words;      // uint32 (column << code_bits) | code, when packed
     DevBuf cols;       // int32 column per nonzero, when not packed
     DevBuf codes;      // uint16 code per nonzero, when not packed
+    DevBuf tables;     // holds the small tables below
     DevBuf table64;    // complex double value per code
     DevBuf table32;    // complex float value per code
     DevBuf table_df;   // per code: re hi, re lo, im hi, im lo (float)

@@ -708,7 +708,7 @@ void detect_fast_group(Basis& b, const Closure& C, int kmom, int nT) {
 }
 
 // The split rank tables of a fixed-weight parent sector of at most 32 sites.
-void build_rank_split(Basis& b, const std::vector<uint64_t>& binom) {
+void build_rank_split(Basis& b, const std::vector<uint64_t>& binom, BufPack& pack) {
     if (b.nup < 0 || b.L > 32) return;
     RankSplit& R = b.rank;
     const int L = b.L;
@@ -728,20 +728,33 @@ void build_rank_split(Basis& b, const std::vector<uint64_t>& binom) {
             }
     }
     R.size = (int)tab.size();
-    b.d_rank.alloc(tab.size() * sizeof(uint32_t));
-    QS_CUDA(cudaMemcpy(b.d_rank.p, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    pack.add(b.d_rank, tab.size() * sizeof(uint32_t), tab.data());
 }
 
 // sqrt(i) and 1/sqrt(i) of every stabiliser order, correctly rounded (a square
 // root or a division per row would cost more FP64 work than the row's sum)
-void build_sqrt_table(Basis& b) {
+void build_sqrt_table(Basis& b, BufPack& pack) {
     std::vector<double> t(2 * (kMaxGroup + 1), 0.0);
     for (int i = 1; i <= kMaxGroup; ++i) {
         t[i] = std::sqrt((double)i);
         t[kMaxGroup + 1 + i] = 1.0 / std::sqrt((double)i);
     }
-    b.d_sqrt.alloc(t.size() * sizeof(double));
-    QS_CUDA(cudaMemcpy(b.d_sqrt.p, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice));
+    pack.add(b.d_sqrt, t.size() * sizeof(double), t.data());
+}
+
+// Places the tables and enumerates a symmetric sector.
+void finish_sector(Basis& b, BufPack& pack) {
+    DevBuf d_chi_one;
+    if (b.symmetric) {
+        std::vector<int8_t> chi_one(kMaxGroup, 0);
+        for (int e = 0; e < b.group.ng; ++e)
+            chi_one[e] = (std::fabs(b.group.chi_re[e] - 1.0) < 1e-9 && std::fabs(b.group.chi_im[e]) < 1e-9) ? 1 : 0;
+        pack.add(d_chi_one, kMaxGroup, chi_one.data());
+    }
+    pack.place(b.d_tables);
+    if (!b.symmetric) b.n = b.n_parent;
+    else if (b.wide) enumerate_sector<uint64_t>(b, d_chi_one);
+    else enumerate_sector<uint32_t>(b, d_chi_one);
 }
 
 }  // namespace
@@ -874,29 +887,14 @@ void basis_build(Basis& b) {
     std::vector<uint64_t> binom(64 * 65, 0);
     for (int n = 0; n < 64; ++n)
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
-    b.d_binom.alloc(binom.size() * sizeof(uint64_t));
-    QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
-    build_rank_split(b, binom);
-    if (b.symmetric) build_sqrt_table(b);
-    b.d_group.alloc(sizeof(GroupDesc));
-    QS_CUDA(cudaMemcpy(b.d_group.p, &b.group, sizeof(GroupDesc), cudaMemcpyHostToDevice));
+    BufPack pack;
+    pack.add(b.d_binom, binom.size() * sizeof(uint64_t), binom.data());
+    build_rank_split(b, binom, pack);
+    if (b.symmetric) build_sqrt_table(b, pack);
+    pack.add(b.d_group, sizeof(GroupDesc), &b.group);
     detect_fast_group(b, C, kmom, nT);
-    if (b.fast.enabled) {
-        b.d_fast_chi.alloc(b.fast_chi.size() * sizeof(cplx));
-        QS_CUDA(cudaMemcpy(b.d_fast_chi.p, b.fast_chi.data(), b.fast_chi.size() * sizeof(cplx), cudaMemcpyHostToDevice));
-    }
-
-    if (!b.symmetric) {
-        b.n = b.n_parent;
-        return;
-    }
-    std::vector<int8_t> chi_one(kMaxGroup, 0);
-    for (int e = 0; e < b.group.ng; ++e)
-        chi_one[e] = (std::fabs(b.group.chi_re[e] - 1.0) < 1e-9 && std::fabs(b.group.chi_im[e]) < 1e-9) ? 1 : 0;
-    DevBuf d_chi_one(kMaxGroup);
-    QS_CUDA(cudaMemcpy(d_chi_one.p, chi_one.data(), kMaxGroup, cudaMemcpyHostToDevice));
-    if (b.wide) enumerate_sector<uint64_t>(b, d_chi_one);
-    else enumerate_sector<uint32_t>(b, d_chi_one);
+    if (b.fast.enabled) pack.add(b.d_fast_chi, b.fast_chi.size() * sizeof(cplx), b.fast_chi.data());
+    finish_sector(b, pack);
 }
 
 // ------------------------------------------------- basis_build_general
@@ -1053,10 +1051,10 @@ void basis_build_general(Basis& b, const qs_general_spec& gs) {
     std::vector<uint64_t> binom(64 * 65, 0);
     for (int n = 0; n < 64; ++n)
         for (int k = 0; k <= 64; ++k) binom[n * 65 + k] = (uint64_t)binom_host(n, k);
-    b.d_binom.alloc(binom.size() * sizeof(uint64_t));
-    QS_CUDA(cudaMemcpy(b.d_binom.p, binom.data(), binom.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
-    build_rank_split(b, binom);
-    if (b.symmetric) build_sqrt_table(b);
+    BufPack pack;
+    pack.add(b.d_binom, binom.size() * sizeof(uint64_t), binom.data());
+    build_rank_split(b, binom, pack);
+    if (b.symmetric) build_sqrt_table(b, pack);
     b.d_gtab.alloc(std::max<size_t>(1, tables.size()) * sizeof(uint64_t));
     if (!tables.empty())
         QS_CUDA(cudaMemcpy(b.d_gtab.p, tables.data(), tables.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
@@ -1068,20 +1066,9 @@ void basis_build_general(Basis& b, const qs_general_spec& gs) {
                            cudaMemcpyHostToDevice));
         b.level_groups[lvl].gtab = b.d_level_gtab.back().as<uint64_t>();
     }
-    b.d_group.alloc(sizeof(GroupDesc));
-    QS_CUDA(cudaMemcpy(b.d_group.p, &b.group, sizeof(GroupDesc), cudaMemcpyHostToDevice));
+    pack.add(b.d_group, sizeof(GroupDesc), &b.group);
     b.fast = FastGroup{};
-    if (!b.symmetric) {
-        b.n = b.n_parent;
-        return;
-    }
-    std::vector<int8_t> chi_one(kMaxGroup, 0);
-    for (int e = 0; e < b.group.ng; ++e)
-        chi_one[e] = (std::fabs(b.group.chi_re[e] - 1.0) < 1e-9 && std::fabs(b.group.chi_im[e]) < 1e-9) ? 1 : 0;
-    DevBuf d_chi_one(kMaxGroup);
-    QS_CUDA(cudaMemcpy(d_chi_one.p, chi_one.data(), kMaxGroup, cudaMemcpyHostToDevice));
-    if (b.wide) enumerate_sector<uint64_t>(b, d_chi_one);
-    else enumerate_sector<uint32_t>(b, d_chi_one);
+    finish_sector(b, pack);
 }
 
 // ------------------------------------------------------------- index_of

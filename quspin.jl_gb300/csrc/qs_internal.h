@@ -5,6 +5,7 @@
 
 #include <complex>
 #include <cstdint>
+#include <cstring>
 #include <functional>
 #include <memory>
 #include <stdexcept>
@@ -38,32 +39,41 @@ struct Error : std::runtime_error {
 // DevBuf or of the pool); qs_device_alloc_count reports it.
 void note_device_alloc();
 
-// Owning device buffer.
+// cudaMalloc; when memory is short, the pool's free blocks are given back first
+// (qs_pool.cpp).
+void* device_alloc(size_t bytes);
+
+// Owning device buffer, or a part of another one (view), which has to outlive it.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool own = true;
     DevBuf() = default;
     explicit DevBuf(size_t n) { alloc(n); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; o.bytes = 0; }
+    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), own(o.own) { o.p = nullptr; o.bytes = 0; }
     DevBuf& operator=(DevBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; bytes = o.bytes; o.p = nullptr; o.bytes = 0; }
+        if (this != &o) { release(); p = o.p; bytes = o.bytes; own = o.own; o.p = nullptr; o.bytes = 0; }
         return *this;
     }
     ~DevBuf() { release(); }
     void alloc(size_t n) {
         release();
-        if (n) {
-            note_device_alloc();
-            QS_CUDA(cudaMalloc(&p, n));
-        }
+        if (n) p = device_alloc(n);
         bytes = n;
     }
+    void view(const DevBuf& store, size_t offset, size_t n) {
+        release();
+        p = n ? static_cast<char*>(store.p) + offset : nullptr;
+        bytes = n;
+        own = false;
+    }
     void release() {
-        if (p) cudaFree(p);
+        if (p && own) cudaFree(p);
         p = nullptr;
         bytes = 0;
+        own = true;
     }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
@@ -89,6 +99,35 @@ void* mapped_host_address(void* p);
 void touch_host(void* p, size_t bytes);
 // touch_host(dst), then the copy of device memory into it on s.
 void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+
+// Several buffers in one allocation: add() each with its host contents (null:
+// left unset), then place() them.  A cudaMalloc and cudaFree pair takes 13 us
+// for a small buffer and 200 us for one of 20 MB.
+class BufPack {
+   public:
+    void add(DevBuf& b, size_t bytes, const void* from = nullptr) {
+        parts_.push_back({&b, size_, bytes});
+        size_ += (bytes + 255) / 256 * 256;
+        if (from) {
+            host_.resize(size_);
+            std::memcpy(host_.data() + parts_.back().offset, from, bytes);
+        }
+    }
+    void place(DevBuf& store) {
+        store.alloc(size_);
+        if (!host_.empty()) QS_CUDA(cudaMemcpy(store.p, host_.data(), host_.size(), cudaMemcpyHostToDevice));
+        for (const Part& q : parts_) q.buf->view(store, q.offset, q.bytes);
+    }
+
+   private:
+    struct Part {
+        DevBuf* buf;
+        size_t offset, bytes;
+    };
+    std::vector<Part> parts_;
+    std::vector<char> host_;
+    size_t size_ = 0;
+};
 
 struct PoolBuf {
     void* p = nullptr;
@@ -138,6 +177,7 @@ struct Basis {
     int nup = -1;
     bool symmetric = false;
     bool general = false;            // general site maps (GEN_GENERAL generators)
+    DevBuf d_tables;                 // holds the small tables below
     DevBuf d_gtab;                   // their permutation tables (GroupDesc::gtab)
     std::vector<int> gen_perm_index; // each generator's permutation in those tables
     std::vector<DevBuf> d_level_gtab;// the level groups' tables
@@ -210,6 +250,7 @@ struct Op {
     std::vector<TermProg> progs;    // off-diagonal transition programs
     std::vector<TermProg> diag_progs;
     std::vector<std::complex<double>> user_diag;
+    DevBuf d_tables;                // holds d_progs, d_rowprogs, d_amp
     DevBuf d_progs;
     // the programs as the row kernels read them, the amplitude of every class
     // (complex double), and whether a sign depends on the state / a program
@@ -218,6 +259,7 @@ struct Op {
     std::vector<uint32_t> prog_class;
     int nclass = 0;
     bool any_zy = false, check_weight = false, any_chars = false;
+    DevBuf d_diags;                 // holds the five forms of the diagonal
     DevBuf d_diag;                  // complex diagonal (user + extracted), 2*n doubles
     DevBuf d_diag32;                // single-precision copy
     DevBuf d_diag_re, d_diag32_re;  // real parts (read by real operators)

@@ -70,6 +70,10 @@ void* pool_get(size_t bytes) {
         }
         return b.p;
     }
+    return device_alloc(bytes);
+}
+
+void* device_alloc(size_t bytes) {
     void* p = nullptr;
     note_device_alloc();
     cudaError_t e = cudaMalloc(&p, bytes);
