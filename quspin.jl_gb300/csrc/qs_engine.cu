@@ -393,8 +393,10 @@ __device__ __forceinline__ double block_sum(A v, double* sh) {
     __syncthreads();
     if (lane == 0) sh[wid] = to_d(v);
     __syncthreads();
+    // only the first warp: a warp's FP64 add takes its SM's pipe 16 cycles
     double t = 0;
-    for (int q = 0; q < kT / 32; ++q) t += sh[q];
+    if (wid == 0)
+        for (int q = 0; q < kT / 32; ++q) t += sh[q];
     return t;
 }
 
@@ -494,24 +496,108 @@ __device__ __forceinline__ void fused_epilogue(A (&acc)[NV + 1], int nv, bool no
     }
 }
 
+// Three-term slots (Hermitian, no reorthogonalisation): alpha = <v_j, w> and
+// both coefficients of the recurrence are real, so the dot takes two
+// multiply-adds a row instead of four and the update four instead of ten (the
+// imaginary parts are rounding).
+template <class A, bool CV>
+__device__ __forceinline__ A three_dot_rows(const SlotDev& S, int64_t r0, int64_t r1) {
+    const void* w = colp<A>(S, S.j + 1);
+    const void* v = colp<A>(S, S.j);
+    A acc = zero<A>();
+    auto one = [&](const CA<A>& a, const CA<A>& b) {
+        mac(acc, a.re, b.re);
+        if (CV) mac(acc, a.im, b.im);
+    };
+    const int64_t step = blockDim.x;
+    int64_t r = r0 + threadIdx.x;
+#pragma unroll 1
+    for (; r + step < r1; r += 2 * step) {
+        const CA<A> a0 = ldv<A, CV>(v, r), a1 = ldv<A, CV>(v, r + step);
+        const CA<A> b0 = ldv<A, CV>(w, r), b1 = ldv<A, CV>(w, r + step);
+        one(a0, b0);
+        one(a1, b1);
+    }
+#pragma unroll 1
+    for (; r < r1; r += step) one(ldv<A, CV>(v, r), ldv<A, CV>(w, r));
+    return acc;
+}
+// w -= alpha v_j + beta v_{j-1}; returns the part of ||w||^2
+template <class A, bool CV>
+__device__ __forceinline__ A three_update_rows(const SlotDev& S, int64_t r0, int64_t r1, A alpha, A beta) {
+    void* w = colp<A>(S, S.j + 1);
+    const void* v = colp<A>(S, S.j);
+    const bool two = S.j > 0;
+    const void* u = colp<A>(S, two ? S.j - 1 : S.j);
+    A nacc = zero<A>();
+    auto one = [&](CA<A> o, const CA<A>& a, const CA<A>& b) {
+        msub(o.re, a.re, alpha);
+        if (CV) msub(o.im, a.im, alpha);
+        if (two) {
+            msub(o.re, b.re, beta);
+            if (CV) msub(o.im, b.im, beta);
+        }
+        mac(nacc, o.re, o.re);
+        if (CV) mac(nacc, o.im, o.im);
+        return o;
+    };
+    const int64_t step = blockDim.x;
+    int64_t r = r0 + threadIdx.x;
+#pragma unroll 1
+    for (; r + step < r1; r += 2 * step) {
+        const CA<A> o0 = ldv<A, CV>(w, r), o1 = ldv<A, CV>(w, r + step);
+        const CA<A> a0 = ldv<A, CV>(v, r), a1 = ldv<A, CV>(v, r + step);
+        const CA<A> b0 = ldv<A, CV>(u, r), b1 = ldv<A, CV>(u, r + step);
+        stv<A, CV>(w, r, one(o0, a0, b0));
+        stv<A, CV>(w, r + step, one(o1, a1, b1));
+    }
+#pragma unroll 1
+    for (; r < r1; r += step) stv<A, CV>(w, r, one(ldv<A, CV>(w, r), ldv<A, CV>(v, r), ldv<A, CV>(u, r)));
+    return nacc;
+}
+template <class A, bool UPDATE>
+__device__ __forceinline__ void three_block(const SlotDev& S, int mmax, double* partial, int bx) {
+    const int64_t lb = bx - S.rb_begin;
+    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
+    A acc;
+    if (UPDATE) {
+        const A alpha = from_d<A>(S.h1[S.j].x), beta = S.j > 0 ? from_d<A>(S.h1[S.j - 1].x) : zero<A>();
+        acc = S.cv ? three_update_rows<A, true>(S, r0, r1, alpha, beta) : three_update_rows<A, false>(S, r0, r1, alpha, beta);
+    } else {
+        acc = S.cv ? three_dot_rows<A, true>(S, r0, r1) : three_dot_rows<A, false>(S, r0, r1);
+    }
+    __shared__ double sh[kT / 32];
+    const double t = block_sum(acc, sh);
+    if (threadIdx.x == 0) {
+        double* at = partial + ((size_t)bx * (mmax + 1) + (UPDATE ? mmax : S.j)) * 2;
+        at[0] = t;
+        at[1] = 0.0;
+    }
+}
+// The dots or the update of an engine whose slots are all three-term:
+// four blocks an SM, where the Gram-Schmidt kernels with their columns in registers
+// hold two or three.
+template <class A, bool UPDATE>
+__global__ void __launch_bounds__(kT, 4) eng_three(const SlotDev* __restrict__ sl, const int* __restrict__ rmap,
+                                                   int mmax, double* __restrict__ partial) {
+    const SlotDev& S = sl[rmap[blockIdx.x]];
+    if (S.state == kSlotStep) three_block<A, UPDATE>(S, mmax, partial, blockIdx.x);
+}
+
 template <class A>
 __device__ __forceinline__ void dots_block(const SlotDev* sl, const int* __restrict__ rmap, int mmax, int mode,
                                            double* partial, int bx, int by) {
     const SlotDev& S = sl[rmap[bx]];
     if (S.state != (mode == 2 ? kSlotNormalize : kSlotStep)) return;
     if (mode == 1 && (!S.shift || S.nrm[4] == 0.0)) return;
-    const int P = mmax + 1;
-    int first, nv;
-    const void* w;
-    if (mode == 2) {
-        first = S.ncol;
-        nv = S.ncol + 1;
-        w = colp<A>(S, S.ncol);
-    } else {
-        first = (mode == 0 && S.orth == 2) ? S.j : 0;
-        nv = S.j + 1;
-        w = colp<A>(S, S.j + 1);
+    if (mode == 0 && S.orth == 2) {
+        if (by == 0) three_block<A, false>(S, mmax, partial, bx);
+        return;
     }
+    const int P = mmax + 1;
+    const int first = mode == 2 ? S.ncol : 0;
+    const int nv = (mode == 2 ? S.ncol : S.j) + 1;
+    const void* w = colp<A>(S, mode == 2 ? S.ncol : S.j + 1);
     const int i0 = first + by * jt<A>();
     if (i0 >= nv) return;
     const bool want_wn = mode == 0 && S.orth == 1 && by == 0;
@@ -714,12 +800,12 @@ __global__ void __launch_bounds__(kT) eng_reduce(SlotDev* sl, int mmax, int mode
 }
 
 // ------------------------------------------------------------ update
-// col(j+1) -= sum_i col(i) h_i over the pass's vectors (pass 0: h1 from
-// `first`, pass 1: h2 over 0..j, only where the step's flag asks), leaving the
+// col(j+1) -= sum_i col(i) h_i over the pass's vectors (pass 0: h1, pass 1: h2,
+// over 0..j, the second only where the step's flag asks), leaving the
 // block's part of ||col(j+1)||^2 at partial[b][mmax]; pass 0 of an unshifted
 // Gram-Schmidt slot also leaves the second-pass dots at partial[b][0..j].
 template <class A, bool CV>
-__device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r1, int first, int nv, const CA<A>* hs) {
+__device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const CA<A>* hs) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, CV>();
     void* w = (void*)(V + (size_t)(S.j + 1) * cs);
@@ -732,13 +818,13 @@ __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r
             mac(ai, v.im, h.re);
         }
     };
-    if (nv - first <= 2) {
-        // the three-term update (or a first step): two rows per iteration, all
-        // their loads issued before either row's store
-        const int two = nv - first == 2;
-        const char* va = V + (size_t)first * cs;
-        const char* vb = V + (size_t)(first + two) * cs;
-        const CA<A> ha = hs[first], hb = two ? hs[first + 1] : CA<A>{zero<A>(), zero<A>()};
+    if (nv <= 2) {
+        // the first steps: two rows per iteration, all their loads issued before
+        // either row's store
+        const int two = nv == 2;
+        const char* va = V;
+        const char* vb = V + (size_t)two * cs;
+        const CA<A> ha = hs[0], hb = two ? hs[1] : CA<A>{zero<A>(), zero<A>()};
         auto one = [&](CA<A> o, const CA<A>& a, const CA<A>& b) {
             A ar = zero<A>(), ai = zero<A>();
             term(ar, ai, a, ha);
@@ -764,7 +850,7 @@ __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r
     }
     for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
         A ar = zero<A>(), ai = zero<A>();
-        int t = first;
+        int t = 0;
         // four vector loads in flight before their arithmetic
         for (; t + 4 <= nv; t += 4) {
             CA<A> v[4];
@@ -790,18 +876,21 @@ __device__ __forceinline__ void update_block(const SlotDev* sl, const int* __res
     const SlotDev& S = sl[rmap[bx]];
     if (S.state != kSlotStep) return;
     if (pass == 1 && S.nrm[4] == 0.0) return;
+    if (S.orth == 2) {
+        three_block<A, true>(S, mmax, partial, bx);
+        return;
+    }
     __shared__ CA<A> hs[kMaxM];
     const int nv = S.j + 1;
-    const int first = (pass == 0 && S.orth == 2) ? (S.j > 0 ? S.j - 1 : 0) : 0;
     const double2* h = pass ? S.h2 : S.h1;
-    for (int t = first + threadIdx.x; t < nv; t += blockDim.x) {
+    for (int t = threadIdx.x; t < nv; t += blockDim.x) {
         const double2 v = h[t];
         hs[t] = CA<A>{from_d<A>(v.x), from_d<A>(v.y)};
     }
     __syncthreads();
     const int64_t lb = bx - S.rb_begin;
     const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
-    A nacc = S.cv ? update_rows<A, true>(S, r0, r1, first, nv, hs) : update_rows<A, false>(S, r0, r1, first, nv, hs);
+    A nacc = S.cv ? update_rows<A, true>(S, r0, r1, nv, hs) : update_rows<A, false>(S, r0, r1, nv, hs);
     __shared__ double sh[kT / 32];
     const double t = block_sum(nacc, sh);
     const int P = mmax + 1;
@@ -809,7 +898,7 @@ __device__ __forceinline__ void update_block(const SlotDev* sl, const int* __res
         partial[((size_t)bx * P + mmax) * 2] = t;
         partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
     }
-    if (pass == 0 && S.orth != 2 && !S.shift) {
+    if (pass == 0 && !S.shift) {
         // the unshifted slots' second-pass dots V^* w' over this block's rows,
         // while V and w' are still in cache
         const void* w = colp<A>(S, S.j + 1);
@@ -1507,12 +1596,14 @@ template <class A>
 static int launch_step_t(const SlotDev* ds, SlotDev* dsw, const int* rm, const int* sm, double* pa, const void* rsq,
                          int nrb, int nsb, int mmax, int dmax, bool cgs, bool shift, int ns, cudaStream_t s) {
     const dim3 gd(nrb, (dmax + jt<A>() - 1) / jt<A>());
-    const bool fused = fused_update_on();
+    const bool fused = fused_update_on() && cgs;
     eng_spmv<A><<<nsb, kT, 0, s>>>(ds, sm, rsq);
-    if (fused) eng_dots_fused<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 0, pa);
+    if (!cgs) eng_three<A, false><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
+    else if (fused) eng_dots_fused<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 0, pa);
     else eng_dots<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 0, pa);
     eng_reduce<<<dim3(ns, dmax + 1), kT, 0, s>>>(dsw, mmax, 0, pa, dmax, false);
-    if (fused) eng_update_fused<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
+    if (!cgs) eng_three<A, true><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
+    else if (fused) eng_update_fused<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
     else eng_update<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, 0, pa);
     eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 1, pa, 0, !cgs);
     int n = 6;
@@ -1598,14 +1689,21 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
         const bool want_wn = orth == 1;
         const void* w = colp<A>(Ls, j + 1);
         A wn = zero<A>();
-        for (int i0 = first; i0 < nv; i0 += jt<A>()) {
+        if (orth == 2) {
+            const double t = block_sum(three_dot_rows<A, CV>(Ls, r0, r1), shb);
+            if (threadIdx.x == 0) {
+                part1[j * 2] = t;
+                part1[j * 2 + 1] = 0.0;
+            }
+        }
+        for (int i0 = 0; i0 < nv && orth != 2; i0 += jt<A>()) {
             A re[jt<A>()], im[jt<A>()];
 #pragma unroll
             for (int q = 0; q < jt<A>(); ++q) re[q] = im[q] = zero<A>();
-            dots_rows<A, CV>(Ls, r0, r1, i0, nv, w, re, im, want_wn && i0 == first, wn);
+            dots_rows<A, CV>(Ls, r0, r1, i0, nv, w, re, im, want_wn && i0 == 0, wn);
             dots_epilogue<A>(re, im, CV, i0, nv, i0, part1);
         }
-        {
+        if (want_wn) {
             const double t = block_sum(wn, shb);
             if (threadIdx.x == 0) part1[m * 2] = t;
         }
@@ -1622,7 +1720,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
         }
         if (threadIdx.x == 0) {
             double t = 0;
-            for (uint32_t r = 0; r < C; ++r) t += cl_ld(&part1[m * 2], r);
+            for (uint32_t r = 0; r < C && want_wn; ++r) t += cl_ld(&part1[m * 2], r);
             scal[0] = t;
             // the three-term recurrence takes beta_{j-1} from the record
             if (orth == 2 && j > 0) {
@@ -1639,7 +1737,8 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             hs[t] = CA<A>{from_d<A>(h1[t * 2]), from_d<A>(h1[t * 2 + 1])};
         __syncthreads();
         {
-            const A nacc = update_rows<A, CV>(Ls, r0, r1, first_u, nv, hs);
+            const A nacc = orth == 2 ? three_update_rows<A, CV>(Ls, r0, r1, hs[j].re, j > 0 ? hs[j - 1].re : zero<A>())
+                                     : update_rows<A, CV>(Ls, r0, r1, nv, hs);
             const double t = block_sum(nacc, shb);
             if (threadIdx.x == 0) part2[m * 2] = t;
         }
@@ -1698,7 +1797,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             for (int t = threadIdx.x; t < nv; t += blockDim.x)
                 hs[t] = CA<A>{from_d<A>(h2[t * 2]), from_d<A>(h2[t * 2 + 1])};
             __syncthreads();
-            const A nacc = update_rows<A, CV>(Ls, r0, r1, 0, nv, hs);
+            const A nacc = update_rows<A, CV>(Ls, r0, r1, nv, hs);
             const double t3 = block_sum(nacc, shb);
             if (threadIdx.x == 0) part1[m * 2] = t3;
             cl_sync();
