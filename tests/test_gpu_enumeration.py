@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
     (20, 10, dict(kblock=0, pblock=1, zblock=1)), (20, 10, dict(kblock=10, pblock=-1, zblock=-1)),
     (19, 7, dict(kblock=3)), (18, 9, dict(pblock=1, zblock=-1)),            # 50,388; no rotations
     (32, 5, dict(kblock=16, pblock=1)), (18, 9, dict(kblock=3, a=2, zblock=1)),
-    (33, 4, dict(kblock=0, pblock=-1)), (40, 3, dict(kblock=20)), (36, 4, dict(pblock=1))])   # 64-bit states
+    (2, 1, dict(kblock=0)), (3, 2, dict(kblock=1)), (9, 1, dict(kblock=2)), (9, 8, dict(kblock=2)),   # few odd ones
+    (24, 9, dict(kblock=12, pblock=1)), (33, 4, dict(kblock=0, pblock=-1)), (40, 3, dict(kblock=20)), (36, 4, dict(pblock=1))])   # 64-bit states
 def test_matches_oracle(qs, ora, L, nup, kw):
     b = qs.SpinBasis1D(L, nup=nup, pauli=False, **kw)
     ref = ora.RepBasis(L, nup=nup, pauli=False, **kw)
