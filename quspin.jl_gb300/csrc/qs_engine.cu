@@ -168,37 +168,9 @@ template <class A> __device__ __forceinline__ char* colp(const SlotDev& S, int c
 // ------------------------------------------------------------ SpMV
 // y = col(j + 1) = H col(j) on every stepping slot: sliced ELL, one thread per
 // row, the slot's value table staged in shared memory.
-//
-// A Lanczos step of a shifted slot (DGKS in FP64 and double-float storage) past
-// its first column subtracts the known part of the recurrence at once: y = H v_j
-// - sigma v_j - beta_{j-1} v_{j-1} with sigma = alpha_{j-1}, two multiply-adds a
-// row, so that what is left for the
-// Gram-Schmidt pass is small against ||y|| and its DGKS test (||w'|| >= 0.717
-// ||y||) passes: on 60 to 80 steps of four models 33 to 53 second passes became
-// none, with the basis no less orthogonal (2e-15).  Both are rounded to FP32, so
-// that every storage subtracts the same numbers; the record adds them back, and
-// what the rounding leaves is the Gram-Schmidt pass's.  FP32 slots keep two
-// passes without it: one pass there leaves residuals of 5.5e-7 ||H|| where two
-// leave less than 1e-7.
-template <class A>
-struct Shift {
-    bool on;
-    A sigma, beta;
-};
-template <class A>
-__device__ __forceinline__ Shift<A> step_shift(const SlotDev& S) {
-    Shift<A> h{S.shift && S.j > S.j0, zero<A>(), zero<A>()};
-    if (h.on) {
-        const double2* c = S.rec + (size_t)(S.j - 1) * (S.m + 1) + S.j - 1;
-        h.sigma = from_d<A>((double)(float)__ldcg(c).x);
-        h.beta = from_d<A>((double)(float)__ldcg(c + 1).x);
-    }
-    return h;
-}
-
-template <class A, bool CV, bool CM, bool PACKED, bool SHIFT>
+template <class A, bool CV, bool CM, bool PACKED>
 __device__ __forceinline__ void spmv_rows(const SlotDev& S, int64_t s0, int64_t s1, const CA<A>* tab, bool smem_tab,
-                                          const A* rsq, const Shift<A>& sh) {
+                                          const A* rsq) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int64_t n = S.n;
     const void* x = colp<A>(S, S.j);
@@ -228,8 +200,6 @@ __device__ __forceinline__ void spmv_rows(const SlotDev& S, int64_t s0, int64_t 
                             });
         // the row's own entries, loaded beside its words
         const CA<A> d = lddiag<A>(S, r), xr = ldv<A, CV>(x, r);
-        CA<A> vp{zero<A>(), zero<A>()};
-        if (SHIFT) vp = ldv<A, CV>(colp<A>(S, S.j - 1), r);
         const int st = stab ? stab[r] : 0;
         const A sc = stab ? rsq[st] : one<A>();
         CA<A> out;
@@ -241,36 +211,23 @@ __device__ __forceinline__ void spmv_rows(const SlotDev& S, int64_t s0, int64_t 
             mac(out.im, d.re, xr.im);
             mac(out.im, d.im, xr.re);
         }
-        if (SHIFT) {
-            msub(out.re, sh.sigma, xr.re);
-            msub(out.re, sh.beta, vp.re);
-            if (CV) {
-                msub(out.im, sh.sigma, xr.im);
-                msub(out.im, sh.beta, vp.im);
-            }
-        }
         stv<A, CV>(y, r, out);
     }
 }
 
-// the slot's slices [s0, s1) of y = col(j + 1) = H col(j) (less the shift)
+// the slot's slices [s0, s1) of y = col(j + 1) = H col(j)
 template <class A, bool CV, bool CM>
 __device__ __forceinline__ void spmv_kind(const SlotDev& S, int64_t s0, int64_t s1, const CA<A>* tab, bool smem_tab,
-                                          const A* rsq, const Shift<A>& sh) {
-    if (S.packed) {
-        if (sh.on) spmv_rows<A, CV, CM, true, true>(S, s0, s1, tab, smem_tab, rsq, sh);
-        else spmv_rows<A, CV, CM, true, false>(S, s0, s1, tab, smem_tab, rsq, sh);
-    } else {
-        if (sh.on) spmv_rows<A, CV, CM, false, true>(S, s0, s1, tab, smem_tab, rsq, sh);
-        else spmv_rows<A, CV, CM, false, false>(S, s0, s1, tab, smem_tab, rsq, sh);
-    }
+                                          const A* rsq) {
+    if (S.packed) spmv_rows<A, CV, CM, true>(S, s0, s1, tab, smem_tab, rsq);
+    else spmv_rows<A, CV, CM, false>(S, s0, s1, tab, smem_tab, rsq);
 }
 template <class A>
 __device__ __forceinline__ void spmv_slices(const SlotDev& S, int64_t s0, int64_t s1, const CA<A>* tab, bool smem_tab,
-                                            const A* rsq, const Shift<A>& sh) {
-    if (!S.cv) spmv_kind<A, false, false>(S, s0, s1, tab, smem_tab, rsq, sh);
-    else if (!S.cm) spmv_kind<A, true, false>(S, s0, s1, tab, smem_tab, rsq, sh);
-    else spmv_kind<A, true, true>(S, s0, s1, tab, smem_tab, rsq, sh);
+                                            const A* rsq) {
+    if (!S.cv) spmv_kind<A, false, false>(S, s0, s1, tab, smem_tab, rsq);
+    else if (!S.cm) spmv_kind<A, true, false>(S, s0, s1, tab, smem_tab, rsq);
+    else spmv_kind<A, true, true>(S, s0, s1, tab, smem_tab, rsq);
 }
 
 template <class A>
@@ -287,7 +244,7 @@ __device__ __forceinline__ void spmv_block(const SlotDev* sl, const int* __restr
         for (int i = threadIdx.x; i <= S.max_stab; i += blockDim.x) rsq[i] = ldrsq<A>(rsqt, i);
     __syncthreads();
     const int64_t lb = bx - S.sb_begin;
-    spmv_slices<A>(S, lb * S.spb, min(S.nslices, lb * S.spb + S.spb), tab, smem_tab, rsq, step_shift<A>(S));
+    spmv_slices<A>(S, lb * S.spb, min(S.nslices, lb * S.spb + S.spb), tab, smem_tab, rsq);
 }
 
 template <class A>
@@ -301,8 +258,7 @@ __global__ void __launch_bounds__(kT, 5) eng_spmv(const SlotDev* __restrict__ sl
 // P = mmax + 1; index mmax holds norms.
 // mode 0 (first pass): i in [first, j] with first = j for the three-term
 //   recurrence, else 0; DGKS slots also accumulate ||w||^2 at index mmax;
-// mode 1 (second pass of a shifted slot, only where the step's flag asks): i in
-//   [0, j] (the others take these dots from the first update, see eng_update);
+// (the second pass's dots come from the first update, see eng_update)
 // mode 2 (normalise): partial[b][0] = <col ncol, col ncol>.
 template <class A, bool CV>
 __device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r0, int64_t r1, int i0, int nv, const void* w,
@@ -589,7 +545,6 @@ __device__ __forceinline__ void dots_block(const SlotDev* sl, const int* __restr
                                            double* partial, int bx, int by) {
     const SlotDev& S = sl[rmap[bx]];
     if (S.state != (mode == 2 ? kSlotNormalize : kSlotStep)) return;
-    if (mode == 1 && (!S.shift || S.nrm[4] == 0.0)) return;
     if (mode == 0 && S.orth == 2) {
         if (by == 0) three_block<A, false>(S, mmax, partial, bx);
         return;
@@ -665,7 +620,6 @@ __global__ void __launch_bounds__(kT, 2) eng_dots_fused(const SlotDev* __restric
         dots_block<A>(sl, rmap, mmax, mode, partial, bx, by);
         return;
     }
-    if (mode == 1 && (!S.shift || S.nrm[4] == 0.0)) return;
     if (by) return;
     const int64_t lb = bx - S.rb_begin;
     const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
@@ -673,13 +627,6 @@ __global__ void __launch_bounds__(kT, 2) eng_dots_fused(const SlotDev* __restric
     const bool want_wn = mode == 0 && S.orth == 1;
     if (nv <= 12) dots_fused_rows<A, 12>(S, r0, r1, nv, w, want_wn, mmax, partial, bx);
     else dots_fused_rows<A, 20>(S, r0, r1, nv, w, want_wn, mmax, partial, bx);
-}
-
-// what the product of a shifted step took out of entry q of its record column:
-// sigma = alpha_{j-1} from entry j, beta_{j-1} from entry j - 1
-__device__ __forceinline__ double shift_part(const SlotDev& S, int q) {
-    if (!S.shift || S.j <= S.j0 || q < S.j - 1) return 0.0;
-    return (double)(float)S.rec[(size_t)(S.j - 1) * (S.m + 1) + 2 * S.j - 1 - q].x;
 }
 
 // ------------------------------------------------------------ reduce
@@ -773,7 +720,7 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
             const int first = S.orth == 2 ? (j > 0 ? j - 1 : 0) : 0;
             for (int q = first; q <= j; ++q) {
                 const double2 a = S.h1[q];
-                col[q] = make_double2(a.x + shift_part(S, q), a.y);
+                col[q] = a;
             }
             col[j + 1] = make_double2(nb, 0.0);
             S.nrm[0] = re;
@@ -783,7 +730,7 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
     } else if (mode == 2) {
         S.h2[i] = make_double2(re, im);
         const double2 a = S.h1[i];
-        col[i] = make_double2(a.x + re + shift_part(S, i), a.y + im);
+        col[i] = make_double2(a.x + re, a.y + im);
     } else {
         const double nb = sqrt(fmax(re, 0.0));
         S.nrm[0] = re;
@@ -802,7 +749,7 @@ __global__ void __launch_bounds__(kT) eng_reduce(SlotDev* sl, int mmax, int mode
 // ------------------------------------------------------------ update
 // col(j+1) -= sum_i col(i) h_i over the pass's vectors (pass 0: h1, pass 1: h2,
 // over 0..j, the second only where the step's flag asks), leaving the
-// block's part of ||col(j+1)||^2 at partial[b][mmax]; pass 0 of an unshifted
+// block's part of ||col(j+1)||^2 at partial[b][mmax]; pass 0 of a
 // Gram-Schmidt slot also leaves the second-pass dots at partial[b][0..j].
 template <class A, bool CV>
 __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const CA<A>* hs) {
@@ -898,8 +845,8 @@ __device__ __forceinline__ void update_block(const SlotDev* sl, const int* __res
         partial[((size_t)bx * P + mmax) * 2] = t;
         partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
     }
-    if (pass == 0 && !S.shift) {
-        // the unshifted slots' second-pass dots V^* w' over this block's rows,
+    if (pass == 0) {
+        // the second-pass dots V^* w' over this block's rows,
         // while V and w' are still in cache
         const void* w = colp<A>(S, S.j + 1);
         double* row = partial + (size_t)bx * P * 2;
@@ -931,18 +878,15 @@ __device__ __forceinline__ double ld_volatile(const volatile double* p) { return
 __device__ __forceinline__ float ld_volatile(const volatile float* p) { return *p; }
 __device__ __forceinline__ DF ld_volatile(const volatile DF* p) { return DF{p->h, p->l}; }
 
-// DOTS: unshifted slots, whose second pass runs always (CGS2) or in two steps
-// of three (DGKS); a shifted slot's hardly ever does.
-template <class A, int NV, bool DOTS>
+template <class A, int NV>
 __device__ __forceinline__ void update_fused_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const CA<A>* hs,
                                                   int mmax, double* partial, int bx) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, false>();
     void* w = (void*)(V + (size_t)(S.j + 1) * cs);
-    constexpr int NA = DOTS ? NV : 0;
-    A acc[NA + 1];   // the second-pass dots, then ||w'||^2
+    A acc[NV + 1];   // the second-pass dots, then ||w'||^2
 #pragma unroll
-    for (int t = 0; t <= NA; ++t) acc[t] = zero<A>();
+    for (int t = 0; t <= NV; ++t) acc[t] = zero<A>();
     for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
         A v[NV];
 #pragma unroll
@@ -958,14 +902,12 @@ __device__ __forceinline__ void update_fused_rows(const SlotDev& S, int64_t r0, 
         A o = ldv<A, false>(w, r).re;
         o = sub(o, ar);
         stv<A, false>(w, r, CA<A>{o, zero<A>()});
-        mac(acc[NA], o, o);
-        if (DOTS) {
+        mac(acc[NV], o, o);
 #pragma unroll
-            for (int t = 0; t < NA; ++t)
-                if (t < nv) mac(acc[t], v[t], o);
-        }
+        for (int t = 0; t < NV; ++t)
+            if (t < nv) mac(acc[t], v[t], o);
     }
-    fused_epilogue<A, NA>(acc, DOTS ? nv : 0, true, mmax, partial + (size_t)bx * (mmax + 1) * 2);
+    fused_epilogue<A, NV>(acc, nv, true, mmax, partial + (size_t)bx * (mmax + 1) * 2);
 }
 
 template <class A>
@@ -987,13 +929,8 @@ __global__ void __launch_bounds__(kT, 2) eng_update_fused(const SlotDev* __restr
     __syncthreads();
     const int64_t lb = bx - S.rb_begin;
     const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
-    if (!S.shift) {
-        if (nv <= 12) update_fused_rows<A, 12, true>(S, r0, r1, nv, hs, mmax, partial, bx);
-        else update_fused_rows<A, 20, true>(S, r0, r1, nv, hs, mmax, partial, bx);
-    } else {
-        if (nv <= 12) update_fused_rows<A, 12, false>(S, r0, r1, nv, hs, mmax, partial, bx);
-        else update_fused_rows<A, 20, false>(S, r0, r1, nv, hs, mmax, partial, bx);
-    }
+    if (nv <= 12) update_fused_rows<A, 12>(S, r0, r1, nv, hs, mmax, partial, bx);
+    else update_fused_rows<A, 20>(S, r0, r1, nv, hs, mmax, partial, bx);
 }
 
 // ------------------------------------------------------------ scale
@@ -1484,7 +1421,6 @@ int Engine::add(Op& op, int m, bool cv, int tmp_cols, int orth) {
     d.state = kSlotIdle;
     d.carry = -1;
     d.orth = orth;
-    d.shift = orth == 1 && op.hermitian && st_ != Store::F32;
     sl.tcols = tc;
     const Tiles t = tiles_for(n, M.nslices);
     d.rpb = t.rpb;
@@ -1512,7 +1448,7 @@ void Engine::remove(int id) {
 void Engine::build_maps() {
     nrb_ = nsb_ = 0;
     mmax_ = dmax_ = 1;
-    cgs_ = shift_ = false;
+    cgs_ = false;
     for (auto& sl : slots_) {
         SlotDev& d = sl.d;
         if (!sl.live) {
@@ -1529,7 +1465,6 @@ void Engine::build_maps() {
         mmax_ = std::max(mmax_, d.m);
         dmax_ = std::max(dmax_, d.orth == 2 ? 1 : d.m);
         cgs_ = cgs_ || d.orth != 2;
-        shift_ = shift_ || d.shift;
     }
     std::vector<int> rm(std::max(1, nrb_)), sm(std::max(1, nsb_));
     for (int i = 0; i < (int)slots_.size(); ++i) {
@@ -1594,7 +1529,7 @@ static bool fused_update_on() {
 
 template <class A>
 static int launch_step_t(const SlotDev* ds, SlotDev* dsw, const int* rm, const int* sm, double* pa, const void* rsq,
-                         int nrb, int nsb, int mmax, int dmax, bool cgs, bool shift, int ns, cudaStream_t s) {
+                         int nrb, int nsb, int mmax, int dmax, bool cgs, int ns, cudaStream_t s) {
     const dim3 gd(nrb, (dmax + jt<A>() - 1) / jt<A>());
     const bool fused = fused_update_on() && cgs;
     eng_spmv<A><<<nsb, kT, 0, s>>>(ds, sm, rsq);
@@ -1609,11 +1544,6 @@ static int launch_step_t(const SlotDev* ds, SlotDev* dsw, const int* rm, const i
     int n = 6;
     if (cgs) {
         // the second pass, where a step asks for it
-        if (shift) {
-            if (fused) eng_dots_fused<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 1, pa);
-            else eng_dots<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 1, pa);
-            ++n;
-        }
         eng_reduce<<<dim3(ns, mmax), kT, 0, s>>>(dsw, mmax, 2, pa, 0, false);
         eng_update<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, 1, pa);
         eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 3, pa, 0, true);
@@ -1674,14 +1604,11 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
     const int64_t s0 = Ls.nslices * (int64_t)rank / C, s1 = Ls.nslices * (int64_t)(rank + 1) / C;
     const int64_t r0 = min(Ls.n, s0 * kSellSlice), r1 = min(Ls.n, s1 * kSellSlice);
     int j = Ls.j;
-    // the shift of a step (Shift): every CTA has the coefficients
-    Shift<A> sh = step_shift<A>(Ls);
-    double sigma = to_d(sh.sigma), beta = to_d(sh.beta);
     for (int step = 0; step < nsteps && j < m; ++step) {
         if (threadIdx.x == 0) Ls.j = j;
         __syncthreads();
         // product over this CTA's slices: col(j + 1) = H col(j)
-        spmv_slices<A>(Ls, s0, s1, tab, smem_tab, rsq, sh);
+        spmv_slices<A>(Ls, s0, s1, tab, smem_tab, rsq);
         __syncthreads();
         // first-pass dots over this CTA's rows (and ||w||^2 for DGKS)
         const int nv = j + 1;
@@ -1730,7 +1657,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             }
         }
         __syncthreads();
-        // pass 0: w' = w - V h1 over this CTA's rows, ||w'||^2 and (unshifted
+        // pass 0: w' = w - V h1 over this CTA's rows, ||w'||^2 and (Gram-Schmidt
         // slots) the second-pass dots V^* w'
         const int first_u = orth == 2 ? (j > 0 ? j - 1 : 0) : 0;
         for (int t = first_u + threadIdx.x; t < nv; t += blockDim.x)
@@ -1742,7 +1669,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             const double t = block_sum(nacc, shb);
             if (threadIdx.x == 0) part2[m * 2] = t;
         }
-        auto second_dots = [&]() {
+        if (orth != 2) {
             for (int c0 = 0; c0 < nv; c0 += jt<A>()) {
                 A re[jt<A>()], im[jt<A>()], dummy = zero<A>();
 #pragma unroll
@@ -1750,8 +1677,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
                 dots_rows<A, CV>(Ls, r0, r1, c0, nv, w, re, im, false, dummy);
                 dots_epilogue<A>(re, im, CV, c0, nv, c0, part2);
             }
-        };
-        if (orth != 2 && !Ls.shift) second_dots();
+        }
         cl_sync();
         if (threadIdx.x == 0) {
             double t = 0;
@@ -1763,21 +1689,14 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
         }
         __syncthreads();
         double2* col = Ls.rec + (size_t)j * ld;
-        double nb = scal[1], alpha = h1[j * 2];
+        double nb = scal[1];
         if (scal[2] == 0.0) {
             if (rank == 0 && threadIdx.x == 0) {
-                for (int q = first_u; q <= j; ++q) {
-                    const double part = q == j ? sigma : (q == j - 1 ? beta : 0.0);
-                    col[q] = make_double2(h1[q * 2] + part, h1[q * 2 + 1]);
-                }
+                for (int q = first_u; q <= j; ++q) col[q] = make_double2(h1[q * 2], h1[q * 2 + 1]);
                 col[j + 1] = make_double2(nb, 0.0);
             }
         } else {
             // second pass: w'' = w' - V h2, the record column h1 + h2
-            if (Ls.shift) {
-                second_dots();
-                cl_sync();
-            }
             for (int i = threadIdx.x; i <= j; i += blockDim.x) {
                 double re = 0, im = 0;
                 for (uint32_t r = 0; r < C; ++r) {
@@ -1788,12 +1707,9 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
                 h2[i * 2 + 1] = im;
             }
             __syncthreads();
-            alpha += h2[j * 2];
             if (rank == 0)
-                for (int i = threadIdx.x; i <= j; i += blockDim.x) {
-                    const double part = i == j ? sigma : (i == j - 1 ? beta : 0.0);
-                    col[i] = make_double2(h1[i * 2] + h2[i * 2] + part, h1[i * 2 + 1] + h2[i * 2 + 1]);
-                }
+                for (int i = threadIdx.x; i <= j; i += blockDim.x)
+                    col[i] = make_double2(h1[i * 2] + h2[i * 2], h1[i * 2 + 1] + h2[i * 2 + 1]);
             for (int t = threadIdx.x; t < nv; t += blockDim.x)
                 hs[t] = CA<A>{from_d<A>(h2[t * 2]), from_d<A>(h2[t * 2 + 1])};
             __syncthreads();
@@ -1809,11 +1725,6 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             }
             __syncthreads();
             nb = scal[1];
-        }
-        if (Ls.shift) {
-            sigma = (double)(float)(alpha + sigma);
-            beta = (double)(float)nb;
-            sh = Shift<A>{true, from_d<A>(sigma), from_d<A>(beta)};
         }
         // col(j + 1) /= beta over this CTA's rows
         const A f = from_d<A>(nb > 0 ? 1.0 / nb : 0.0);
@@ -1959,7 +1870,6 @@ __global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3)
         QS_PHASE(nrb, update_block<A>(sl, rm, mmax, 0, pa, v));
         QS_PHASE(ns, reduce_block(sl, mmax, 1, pa, 0, v, 0, !cgs));
         if (cgs) {
-            QS_PHASE(nrb * ydots, dots_block<A>(sl, rm, mmax, 1, pa, v % nrb, v / nrb));
             QS_PHASE(ns * mmax, reduce_block(sl, mmax, 2, pa, 0, v % ns, v / ns, false));
             QS_PHASE(nrb, update_block<A>(sl, rm, mmax, 1, pa, v));
             QS_PHASE(ns, reduce_block(sl, mmax, 3, pa, 0, v, 0, true));
@@ -1984,7 +1894,7 @@ void Engine::launch_step() {
         using A = decltype(tag);
         step_launches_ = launch_step_t<A>(dslots_.as<SlotDev>(), dslots_.as<SlotDev>(), rmap_.as<int>(),
                                           smap_.as<int>(), partial_.as<double>(), rsq, nrb_, nsb_, mmax_, dmax_,
-                                          cgs_, shift_, ns, s_);
+                                          cgs_, ns, s_);
     });
 }
 
@@ -2113,9 +2023,10 @@ void grid_barrier_check(int phantom, double limit_ms, int blocks) {
 // slot and the storage, so that a slot's result is the same alone and in any
 // batch.  Up to 8,192 rows eight CTAs win everywhere (2,703 rows, ground state:
 // 3.4 against 4.5 ms on the graph replay).  Above, sixteen CTAs save the launch
-// gaps of ten kernels a step but have 16 SMs' FP64 rate, where the graph spreads a
+// gaps of nine kernels a step but have 16 SMs' FP64 rate, where the graph spreads a
 // slot over all of them; so the limit is where the work of a row overtakes the
-// gaps (ground states on GB300, cluster / graph in ms):
+// gaps (ground states on GB300, one Gram-Schmidt pass on most steps, cluster / graph
+// in ms):
 //   real matrix:  14,310 rows 3.4/3.8, 19,448 rows 3.6/3.8, 24,310 rows 4.05/3.83,
 //                 28,968 rows 6.5/4.6; evolution 16,384 rows 6.6/7.6, 32,768 9.2/8.5
 //   complex, FP64 (four multiply-adds an entry on the FP64 pipe):

@@ -1,9 +1,9 @@
 // qs_engine.h -- the batched Krylov engine: many Krylov processes ("slots"),
 // each on its own assembled operator and its own vectors, advanced together.
 //
-// One Lanczos/Arnoldi step of every stepping slot is a fixed sequence of ten
-// launches (SpMV; dots + reduce; the update with the norm + reduce; the second
-// Gram-Schmidt pass where a step asks for it: dots + reduce, update + reduce;
+// One Lanczos/Arnoldi step of every stepping slot is a fixed sequence of nine
+// launches (SpMV; dots + reduce; the update with the norm and the next dots +
+// reduce; the second Gram-Schmidt pass where a step asks for it: reduce, update + reduce;
 // scale; six when every slot runs the three-term recurrence), each
 // covering all slots through a block -> slot map.  The step
 // counters live on the device, so the sequence is captured once in a CUDA
@@ -76,7 +76,6 @@ struct SlotDev {
     // dsaitr test); 2 Lanczos three-term recurrence (Hermitian operators,
     // the reference's Krylov exponential)
     int32_t orth;
-    int32_t shift;          // steps take the known part of the recurrence out in the product (Shift)
     // rotation: V[:, out0 + c] = sum_{i < rot_in} V[:, i] Y[i, c] for c < p, then
     // V[:, cdst] = V[:, carry] when carry >= 0
     int32_t rot_in, p, out0, carry, cdst;
@@ -193,8 +192,8 @@ class Engine {
     // most vectors any slot dots against in a step (1 for three-term slots,
     // m for Gram-Schmidt ones) and whether any slot takes a second pass
     int dmax_ = 1;
-    bool cgs_ = false, shift_ = false;
-    int step_launches_ = 10;
+    bool cgs_ = false;
+    int step_launches_ = 9;
     size_t cap_partial_ = 0, cap_rmap_ = 0, cap_smap_ = 0;
     bool dirty_ = true, maps_dirty_ = true;
     cudaGraph_t graph_ = nullptr;

@@ -1,6 +1,6 @@
-"""The shifted Lanczos step (the product takes out alpha_{j-1} v_j + beta_{j-1}
-v_{j-1}) on both step forms, real and complex, single and restarted: the Ritz
-values against the dense spectrum and the vectors' residuals."""
+"""Extremal pairs on both step forms, real and complex, with and without a large
+constant on the diagonal: the Ritz values against the dense spectrum and the
+vectors' residuals."""
 import numpy as np
 import pytest
 
