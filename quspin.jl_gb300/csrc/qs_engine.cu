@@ -27,7 +27,8 @@ namespace qs {
 
 namespace {
 
-constexpr int kT = 256;       // threads per block
+constexpr int kT = 256;       // threads per block; lanes of a row block
+constexpr int kRowT = 32;     // threads per block of the vector kernels
 // vectors per dots block (eight measured slower than four for FP64 on GB300:
 // the dots are FP64-pipe bound, and the larger tile needs twice the
 // registers)
@@ -253,20 +254,47 @@ __global__ void __launch_bounds__(kT, 5) eng_spmv(const SlotDev* __restrict__ sl
     spmv_block<A>(sl, smap, rsqt, blockIdx.x);
 }
 
+// ------------------------------------------------------------ rows of a block
+// A row block's sums: eight warps, lane l of warp w adds rows 32 w + l, + kT,
+// + 2 kT, ... in ascending order, the lanes' sums meet in a butterfly, the
+// warps' in ascending order, the blocks' in eng_reduce.  That order is the
+// slot's alone and fixes every bit of a solve; who does the additions is
+// free: a CTA of the vector kernels holds blockDim.x / 32 of a block's warps,
+// and each warp leaves its own partial sums.  The 88 blocks of 358,584 rows
+// are 704 warps: in CTAs of kRowT = 32 threads 4 or 5 to an SM (64: 4 or 6, a
+// ground state 16.2 against 15.3 ms, with V read once per pass; 256: 64 of
+// 152 SMs idle); with the columns in tiles of their own (fused_slot) 12.8 ms.
+struct RowSpan {
+    int64_t r, r1;   // this lane's first row, the block's end
+    int rb, wid;     // the block among all slots', the warp in it
+    // the warp's partial sums: of index i at sums(...)[(2 i + {re, im}) * 8]
+    __device__ double* sums(double* partial, int mmax) const {
+        return partial + (size_t)rb * (mmax + 1) * 2 * (kT / 32) + wid;
+    }
+};
+__device__ __forceinline__ int row_block(int bx) { return bx / (kT / (int)blockDim.x); }
+__device__ __forceinline__ RowSpan row_span(const SlotDev& S, int bx) {
+    const int parts = kT / (int)blockDim.x;
+    const int rb = bx / parts, t = (bx % parts) * (int)blockDim.x + (int)threadIdx.x;
+    const int64_t r0 = (int64_t)(rb - S.rb_begin) * S.rpb;
+    return RowSpan{r0 + t, min(S.n, r0 + S.rpb), rb, t / 32};
+}
+
 // ------------------------------------------------------------ dots
-// Partial sums per row block b live at partial[(b * P + i) * 2 + {re, im}],
-// P = mmax + 1; index mmax holds norms.
+// Partial sums of a block and an index i (a vector's, or mmax: norms) lie
+// together, the eight warps' re, then their im (RowSpan::sums).
 // mode 0 (first pass): i in [first, j] with first = j for the three-term
 //   recurrence, else 0; DGKS slots also accumulate ||w||^2 at index mmax;
-// (the second pass's dots come from the first update, see eng_update)
-// mode 2 (normalise): partial[b][0] = <col ncol, col ncol>.
+// mode 1 (after the first update): the second pass's dots, and ||w'||^2 at mmax;
+// mode 2 (normalise): <col ncol, col ncol> at index 0;
+// mode 3 (after the second update, where it ran): ||w''||^2 at mmax.
+// (r: the lane's first row; step: kT)
 template <class A, bool CV>
-__device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r0, int64_t r1, int i0, int nv, const void* w,
+__device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r, int64_t r1, int64_t step, int i0, int nv, const void* w,
                                           A* re, A* im, bool want_wn, A& wn) {
     const int64_t n = S.n;
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)n * vbytes<A, CV>();
-    const int64_t step = blockDim.x;
     if (nv - i0 == 1) {
         // one vector (a three-term step, a normalisation, the first CGS step):
         // four rows' loads of w and the column in flight, nothing else read
@@ -283,7 +311,6 @@ __device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r0, int64_t 
                 if (CV) mac(wn, wv.im, wv.im);
             }
         };
-        int64_t r = r0 + threadIdx.x;
         for (; r + 3 * step < r1; r += 4 * step) {
             CA<A> wv[4], v[4];
 #pragma unroll
@@ -321,7 +348,6 @@ __device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r0, int64_t 
     };
     // real vectors: two rows per iteration, 2 (jt<A>() + 1) loads issued before the
     // arithmetic; complex vectors hold twice the data per row, one row at a time
-    int64_t r = r0 + threadIdx.x;
     for (; !CV && r + step < r1; r += 2 * step) {
         const CA<A> w0 = ldv<A, CV>(w, r), w1 = ldv<A, CV>(w, r + step);
         CA<A> v0[jt<A>()], v1[jt<A>()];
@@ -343,11 +369,17 @@ __device__ __forceinline__ void dots_rows(const SlotDev& S, int64_t r0, int64_t 
 }
 
 template <class A>
-__device__ __forceinline__ double block_sum(A v, double* sh) {
+__device__ __forceinline__ double warp_sum(A v) {
     for (int o = 16; o > 0; o >>= 1) v = add(v, shfl(v, o));
+    return to_d(v);
+}
+// block totals (the cluster step)
+template <class A>
+__device__ __forceinline__ double block_sum(A v, double* sh) {
+    const double s = warp_sum(v);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __syncthreads();
-    if (lane == 0) sh[wid] = to_d(v);
+    if (lane == 0) sh[wid] = s;
     __syncthreads();
     // only the first warp: a warp's FP64 add takes its SM's pipe 16 cycles
     double t = 0;
@@ -439,17 +471,47 @@ __device__ __forceinline__ void dots_epilogue(A* re, A* im, bool cv, int i0, int
     }
 }
 
-// The fused kernels' block sums: accumulators 0 .. nv-1 into their vectors'
-// partials and accumulator NV (a norm, when kept) into partial index mmax.
-template <class A, int NV>
-__device__ __forceinline__ void fused_epilogue(A (&acc)[NV + 1], int nv, bool norm, int mmax, double* row) {
-    const double t = block_totals<A, NV + 1>(acc);
-    const int i = threadIdx.x;
-    const int at = i < nv ? i : (i == NV && norm ? mmax : -1);
-    if (i <= NV && at >= 0) {
-        row[at * 2] = t;
-        row[at * 2 + 1] = 0.0;
+// A warp's sums into its partials (row): those of dots_epilogue (imaginary
+// parts of complex Gram-Schmidt slots alone) ...
+constexpr int kW = kT / 32;
+template <class A>
+__device__ __forceinline__ void warp_dots(A* re, A* im, bool cv, int i0, int nv, int base, double* row) {
+    constexpr int J = jt<A>();
+    const int lane = threadIdx.x & 31;
+    if (cv) {
+        A v[2 * J];
+#pragma unroll
+        for (int q = 0; q < J; ++q) {
+            v[2 * q] = re[q];
+            v[2 * q + 1] = im[q];
+        }
+        halve_sums<A, 2 * J, 16>(v, lane);
+        const int pos = halve_pos<2 * J>(lane);
+        if (pos >= 0 && i0 + pos / 2 < nv) row[(base * 2 + pos) * kW] = to_d(v[0]);
+    } else {
+        A v[J];
+#pragma unroll
+        for (int q = 0; q < J; ++q) v[q] = re[q];
+        halve_sums<A, J, 16>(v, lane);
+        const int pos = halve_pos<J>(lane);
+        if (pos >= 0 && i0 + pos < nv) row[(base + pos) * 2 * kW] = to_d(v[0]);
     }
+}
+// ... the fused kernels': accumulators 0 .. nv-1 of their vectors and
+// accumulator NV (a norm, when kept) at index mmax ...
+template <class A, int NV>
+__device__ __forceinline__ void warp_fused(A (&acc)[NV + 1], int nv, bool norm, int mmax, double* row) {
+    const int lane = threadIdx.x & 31;
+    halve_sums<A, NV + 1, 16>(acc, lane);
+    const int i = halve_pos<NV + 1>(lane);
+    const int at = i < 0 ? -1 : i < nv ? i : (i == NV && norm ? mmax : -1);
+    if (at >= 0) row[at * 2 * kW] = to_d(acc[0]);
+}
+// ... and one real sum
+template <class A>
+__device__ __forceinline__ void warp_one(A v, int at, double* row) {
+    const double t = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) row[at * 2 * kW] = t;
 }
 
 // Three-term slots (Hermitian, no reorthogonalisation): alpha = <v_j, w> and
@@ -457,7 +519,7 @@ __device__ __forceinline__ void fused_epilogue(A (&acc)[NV + 1], int nv, bool no
 // multiply-adds a row instead of four and the update four instead of ten (the
 // imaginary parts are rounding).
 template <class A, bool CV>
-__device__ __forceinline__ A three_dot_rows(const SlotDev& S, int64_t r0, int64_t r1) {
+__device__ __forceinline__ A three_dot_rows(const SlotDev& S, int64_t r, int64_t r1, int64_t step) {
     const void* w = colp<A>(S, S.j + 1);
     const void* v = colp<A>(S, S.j);
     A acc = zero<A>();
@@ -465,8 +527,6 @@ __device__ __forceinline__ A three_dot_rows(const SlotDev& S, int64_t r0, int64_
         mac(acc, a.re, b.re);
         if (CV) mac(acc, a.im, b.im);
     };
-    const int64_t step = blockDim.x;
-    int64_t r = r0 + threadIdx.x;
 #pragma unroll 1
     for (; r + step < r1; r += 2 * step) {
         const CA<A> a0 = ldv<A, CV>(v, r), a1 = ldv<A, CV>(v, r + step);
@@ -480,7 +540,7 @@ __device__ __forceinline__ A three_dot_rows(const SlotDev& S, int64_t r0, int64_
 }
 // w -= alpha v_j + beta v_{j-1}; returns the part of ||w||^2
 template <class A, bool CV>
-__device__ __forceinline__ A three_update_rows(const SlotDev& S, int64_t r0, int64_t r1, A alpha, A beta) {
+__device__ __forceinline__ A three_update_rows(const SlotDev& S, int64_t r, int64_t r1, int64_t step, A alpha, A beta) {
     void* w = colp<A>(S, S.j + 1);
     const void* v = colp<A>(S, S.j);
     const bool two = S.j > 0;
@@ -497,8 +557,6 @@ __device__ __forceinline__ A three_update_rows(const SlotDev& S, int64_t r0, int
         if (CV) mac(nacc, o.im, o.im);
         return o;
     };
-    const int64_t step = blockDim.x;
-    int64_t r = r0 + threadIdx.x;
 #pragma unroll 1
     for (; r + step < r1; r += 2 * step) {
         const CA<A> o0 = ldv<A, CV>(w, r), o1 = ldv<A, CV>(w, r + step);
@@ -511,130 +569,141 @@ __device__ __forceinline__ A three_update_rows(const SlotDev& S, int64_t r0, int
     for (; r < r1; r += step) stv<A, CV>(w, r, one(ldv<A, CV>(w, r), ldv<A, CV>(v, r), ldv<A, CV>(u, r)));
     return nacc;
 }
-template <class A, bool UPDATE>
+// kOne: a CTA of kT threads leaves the block's total in its first warp's place.
+template <class A, bool UPDATE, bool kOne = false>
 __device__ __forceinline__ void three_block(const SlotDev& S, int mmax, double* partial, int bx) {
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
+    const RowSpan R = row_span(S, bx);
     A acc;
     if (UPDATE) {
         const A alpha = from_d<A>(S.h1[S.j].x), beta = S.j > 0 ? from_d<A>(S.h1[S.j - 1].x) : zero<A>();
-        acc = S.cv ? three_update_rows<A, true>(S, r0, r1, alpha, beta) : three_update_rows<A, false>(S, r0, r1, alpha, beta);
+        acc = S.cv ? three_update_rows<A, true>(S, R.r, R.r1, kT, alpha, beta)
+                   : three_update_rows<A, false>(S, R.r, R.r1, kT, alpha, beta);
     } else {
-        acc = S.cv ? three_dot_rows<A, true>(S, r0, r1) : three_dot_rows<A, false>(S, r0, r1);
+        acc = S.cv ? three_dot_rows<A, true>(S, R.r, R.r1, kT) : three_dot_rows<A, false>(S, R.r, R.r1, kT);
     }
-    __shared__ double sh[kT / 32];
-    const double t = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-        double* at = partial + ((size_t)bx * (mmax + 1) + (UPDATE ? mmax : S.j)) * 2;
-        at[0] = t;
-        at[1] = 0.0;
+    const int at = UPDATE ? mmax : S.j;
+    if constexpr (kOne) {
+        __shared__ double sh[kW];
+        const double t = block_sum(acc, sh);
+        if (threadIdx.x == 0) R.sums(partial, mmax)[at * 2 * kW] = t;
+    } else {
+        warp_one(acc, at, R.sums(partial, mmax));
     }
 }
-// The dots or the update of an engine whose slots are all three-term:
-// four blocks an SM, where the Gram-Schmidt kernels with their columns in registers
-// hold two or three.
+// The dots or the update of an engine whose slots are all three-term: four
+// blocks an SM, where the Gram-Schmidt kernels with their columns in registers
+// hold two or three, and one sum per block for the reductions.
 template <class A, bool UPDATE>
 __global__ void __launch_bounds__(kT, 4) eng_three(const SlotDev* __restrict__ sl, const int* __restrict__ rmap,
                                                    int mmax, double* __restrict__ partial) {
     const SlotDev& S = sl[rmap[blockIdx.x]];
-    if (S.state == kSlotStep) three_block<A, UPDATE>(S, mmax, partial, blockIdx.x);
+    if (S.state == kSlotStep) three_block<A, UPDATE, true>(S, mmax, partial, blockIdx.x);
 }
 
 template <class A>
 __device__ __forceinline__ void dots_block(const SlotDev* sl, const int* __restrict__ rmap, int mmax, int mode,
                                            double* partial, int bx, int by) {
-    const SlotDev& S = sl[rmap[bx]];
+    const SlotDev& S = sl[rmap[row_block(bx)]];
     if (S.state != (mode == 2 ? kSlotNormalize : kSlotStep)) return;
-    if (mode == 0 && S.orth == 2) {
-        if (by == 0) three_block<A, false>(S, mmax, partial, bx);
+    if (mode != 2 && S.orth == 2) {
+        if (mode == 0 && by == 0) three_block<A, false>(S, mmax, partial, bx);
         return;
     }
-    const int P = mmax + 1;
-    const int first = mode == 2 ? S.ncol : 0;
-    const int nv = (mode == 2 ? S.ncol : S.j) + 1;
-    const void* w = colp<A>(S, mode == 2 ? S.ncol : S.j + 1);
+    if (mode == 3 && S.nrm[4] == 0.0) return;
+    // modes 2 and 3: a column with itself
+    const bool self = mode >= 2;
+    const int wc = mode == 2 ? S.ncol : S.j + 1;
+    const int first = self ? wc : 0, nv = self ? wc + 1 : S.j + 1;
+    const void* w = colp<A>(S, wc);
     const int i0 = first + by * jt<A>();
     if (i0 >= nv) return;
-    const bool want_wn = mode == 0 && S.orth == 1 && by == 0;
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
+    const bool want_wn = by == 0 && (mode == 1 || (mode == 0 && S.orth == 1));
+    const RowSpan R = row_span(S, bx);
+    double* row = R.sums(partial, mmax);
     A re[jt<A>()], im[jt<A>()], wn = zero<A>();
 #pragma unroll
     for (int q = 0; q < jt<A>(); ++q) re[q] = im[q] = zero<A>();
-    if (S.cv) dots_rows<A, true>(S, r0, r1, i0, nv, w, re, im, want_wn, wn);
-    else dots_rows<A, false>(S, r0, r1, i0, nv, w, re, im, want_wn, wn);
-    dots_epilogue<A>(re, im, S.cv, i0, nv, mode == 2 ? 0 : i0, partial + (size_t)bx * P * 2);
-    if (want_wn) {
-        __shared__ double sw[kT / 32];
-        const double t = block_sum(wn, sw);
-        if (threadIdx.x == 0) {
-            partial[((size_t)bx * P + mmax) * 2] = t;
-            partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
-        }
+    if (S.cv) dots_rows<A, true>(S, R.r, R.r1, kT, i0, nv, w, re, im, want_wn, wn);
+    else dots_rows<A, false>(S, R.r, R.r1, kT, i0, nv, w, re, im, want_wn, wn);
+    if (self) {
+        warp_one(re[0], mode == 2 ? 0 : mmax, row);
+    } else {
+        warp_dots<A>(re, im, S.cv, i0, nv, i0, row);
+        if (want_wn) warp_one(wn, mmax, row);
     }
 }
 
 template <class A>
-__global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3) eng_dots(const SlotDev* __restrict__ sl, const int* __restrict__ rmap, int mmax,
+__global__ void __launch_bounds__(kRowT, (std::is_same<A, DF>::value ? 1024 : 768) / kRowT) eng_dots(const SlotDev* __restrict__ sl, const int* __restrict__ rmap, int mmax,
                                                int mode, double* __restrict__ partial) {
+    if (mode != 2 && sl[rmap[row_block(blockIdx.x)]].fused) return;
     dots_block<A>(sl, rmap, mmax, mode, partial, blockIdx.x, blockIdx.y);
 }
 
 // First-pass dots of a real Gram-Schmidt slot with 2 <= nv <= 20 vectors in
-// one block per row block: each row's w and nv vector entries are loaded once
-// (all loads before the arithmetic) and every column's sum advances, where
-// eng_dots reads w once per tile of jt columns.  Per thread the rows and the
+// one pass: each row's w and nv vector entries are loaded once and every
+// column's sum advances, where eng_dots reads w once per tile of jt columns.
+// A lane has 16 rows and an SM few warps, so the next row is on its way while
+// this one is added.  Per thread the rows and the
 // multiply-add order of each column's sum and of ||w||^2 are those of
-// dots_rows, and the block sums add in the order of dots_epilogue / block_sum,
-// so the partials are bit-identical to dots_block's.
+// dots_rows, and the warp sums add in the order of warp_dots, so the partials
+// are bit-identical to dots_block's.
 template <class A, int NV>
-__device__ __forceinline__ void dots_fused_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const void* w,
-                                                bool want_wn, int mmax, double* partial, int bx) {
+struct FusedRow {
+    A v[NV], w;
+    __device__ __forceinline__ void load(const char* V, size_t cs, int nv, const void* wc, int64_t r) {
+#pragma unroll
+        for (int t = 0; t < NV; ++t)
+            if (t < nv) v[t] = ldv<A, false>(V + (size_t)t * cs, r).re;
+        w = ldv<A, false>(wc, r).re;
+    }
+};
+template <class A, int NV>
+__device__ __forceinline__ void dots_fused_rows(const SlotDev& S, const RowSpan& R, int nv, const void* w,
+                                                bool want_wn, int mmax, double* row) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, false>();
     A acc[NV + 1];   // the dots, then ||w||^2
 #pragma unroll
     for (int t = 0; t <= NV; ++t) acc[t] = zero<A>();
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-        A v[NV];
+    FusedRow<A, NV> cur, next;
+    if (R.r < R.r1) cur.load(V, cs, nv, w, R.r);
+    for (int64_t r = R.r; r < R.r1; r += kT) {
+        if (r + kT < R.r1) next.load(V, cs, nv, w, r + kT);
 #pragma unroll
         for (int t = 0; t < NV; ++t)
-            if (t < nv) v[t] = ldv<A, false>(V + (size_t)t * cs, r).re;
-        const A wr = ldv<A, false>(w, r).re;
-#pragma unroll
-        for (int t = 0; t < NV; ++t)
-            if (t < nv) mac(acc[t], v[t], wr);
-        if (want_wn) mac(acc[NV], wr, wr);
+            if (t < nv) mac(acc[t], cur.v[t], cur.w);
+        if (want_wn) mac(acc[NV], cur.w, cur.w);
+        cur = next;
     }
-    fused_epilogue<A, NV>(acc, nv, want_wn, mmax, partial + (size_t)bx * (mmax + 1) * 2);
+    warp_fused<A, NV>(acc, nv, want_wn, mmax, row);
 }
 
 template <class A>
-__global__ void __launch_bounds__(kT, 2) eng_dots_fused(const SlotDev* __restrict__ sl, const int* __restrict__ rmap,
-                                                        int mmax, int mode, double* __restrict__ partial) {
-    const int bx = blockIdx.x, by = blockIdx.y;
-    const SlotDev& S = sl[rmap[bx]];
-    if (S.state != kSlotStep) return;
+__global__ void __launch_bounds__(kRowT, 384 / kRowT)
+    eng_dots_fused(const SlotDev* __restrict__ sl, const int* __restrict__ rmap, int mmax, double* __restrict__ partial) {
+    const int bx = blockIdx.x;
+    const SlotDev& S = sl[rmap[row_block(bx)]];
+    if (S.state != kSlotStep || !S.fused) return;
     const int nv = S.j + 1;
-    if (S.cv || S.orth == 2 || nv < 2 || nv > 20) {
-        dots_block<A>(sl, rmap, mmax, mode, partial, bx, by);
+    if (nv < 2 || nv > 20) {
+        for (int by = 0; by * jt<A>() < nv; ++by) dots_block<A>(sl, rmap, mmax, 0, partial, bx, by);
         return;
     }
-    if (by) return;
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
+    const RowSpan R = row_span(S, bx);
+    double* row = R.sums(partial, mmax);
     const void* w = colp<A>(S, S.j + 1);
-    const bool want_wn = mode == 0 && S.orth == 1;
-    if (nv <= 12) dots_fused_rows<A, 12>(S, r0, r1, nv, w, want_wn, mmax, partial, bx);
-    else dots_fused_rows<A, 20>(S, r0, r1, nv, w, want_wn, mmax, partial, bx);
+    if (nv <= 12) dots_fused_rows<A, 12>(S, R, nv, w, S.orth == 1, mmax, row);
+    else dots_fused_rows<A, 20>(S, R, nv, w, S.orth == 1, mmax, row);
 }
 
 // ------------------------------------------------------------ reduce
-// Per slot and vector, the block partials summed in a fixed order, then:
+// Per slot and vector, the warps' partials summed in a fixed order (those of a
+// block, then the blocks), then:
 // mode 0: h1 (and ||w||^2; the three-term recurrence takes beta_{j-1} from the record)
-// mode 1: ||w'||^2 after the first pass; decides the second pass; without it the
-//         step's record column and norm are final
-// mode 2: h2 and the record column h1 + h2 (second pass only)
+// mode 1: ||w'||^2 after the first pass, which decides the second; without it the
+//         step's record column and norm are final, with it h2 and the record
+//         column h1 + h2 (each vector's block takes the norm and the decision itself)
 // mode 3: ||w''||^2 (second pass only)
 // mode 4: norm of the normalised column
 // `last`: the step's last reduction (mode 3, or mode 1 without Gram-Schmidt
@@ -644,10 +713,51 @@ __device__ __forceinline__ void advance_slot(SlotDev& S) {
     S.j += 1;
     if (S.j >= S.m) S.state = kSlotHold;
 }
+// The slot's sums of index i (thread 0 of the block returns them); one: a
+// block's total is in its first warp's place.
+__device__ __forceinline__ double2 reduce_sums(const SlotDev& S, const double* partial, int mmax, int i, bool one) {
+    const bool cx = S.cv && S.orth != 2 && i != mmax;
+    double re = 0, im = 0;
+    for (int b = threadIdx.x; b < S.rb_count; b += blockDim.x) {
+        const double* at = partial + ((size_t)(S.rb_begin + b) * (mmax + 1) + i) * 2 * kW;
+        if (one) {
+            re += at[0];
+            continue;
+        }
+        double tr = 0, ti = 0;
+#pragma unroll
+        for (int q = 0; q < kW; ++q) tr += at[q];
+        if (cx) {
+#pragma unroll
+            for (int q = 0; q < kW; ++q) ti += at[kW + q];
+        }
+        re += tr;
+        im += ti;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, o);
+        im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+    __shared__ double sr[kT / 32], si[kT / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __syncthreads();   // (an earlier call's readers are done)
+    if (lane == 0) {
+        sr[wid] = re;
+        si[wid] = im;
+    }
+    __syncthreads();
+    re = im = 0;
+    if (threadIdx.x == 0)
+        for (int q = 0; q < kT / 32; ++q) {
+            re += sr[q];
+            im += si[q];
+        }
+    return make_double2(re, im);
+}
 __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, const double* partial, int dy,
-                                             int bx, int by, bool last) {
+                                             int bx, int by, bool last, bool one) {
     SlotDev& S = sl[bx];
-    int i = by;
+    int i = by;   // the vector; mmax: a norm
     if (mode == 4) {
         if (S.state != kSlotNormalize || i) return;
     } else {
@@ -656,7 +766,7 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
             if (last && S.state == kSlotHold && i == 0 && threadIdx.x == 0) S.nrm[6] = 0.0;
             return;
         }
-        if ((mode == 2 || mode == 3) && S.nrm[4] == 0.0) {
+        if (mode == 3 && S.nrm[4] == 0.0) {
             if (last && i == 0 && threadIdx.x == 0) advance_slot(S);
             return;
         }
@@ -671,69 +781,48 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
                 i += first;
                 if (i > S.j) return;
             }
-        } else if (mode == 1 || mode == 3) {
-            if (i) return;
-            i = mmax;
-        } else if (i > S.j) {
-            return;
+        } else {
+            // the norm first, then (mode 1) the second pass's vectors
+            if (i && (mode == 3 || S.orth == 2 || i - 1 > S.j)) return;
+            i = i ? i - 1 : mmax;
         }
-    }
-    const int P = mmax + 1;
-    double re = 0, im = 0;
-    for (int b = threadIdx.x; b < S.rb_count; b += blockDim.x) {
-        re += partial[((size_t)(S.rb_begin + b) * P + i) * 2];
-        im += partial[((size_t)(S.rb_begin + b) * P + i) * 2 + 1];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        re += __shfl_xor_sync(0xffffffffu, re, o);
-        im += __shfl_xor_sync(0xffffffffu, im, o);
-    }
-    __shared__ double sr[kT / 32], si[kT / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        sr[wid] = re;
-        si[wid] = im;
-    }
-    __syncthreads();
-    if (threadIdx.x) return;
-    re = im = 0;
-    for (int q = 0; q < kT / 32; ++q) {
-        re += sr[q];
-        im += si[q];
     }
     const int ld = S.m + 1;
     const int j = S.j;
     double2* col = S.rec + (size_t)j * ld;
+    const double2 t = reduce_sums(S, partial, mmax, mode == 1 ? mmax : i, one);
+    double2 h = make_double2(0.0, 0.0);
+    if (mode == 1 && i != mmax) h = reduce_sums(S, partial, mmax, i, one);
+    if (threadIdx.x) return;
+    const double nb = sqrt(fmax(t.x, 0.0));
     if (mode == 0) {
         if (i == mmax) {
-            S.nrm[3] = re;
+            S.nrm[3] = t.x;
         } else {
-            S.h1[i] = make_double2(re, im);
+            S.h1[i] = t;
             if (S.orth == 2) S.h1[j - 1 >= 0 ? j - 1 : 0] = j > 0 ? S.rec[(size_t)(j - 1) * ld + j] : S.h1[0];
         }
     } else if (mode == 1) {
-        const double nb = sqrt(fmax(re, 0.0));
         const bool second = S.orth == 0 || (S.orth == 1 && nb < 0.717 * sqrt(fmax(S.nrm[3], 0.0)));
+        if (i != mmax) {
+            if (!second) return;
+            S.h2[i] = h;
+            const double2 a = S.h1[i];
+            col[i] = make_double2(a.x + h.x, a.y + h.y);
+            return;
+        }
         S.nrm[4] = second ? 1.0 : 0.0;
         if (!second) {
             // the first pass is final: record column j and the new norm
             const int first = S.orth == 2 ? (j > 0 ? j - 1 : 0) : 0;
-            for (int q = first; q <= j; ++q) {
-                const double2 a = S.h1[q];
-                col[q] = a;
-            }
+            for (int q = first; q <= j; ++q) col[q] = S.h1[q];
             col[j + 1] = make_double2(nb, 0.0);
-            S.nrm[0] = re;
+            S.nrm[0] = t.x;
             S.nrm[1] = nb > 0 ? 1.0 / nb : 0.0;
         }
         if (last) advance_slot(S);
-    } else if (mode == 2) {
-        S.h2[i] = make_double2(re, im);
-        const double2 a = S.h1[i];
-        col[i] = make_double2(a.x + re, a.y + im);
     } else {
-        const double nb = sqrt(fmax(re, 0.0));
-        S.nrm[0] = re;
+        S.nrm[0] = t.x;
         S.nrm[1] = nb > 0 ? 1.0 / nb : 0.0;
         if (mode == 3) col[j + 1] = make_double2(nb, 0.0);
         else S.nrm[2] = nb;
@@ -742,17 +831,17 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
 }
 
 __global__ void __launch_bounds__(kT) eng_reduce(SlotDev* sl, int mmax, int mode, const double* __restrict__ partial,
-                                                 int dy, bool last) {
-    reduce_block(sl, mmax, mode, partial, dy, blockIdx.x, blockIdx.y, last);
+                                                 int dy, bool last, bool one) {
+    reduce_block(sl, mmax, mode, partial, dy, blockIdx.x, blockIdx.y, last, one);
 }
 
 // ------------------------------------------------------------ update
 // col(j+1) -= sum_i col(i) h_i over the pass's vectors (pass 0: h1, pass 1: h2,
 // over 0..j, the second only where the step's flag asks), leaving the
-// block's part of ||col(j+1)||^2 at partial[b][mmax]; pass 0 of a
-// Gram-Schmidt slot also leaves the second-pass dots at partial[b][0..j].
+// warps' parts of ||col(j+1)||^2 at partial[u][mmax]; pass 0 of a
+// Gram-Schmidt slot also leaves the second-pass dots at partial[u][0..j].
 template <class A, bool CV>
-__device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const CA<A>* hs) {
+__device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r, int64_t r1, int64_t step, int nv, const CA<A>* hs) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, CV>();
     void* w = (void*)(V + (size_t)(S.j + 1) * cs);
@@ -782,9 +871,7 @@ __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r
             if (CV) mac(nacc, o.im, o.im);
             return o;
         };
-        const int64_t step = blockDim.x;
-        int64_t r = r0 + threadIdx.x;
-        for (; r + step < r1; r += 2 * step) {
+            for (; r + step < r1; r += 2 * step) {
             const CA<A> o0 = ldv<A, CV>(w, r), o1 = ldv<A, CV>(w, r + step);
             const CA<A> a0 = ldv<A, CV>(va, r), a1 = ldv<A, CV>(va, r + step);
             const CA<A> b0 = ldv<A, CV>(vb, r), b1 = ldv<A, CV>(vb, r + step);
@@ -795,7 +882,7 @@ __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r
         for (; r < r1; r += step) stv<A, CV>(w, r, one(ldv<A, CV>(w, r), ldv<A, CV>(va, r), ldv<A, CV>(vb, r)));
         return nacc;
     }
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+    for (; r < r1; r += step) {
         A ar = zero<A>(), ai = zero<A>();
         int t = 0;
         // four vector loads in flight before their arithmetic
@@ -817,10 +904,21 @@ __device__ __forceinline__ A update_rows(const SlotDev& S, int64_t r0, int64_t r
     return nacc;
 }
 
+// the coefficients of a pass (every thread of the CTA)
+template <class A>
+__device__ __forceinline__ void load_h(const SlotDev& S, int pass, int nv, CA<A>* hs) {
+    const double2* h = pass ? S.h2 : S.h1;
+    for (int t = threadIdx.x; t < nv; t += blockDim.x) {
+        const double2 v = h[t];
+        hs[t] = CA<A>{from_d<A>(v.x), from_d<A>(v.y)};
+    }
+    __syncthreads();
+}
+
 template <class A>
 __device__ __forceinline__ void update_block(const SlotDev* sl, const int* __restrict__ rmap, int mmax, int pass,
                                              double* partial, int bx) {
-    const SlotDev& S = sl[rmap[bx]];
+    const SlotDev& S = sl[rmap[row_block(bx)]];
     if (S.state != kSlotStep) return;
     if (pass == 1 && S.nrm[4] == 0.0) return;
     if (S.orth == 2) {
@@ -829,121 +927,157 @@ __device__ __forceinline__ void update_block(const SlotDev* sl, const int* __res
     }
     __shared__ CA<A> hs[kMaxM];
     const int nv = S.j + 1;
-    const double2* h = pass ? S.h2 : S.h1;
-    for (int t = threadIdx.x; t < nv; t += blockDim.x) {
-        const double2 v = h[t];
-        hs[t] = CA<A>{from_d<A>(v.x), from_d<A>(v.y)};
-    }
-    __syncthreads();
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
-    A nacc = S.cv ? update_rows<A, true>(S, r0, r1, nv, hs) : update_rows<A, false>(S, r0, r1, nv, hs);
-    __shared__ double sh[kT / 32];
-    const double t = block_sum(nacc, sh);
-    const int P = mmax + 1;
-    if (threadIdx.x == 0) {
-        partial[((size_t)bx * P + mmax) * 2] = t;
-        partial[((size_t)bx * P + mmax) * 2 + 1] = 0.0;
-    }
+    load_h(S, pass, nv, hs);
+    const RowSpan R = row_span(S, bx);
+    double* row = R.sums(partial, mmax);
+    const A nacc = S.cv ? update_rows<A, true>(S, R.r, R.r1, kT, nv, hs) : update_rows<A, false>(S, R.r, R.r1, kT, nv, hs);
+    warp_one(nacc, mmax, row);
     if (pass == 0) {
-        // the second-pass dots V^* w' over this block's rows,
+        // the second-pass dots V^* w' over this warp's rows,
         // while V and w' are still in cache
         const void* w = colp<A>(S, S.j + 1);
-        double* row = partial + (size_t)bx * P * 2;
         for (int c0 = 0; c0 < nv; c0 += jt<A>()) {
-            A re[jt<A>()], im[jt<A>()], dummy = zero<A>();
+            A re[jt<A>()], im[jt<A>()], wn = zero<A>();
 #pragma unroll
             for (int q = 0; q < jt<A>(); ++q) re[q] = im[q] = zero<A>();
-            if (S.cv) dots_rows<A, true>(S, r0, r1, c0, nv, w, re, im, false, dummy);
-            else dots_rows<A, false>(S, r0, r1, c0, nv, w, re, im, false, dummy);
-            dots_epilogue<A>(re, im, S.cv, c0, nv, c0, row);
+            if (S.cv) dots_rows<A, true>(S, R.r, R.r1, kT, c0, nv, w, re, im, false, wn);
+            else dots_rows<A, false>(S, R.r, R.r1, kT, c0, nv, w, re, im, false, wn);
+            warp_dots<A>(re, im, S.cv, c0, nv, c0, row);
         }
     }
 }
 
-template <class A>
-__global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3) eng_update(const SlotDev* __restrict__ sl, const int* __restrict__ rmap, int mmax,
-                                                 int pass, double* __restrict__ partial) {
-    update_block<A>(sl, rmap, mmax, pass, partial, blockIdx.x);
+// The update of slots that are not fused: the rows alone, which need no order,
+// spread over gridDim.y warps per lane set (so that a slot of 30,000 rows still
+// meets every SM); the sums follow in eng_dots (modes 1 and 3), spread over
+// tiles of columns.  Each row's terms are those of update_rows.
+template <class A, bool CV>
+__device__ __forceinline__ void spread_rows(const SlotDev& S, int64_t r, int64_t r1, int64_t step, int nv,
+                                            const CA<A>* hs) {
+    const char* V = (const char*)S.V;
+    const size_t cs = (size_t)S.n * vbytes<A, CV>();
+    void* w = (void*)(V + (size_t)(S.j + 1) * cs);
+    constexpr int NL = CV ? 5 : 10;   // vector loads in flight before their arithmetic
+    for (; r < r1; r += step) {
+        CA<A> o = ldv<A, CV>(w, r);
+        A ar = zero<A>(), ai = zero<A>();
+        auto term = [&](const CA<A>& v, const CA<A>& h) {
+            mac(ar, v.re, h.re);
+            if (CV) {
+                msub(ar, v.im, h.im);
+                mac(ai, v.re, h.im);
+                mac(ai, v.im, h.re);
+            }
+        };
+        for (int t = 0; t < nv; t += NL) {
+            CA<A> v[NL];
+#pragma unroll
+            for (int u = 0; u < NL; ++u)
+                if (t + u < nv) v[u] = ldv<A, CV>(V + (size_t)(t + u) * cs, r);
+#pragma unroll
+            for (int u = 0; u < NL; ++u)
+                if (t + u < nv) term(v[u], hs[t + u]);
+        }
+        o.re = sub(o.re, ar);
+        if (CV) o.im = sub(o.im, ai);
+        stv<A, CV>(w, r, o);
+    }
 }
 
-// Pass 0 of a real Gram-Schmidt slot with nv <= NV vectors, each row's nv
+template <class A>
+__global__ void __launch_bounds__(kRowT, 768 / kRowT) eng_update(const SlotDev* __restrict__ sl, const int* __restrict__ rmap,
+                                                                 int mmax, int pass, double* __restrict__ partial) {
+    const SlotDev& S = sl[rmap[row_block(blockIdx.x)]];
+    if (S.state != kSlotStep || S.fused) return;
+    if (S.orth == 2) {
+        if (pass == 0 && blockIdx.y == 0) three_block<A, true>(S, mmax, partial, blockIdx.x);
+        return;
+    }
+    if (pass == 1 && S.nrm[4] == 0.0) return;
+    __shared__ CA<A> hs[kMaxM];
+    const int nv = S.j + 1;
+    load_h(S, pass, nv, hs);
+    const RowSpan R = row_span(S, blockIdx.x);
+    const int64_t r = R.r + (int64_t)blockIdx.y * kT, step = (int64_t)gridDim.y * kT;
+    if (S.cv) spread_rows<A, true>(S, r, R.r1, step, nv, hs);
+    else spread_rows<A, false>(S, r, R.r1, step, nv, hs);
+}
+
+// A pass of a real Gram-Schmidt slot with nv <= NV vectors, each row's nv
 // vector entries held in registers: w'[r] = w[r] - sum_t V[r, t] h_t, then
-// the second-pass dots acc[t] += V[r, t] w'[r] from the same registers (no
-// second read of V).  Per thread the rows, the terms and the argument order
-// of every multiply-add are those of update_rows followed by dots_rows, and
-// the block sums add in the same order, so the results are
+// (kDots, pass 0) the second-pass dots acc[t] += V[r, t] w'[r] from the same
+// registers (no second read of V).  Per thread the rows, the terms and the
+// argument order of every multiply-add are those of update_rows followed by
+// dots_rows, and the sums add in the same order, so the results are
 // bit-identical to update_block's.
 __device__ __forceinline__ double ld_volatile(const volatile double* p) { return *p; }
 __device__ __forceinline__ float ld_volatile(const volatile float* p) { return *p; }
 __device__ __forceinline__ DF ld_volatile(const volatile DF* p) { return DF{p->h, p->l}; }
 
-template <class A, int NV>
-__device__ __forceinline__ void update_fused_rows(const SlotDev& S, int64_t r0, int64_t r1, int nv, const CA<A>* hs,
-                                                  int mmax, double* partial, int bx) {
+template <class A, int NV, bool kDots>
+__device__ __forceinline__ void update_fused_rows(const SlotDev& S, const RowSpan& R, int nv, const CA<A>* hs,
+                                                  int mmax, double* row) {
     const char* V = (const char*)S.V;
     const size_t cs = (size_t)S.n * vbytes<A, false>();
     void* w = (void*)(V + (size_t)(S.j + 1) * cs);
-    A acc[NV + 1];   // the second-pass dots, then ||w'||^2
+    constexpr int ND = kDots ? NV : 0;
+    A acc[ND + 1];   // the second-pass dots, then ||w'||^2
 #pragma unroll
-    for (int t = 0; t <= NV; ++t) acc[t] = zero<A>();
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-        A v[NV];
-#pragma unroll
-        for (int t = 0; t < NV; ++t)
-            if (t < nv) v[t] = ldv<A, false>(V + (size_t)t * cs, r).re;
+    for (int t = 0; t <= ND; ++t) acc[t] = zero<A>();
+    FusedRow<A, NV> cur, next;
+    if (R.r < R.r1) cur.load(V, cs, nv, w, R.r);
+    for (int64_t r = R.r; r < R.r1; r += kT) {
+        if (r + kT < R.r1) next.load(V, cs, nv, w, r + kT);
         A ar = zero<A>();
         // h from shared memory at each use (held in registers across the row
         // loop it would take NV more of them)
         const volatile A* hv = (const volatile A*)hs;
 #pragma unroll
         for (int t = 0; t < NV; ++t)
-            if (t < nv) mac(ar, v[t], ld_volatile(hv + 2 * t));
-        A o = ldv<A, false>(w, r).re;
-        o = sub(o, ar);
+            if (t < nv) mac(ar, cur.v[t], ld_volatile(hv + 2 * t));
+        const A o = sub(cur.w, ar);
         stv<A, false>(w, r, CA<A>{o, zero<A>()});
-        mac(acc[NV], o, o);
+        mac(acc[ND], o, o);
+        if (kDots) {
 #pragma unroll
-        for (int t = 0; t < NV; ++t)
-            if (t < nv) mac(acc[t], v[t], o);
+            for (int t = 0; t < ND; ++t)
+                if (t < nv) mac(acc[t], cur.v[t], o);
+        }
+        cur = next;
     }
-    fused_epilogue<A, NV>(acc, nv, true, mmax, partial + (size_t)bx * (mmax + 1) * 2);
+    if constexpr (kDots) warp_fused<A, NV>(acc, nv, true, mmax, row);
+    else warp_one(acc[0], mmax, row);
 }
 
-template <class A>
-__global__ void __launch_bounds__(kT, 2) eng_update_fused(const SlotDev* __restrict__ sl, const int* __restrict__ rmap,
-                                                          int mmax, double* __restrict__ partial) {
+template <class A, bool kDots>
+__global__ void __launch_bounds__(kRowT, 384 / kRowT)
+    eng_update_fused(const SlotDev* __restrict__ sl, const int* __restrict__ rmap, int mmax, double* __restrict__ partial) {
     const int bx = blockIdx.x;
-    const SlotDev& S = sl[rmap[bx]];
-    if (S.state != kSlotStep) return;
+    const SlotDev& S = sl[rmap[row_block(bx)]];
+    if (S.state != kSlotStep || !S.fused) return;
+    if (!kDots && S.nrm[4] == 0.0) return;
     const int nv = S.j + 1;
-    if (S.cv || S.orth == 2 || nv < 3 || nv > 20) {
-        update_block<A>(sl, rmap, mmax, 0, partial, bx);
+    if (nv < 3 || nv > 20) {
+        update_block<A>(sl, rmap, mmax, kDots ? 0 : 1, partial, bx);
         return;
     }
     __shared__ CA<A> hs[20];
-    for (int t = threadIdx.x; t < nv; t += blockDim.x) {
-        const double2 v = S.h1[t];
-        hs[t] = CA<A>{from_d<A>(v.x), from_d<A>(v.y)};
-    }
-    __syncthreads();
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
-    if (nv <= 12) update_fused_rows<A, 12>(S, r0, r1, nv, hs, mmax, partial, bx);
-    else update_fused_rows<A, 20>(S, r0, r1, nv, hs, mmax, partial, bx);
+    load_h(S, kDots ? 0 : 1, nv, hs);
+    const RowSpan R = row_span(S, bx);
+    double* row = R.sums(partial, mmax);
+    if (nv <= 12) update_fused_rows<A, 12, kDots>(S, R, nv, hs, mmax, row);
+    else update_fused_rows<A, 20, kDots>(S, R, nv, hs, mmax, row);
 }
 
 // ------------------------------------------------------------ scale
-// w[r] *= f over rows r0..r1, four rows' loads in flight before their stores
+// w[r] *= f over a lane's rows, four rows' loads in flight before their stores
 template <class A, bool CV>
-__device__ __forceinline__ void scale_rows(void* w, int64_t r0, int64_t r1, A f) {
-    const int64_t step = blockDim.x;
+__device__ __forceinline__ void scale_rows(void* w, int64_t r, int64_t r1, int64_t step, A f) {
     auto sc = [&](CA<A> v) {
         v.re = mul(v.re, f);
         if (CV) v.im = mul(v.im, f);
         return v;
     };
-    int64_t r = r0 + threadIdx.x;
     for (; r + 3 * step < r1; r += 4 * step) {
         CA<A> v[4];
 #pragma unroll
@@ -957,15 +1091,14 @@ __device__ __forceinline__ void scale_rows(void* w, int64_t r0, int64_t r1, A f)
 // and marked the slot); mode 1: col ncol on normalising slots
 template <class A>
 __device__ __forceinline__ void scale_block(const SlotDev* sl, const int* __restrict__ rmap, int mode, int bx) {
-    const SlotDev& S = sl[rmap[bx]];
+    const SlotDev& S = sl[rmap[row_block(bx)]];
     if (mode == 0 ? !((S.state == kSlotStep || S.state == kSlotHold) && S.nrm[6] != 0.0) : S.state != kSlotNormalize)
         return;
     const A f = from_d<A>(S.nrm[1]);
     void* w = colp<A>(S, mode == 0 ? S.j : S.ncol);
-    const int64_t lb = bx - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
-    if (S.cv) scale_rows<A, true>(w, r0, r1, f);
-    else scale_rows<A, false>(w, r0, r1, f);
+    const RowSpan R = row_span(S, bx);
+    if (S.cv) scale_rows<A, true>(w, R.r, R.r1, kT, f);
+    else scale_rows<A, false>(w, R.r, R.r1, kT, f);
 }
 
 template <class A>
@@ -1058,8 +1191,10 @@ template <class A>
 __global__ void __launch_bounds__(kT, 2) eng_rotate(const SlotDev* __restrict__ sl, const int* __restrict__ rmap) {
     const SlotDev& S = sl[rmap[blockIdx.x]];
     if (S.state != kSlotRotate || S.rot_tc) return;
-    const int64_t lb = blockIdx.x - S.rb_begin;
-    const int64_t r0 = lb * S.rpb, r1 = min(S.n, r0 + S.rpb);
+    // blockIdx.y: this block's share of the row block (gridDim.y shares)
+    const int64_t b0 = (int64_t)(blockIdx.x - S.rb_begin) * S.rpb, b1 = min(S.n, b0 + S.rpb);
+    const int64_t share = (b1 - b0 + gridDim.y - 1) / gridDim.y;
+    const int64_t r0 = min(b1, b0 + (int64_t)blockIdx.y * share), r1 = min(b1, r0 + share);
     if (S.p <= 8) {
         if (S.cv) rotate_rows_tile<A, true, 8>(S, r0, r1);
         else rotate_rows_tile<A, false, 8>(S, r0, r1);
@@ -1300,29 +1435,44 @@ VKind store_kind(Store st, bool cv) {
 }
 
 // ------------------------------------------------------------ tiles
-// Rows per BLAS block and slices per SpMV block, by the slot's rows alone: a
-// slot's reductions add in the order of its row blocks, so its result is the
-// same alone and in any batch, and repeats from run to run.
-// rpb: the fused dots and update hold two blocks per SM (128 registers a
-// thread), so the row blocks are whole waves of 304 equal blocks, of at most
-// 8,192 rows (the double-float solve of 4.7 M rows: 88 ms with two waves, 94
-// with one) and at least 768 (below that a block's epilogue outweighs its
-// rows: 12 complex slots of 112,000 rows solve in 177 ms at 384 rows a block,
-// 154 at 1,024).  Ground state of 358,584 rows, FP64: 12.1 ms with 304 blocks,
-// 14.1 with 351, 16.0 with 88 (4,096 rows a block).
+// Rows per BLAS block and slices per SpMV block, by the slot alone: a slot's
+// reductions add in the order of its row blocks, so its result is the same
+// alone and in any batch, and repeats from run to run.
+// rpb of Gram-Schmidt slots: 4,096.  The eigenvectors of a solve come from
+// its projected matrix, whose eigensolver gives a column either sign, decided
+// by the matrix's last bits; so the order of these sums is part of a solve's
+// output and stays as it is (RowSpan says how it is spread over the GPU).
+// rpb of three-term slots (evolution: no sign is free): whole waves of 304
+// equal blocks of at most 8,192 and at least 768 rows.
 // spb: one slice per warp spreads a slot of 90,000 rows over 352 blocks (5.9
 // ms a solve; 16 slices 6.3, 64 slices 8.7); from 20,000 slices on there are
 // blocks enough and two slices per warp save the value table's staging
 // (4.7 M rows: 128.8 against 130.4 ms).
-constexpr int kWaveBlocks = 304;
+constexpr int kGramRows = 4096, kWaveBlocks = 304;
 
-Tiles tiles_for(int64_t n, int64_t nslices) {
+Tiles tiles_for(int64_t n, int64_t nslices, int orth) {
     Tiles t;
     const int64_t waves = (n + (int64_t)kWaveBlocks * 8192 - 1) / ((int64_t)kWaveBlocks * 8192);
     const int64_t blocks = kWaveBlocks * std::max<int64_t>(1, waves);
-    t.rpb = (int)std::max<int64_t>(768, ((n + blocks - 1) / blocks + 63) / 64 * 64);
+    t.rpb = orth != 2 ? kGramRows : (int)std::max<int64_t>(768, ((n + blocks - 1) / blocks + 63) / 64 * 64);
     t.spb = nslices < 20000 ? 8 : 16;
     return t;
+}
+
+// QS_FUSED_UPDATE=0 / 1: no / every real Gram-Schmidt slot on the fused kernels
+// (both forms give the same bits; read when a slot is added)
+// Fused: V is read once per pass, by one warp per 512 rows; else its columns
+// are spread over warps in tiles of jt, V read twice.  Ground states, fused /
+// not, in ms: FP64 101,340 rows 9.0 / 6.5, 361,270 rows 13.5 / 12.7, 718,146
+// rows 22.1 / 22.8, 1.34 M rows 78.0 / 74.4, 2.6 M rows 72.5 / 77.5, 4.7 M rows
+// 136.5 / 143.2 (bound by the FP64 pipe, so a second read is cheap until V is
+// far above L2); double-float 101,340 rows 6.1 / 5.8, 361,270 rows 10.2 / 10.3,
+// 718,146 rows 16.3 / 18.4; FP32 7.9 / 8.5 at 718,146 rows.
+bool fused_slot(Store st, int64_t n, bool cv, int orth) {
+    if (cv || orth == 2) return false;
+    const char* e = std::getenv("QS_FUSED_UPDATE");
+    if (e && (e[0] == '0' || e[0] == '1')) return e[0] == '1';
+    return n >= (st == Store::F64 ? 2000000 : 300000);
 }
 
 }  // namespace
@@ -1421,8 +1571,9 @@ int Engine::add(Op& op, int m, bool cv, int tmp_cols, int orth) {
     d.state = kSlotIdle;
     d.carry = -1;
     d.orth = orth;
+    d.fused = fused_slot(st_, n, cv, orth);
     sl.tcols = tc;
-    const Tiles t = tiles_for(n, M.nslices);
+    const Tiles t = tiles_for(n, M.nslices, orth);
     d.rpb = t.rpb;
     d.spb = t.spb;
     sl.live = true;
@@ -1448,7 +1599,7 @@ void Engine::remove(int id) {
 void Engine::build_maps() {
     nrb_ = nsb_ = 0;
     mmax_ = dmax_ = 1;
-    cgs_ = false;
+    cgs_ = fused_ = tiled_ = false;
     for (auto& sl : slots_) {
         SlotDev& d = sl.d;
         if (!sl.live) {
@@ -1465,6 +1616,7 @@ void Engine::build_maps() {
         mmax_ = std::max(mmax_, d.m);
         dmax_ = std::max(dmax_, d.orth == 2 ? 1 : d.m);
         cgs_ = cgs_ || d.orth != 2;
+        (d.fused ? fused_ : tiled_) = true;
     }
     std::vector<int> rm(std::max(1, nrb_)), sm(std::max(1, nsb_));
     for (int i = 0; i < (int)slots_.size(); ++i) {
@@ -1480,7 +1632,7 @@ void Engine::build_maps() {
         cap_smap_ = sm.size() * sizeof(int) * 2;
         smap_.alloc(cap_smap_);
     }
-    const size_t pb = (size_t)std::max(1, nrb_) * (mmax_ + 1) * 2 * sizeof(double);
+    const size_t pb = (size_t)std::max(1, nrb_) * (kT / 32) * (mmax_ + 1) * 2 * sizeof(double);
     if (pb > cap_partial_) {
         cap_partial_ = pb * 2;
         partial_.alloc(cap_partial_);
@@ -1518,39 +1670,43 @@ void Engine::sync_table() {
 // One step of every stepping slot; returns the number of launches.  The dots
 // and reduce grids cover the most vectors a slot dots against (dmax), so
 // three-term slots cost one block row however large their basis; without
-// Gram-Schmidt slots the second-pass launches are left out.
-// QS_FUSED_UPDATE=0 keeps the first-pass dots on eng_dots and pass 0 on
-// eng_update (the fused kernels give the same bits; the switch exists to time
-// the two)
-static bool fused_update_on() {
-    const char* e = std::getenv("QS_FUSED_UPDATE");
-    return !(e && e[0] == '0');
-}
-
+// Gram-Schmidt slots the second-pass launches are left out, as are those of
+// the form (fused or not) that no slot has.
 template <class A>
 static int launch_step_t(const SlotDev* ds, SlotDev* dsw, const int* rm, const int* sm, double* pa, const void* rsq,
-                         int nrb, int nsb, int mmax, int dmax, bool cgs, int ns, cudaStream_t s) {
-    const dim3 gd(nrb, (dmax + jt<A>() - 1) / jt<A>());
-    const bool fused = fused_update_on() && cgs;
+                         int nrb, int nsb, int mmax, int dmax, bool cgs, bool fused, bool tiled, int ns,
+                         cudaStream_t s) {
+    const int nrc = nrb * (kT / kRowT);   // CTAs of the vector kernels
+    const dim3 gd(nrc, (dmax + jt<A>() - 1) / jt<A>());
+    // warps that share a lane set's 16 rows in the update: 24 per SM in all
+    int share = 1;
+    while (share < 16 && 2 * share * nrb * (kT / 32) <= 152 * 24) share *= 2;
+    const dim3 gu(nrc, share);
     eng_spmv<A><<<nsb, kT, 0, s>>>(ds, sm, rsq);
-    if (!cgs) eng_three<A, false><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
-    else if (fused) eng_dots_fused<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 0, pa);
-    else eng_dots<A><<<gd, kT, 0, s>>>(ds, rm, mmax, 0, pa);
-    eng_reduce<<<dim3(ns, dmax + 1), kT, 0, s>>>(dsw, mmax, 0, pa, dmax, false);
-    if (!cgs) eng_three<A, true><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
-    else if (fused) eng_update_fused<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
-    else eng_update<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, 0, pa);
-    eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 1, pa, 0, !cgs);
-    int n = 6;
-    if (cgs) {
+    int n = 1;
+    if (!cgs) {
+        eng_three<A, false><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
+        eng_reduce<<<dim3(ns, dmax + 1), kT, 0, s>>>(dsw, mmax, 0, pa, dmax, false, !cgs);
+        eng_three<A, true><<<nrb, kT, 0, s>>>(ds, rm, mmax, pa);
+        eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 1, pa, 0, true, true);
+        n += 4;
+    } else {
+        if (tiled) eng_dots<A><<<gd, kRowT, 0, s>>>(ds, rm, mmax, 0, pa);
+        if (fused) eng_dots_fused<A><<<nrc, kRowT, 0, s>>>(ds, rm, mmax, pa);
+        eng_reduce<<<dim3(ns, dmax + 1), kT, 0, s>>>(dsw, mmax, 0, pa, dmax, false, !cgs);
+        if (tiled) eng_update<A><<<gu, kRowT, 0, s>>>(ds, rm, mmax, 0, pa);
+        if (tiled) eng_dots<A><<<gd, kRowT, 0, s>>>(ds, rm, mmax, 1, pa);
+        if (fused) eng_update_fused<A, true><<<nrc, kRowT, 0, s>>>(ds, rm, mmax, pa);
+        eng_reduce<<<dim3(ns, mmax + 1), kT, 0, s>>>(dsw, mmax, 1, pa, 0, false, false);
         // the second pass, where a step asks for it
-        eng_reduce<<<dim3(ns, mmax), kT, 0, s>>>(dsw, mmax, 2, pa, 0, false);
-        eng_update<A><<<nrb, kT, 0, s>>>(ds, rm, mmax, 1, pa);
-        eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 3, pa, 0, true);
-        n += 3;
+        if (tiled) eng_update<A><<<gu, kRowT, 0, s>>>(ds, rm, mmax, 1, pa);
+        if (tiled) eng_dots<A><<<nrc, kRowT, 0, s>>>(ds, rm, mmax, 3, pa);
+        if (fused) eng_update_fused<A, false><<<nrc, kRowT, 0, s>>>(ds, rm, mmax, pa);
+        eng_reduce<<<dim3(ns, 1), kT, 0, s>>>(dsw, mmax, 3, pa, 0, true, false);
+        n += 3 + (tiled ? 5 : 0) + (fused ? 3 : 0);
     }
-    eng_scale<A><<<nrb, kT, 0, s>>>(ds, rm, 0);
-    return n;
+    eng_scale<A><<<cgs ? nrc : nrb, cgs ? kRowT : kT, 0, s>>>(ds, rm, 0);
+    return n + 1;
 }
 
 // ------------------------------------------------------------ cluster step
@@ -1603,6 +1759,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
     const int m = Ls.m, orth = Ls.orth, ld = m + 1;
     const int64_t s0 = Ls.nslices * (int64_t)rank / C, s1 = Ls.nslices * (int64_t)(rank + 1) / C;
     const int64_t r0 = min(Ls.n, s0 * kSellSlice), r1 = min(Ls.n, s1 * kSellSlice);
+    const int64_t rt = r0 + threadIdx.x, step_r = blockDim.x;   // this thread's rows
     int j = Ls.j;
     for (int step = 0; step < nsteps && j < m; ++step) {
         if (threadIdx.x == 0) Ls.j = j;
@@ -1617,7 +1774,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
         const void* w = colp<A>(Ls, j + 1);
         A wn = zero<A>();
         if (orth == 2) {
-            const double t = block_sum(three_dot_rows<A, CV>(Ls, r0, r1), shb);
+            const double t = block_sum(three_dot_rows<A, CV>(Ls, rt, r1, step_r), shb);
             if (threadIdx.x == 0) {
                 part1[j * 2] = t;
                 part1[j * 2 + 1] = 0.0;
@@ -1627,7 +1784,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             A re[jt<A>()], im[jt<A>()];
 #pragma unroll
             for (int q = 0; q < jt<A>(); ++q) re[q] = im[q] = zero<A>();
-            dots_rows<A, CV>(Ls, r0, r1, i0, nv, w, re, im, want_wn && i0 == 0, wn);
+            dots_rows<A, CV>(Ls, rt, r1, step_r, i0, nv, w, re, im, want_wn && i0 == 0, wn);
             dots_epilogue<A>(re, im, CV, i0, nv, i0, part1);
         }
         if (want_wn) {
@@ -1664,8 +1821,8 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             hs[t] = CA<A>{from_d<A>(h1[t * 2]), from_d<A>(h1[t * 2 + 1])};
         __syncthreads();
         {
-            const A nacc = orth == 2 ? three_update_rows<A, CV>(Ls, r0, r1, hs[j].re, j > 0 ? hs[j - 1].re : zero<A>())
-                                     : update_rows<A, CV>(Ls, r0, r1, nv, hs);
+            const A nacc = orth == 2 ? three_update_rows<A, CV>(Ls, rt, r1, step_r, hs[j].re, j > 0 ? hs[j - 1].re : zero<A>())
+                                     : update_rows<A, CV>(Ls, rt, r1, step_r, nv, hs);
             const double t = block_sum(nacc, shb);
             if (threadIdx.x == 0) part2[m * 2] = t;
         }
@@ -1674,7 +1831,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
                 A re[jt<A>()], im[jt<A>()], dummy = zero<A>();
 #pragma unroll
                 for (int q = 0; q < jt<A>(); ++q) re[q] = im[q] = zero<A>();
-                dots_rows<A, CV>(Ls, r0, r1, c0, nv, w, re, im, false, dummy);
+                dots_rows<A, CV>(Ls, rt, r1, step_r, c0, nv, w, re, im, false, dummy);
                 dots_epilogue<A>(re, im, CV, c0, nv, c0, part2);
             }
         }
@@ -1713,7 +1870,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
             for (int t = threadIdx.x; t < nv; t += blockDim.x)
                 hs[t] = CA<A>{from_d<A>(h2[t * 2]), from_d<A>(h2[t * 2 + 1])};
             __syncthreads();
-            const A nacc = update_rows<A, CV>(Ls, r0, r1, nv, hs);
+            const A nacc = update_rows<A, CV>(Ls, rt, r1, step_r, nv, hs);
             const double t3 = block_sum(nacc, shb);
             if (threadIdx.x == 0) part1[m * 2] = t3;
             cl_sync();
@@ -1728,7 +1885,7 @@ __device__ __forceinline__ void cluster_steps(SlotDev& Ls, SlotDev* Sg, int nste
         }
         // col(j + 1) /= beta over this CTA's rows
         const A f = from_d<A>(nb > 0 ? 1.0 / nb : 0.0);
-        scale_rows<A, CV>(colp<A>(Ls, j + 1), r0, r1, f);
+        scale_rows<A, CV>(colp<A>(Ls, j + 1), rt, r1, step_r, f);
         cl_sync();
         ++j;
     }
@@ -1866,13 +2023,12 @@ __global__ void __launch_bounds__(kT, std::is_same<A, DF>::value ? 4 : 3)
     for (int step = 0; step < nsteps; ++step) {
         QS_PHASE(nsb, spmv_block<A>(sl, sm, rsq, v));
         QS_PHASE(nrb * ydots, dots_block<A>(sl, rm, mmax, 0, pa, v % nrb, v / nrb));
-        QS_PHASE(ns * (dmax + 1), reduce_block(sl, mmax, 0, pa, dmax, v % ns, v / ns, false));
+        QS_PHASE(ns * (dmax + 1), reduce_block(sl, mmax, 0, pa, dmax, v % ns, v / ns, false, false));
         QS_PHASE(nrb, update_block<A>(sl, rm, mmax, 0, pa, v));
-        QS_PHASE(ns, reduce_block(sl, mmax, 1, pa, 0, v, 0, !cgs));
+        QS_PHASE(cgs ? ns * (mmax + 1) : ns, reduce_block(sl, mmax, 1, pa, 0, v % ns, v / ns, !cgs, false));
         if (cgs) {
-            QS_PHASE(ns * mmax, reduce_block(sl, mmax, 2, pa, 0, v % ns, v / ns, false));
             QS_PHASE(nrb, update_block<A>(sl, rm, mmax, 1, pa, v));
-            QS_PHASE(ns, reduce_block(sl, mmax, 3, pa, 0, v, 0, true));
+            QS_PHASE(ns, reduce_block(sl, mmax, 3, pa, 0, v, 0, true, false));
         }
         QS_PHASE(nrb, scale_block<A>(sl, rm, 0, v));
     }
@@ -1894,7 +2050,7 @@ void Engine::launch_step() {
         using A = decltype(tag);
         step_launches_ = launch_step_t<A>(dslots_.as<SlotDev>(), dslots_.as<SlotDev>(), rmap_.as<int>(),
                                           smap_.as<int>(), partial_.as<double>(), rsq, nrb_, nsb_, mmax_, dmax_,
-                                          cgs_, ns, s_);
+                                          cgs_, fused_, tiled_, ns, s_);
     });
 }
 
@@ -1911,7 +2067,7 @@ void Engine::capture() {
 void Engine::start(int id, int j) {
     SlotDev& d = slots_[id].d;
     if (j < 0 || j >= d.m) throw Error(QS_ERR_ARGUMENT, "start column outside the Krylov basis");
-    d.j = d.j0 = j;
+    d.j = j;
     d.state = kSlotStep;
     dirty_ = true;
 }
@@ -2239,13 +2395,13 @@ std::vector<double> Engine::normalize(const std::vector<int>& ids, int col, bool
     const SlotDev* ds = dslots_.as<SlotDev>();
     const int* rm = rmap_.as<int>();
     double* pa = partial_.as<double>();
-    const int ns = (int)slots_.size();
+    const int ns = (int)slots_.size(), nrc = nrb_ * (kT / kRowT);
     if (nrb_ > 0 && !ids.empty()) {
         with_store(st_, [&](auto tag) {
             using A = decltype(tag);
-            eng_dots<A><<<dim3(nrb_, 1), kT, 0, s_>>>(ds, rm, mmax_, 2, pa);
-            eng_reduce<<<dim3(ns, 1), kT, 0, s_>>>(dslots_.as<SlotDev>(), mmax_, 4, pa, 0, false);
-            if (scale) eng_scale<A><<<nrb_, kT, 0, s_>>>(ds, rm, 1);
+            eng_dots<A><<<nrc, kRowT, 0, s_>>>(ds, rm, mmax_, 2, pa);
+            eng_reduce<<<dim3(ns, 1), kT, 0, s_>>>(dslots_.as<SlotDev>(), mmax_, 4, pa, 0, false, false);
+            if (scale) eng_scale<A><<<nrc, kRowT, 0, s_>>>(ds, rm, 1);
         });
         QS_CUDA(cudaGetLastError());
         launches_ += scale ? 3 : 2;
@@ -2330,27 +2486,28 @@ void Engine::rotate(const std::vector<RotReq>& reqs) {
     dirty_ = true;
     sync_table();
     if (nrb_ > 0) {
+        int dev = 0, nsm = 152;
+        QS_CUDA(cudaGetDevice(&dev));
+        QS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        // row blocks split into shares of at least 256 rows (one tile of 128 on
+        // the tensor cores), up to two blocks per SM
+        const int share = std::max(1, std::min(kGramRows / 256, 2 * nsm / nrb_));
         with_store(st_, [&](auto tag) {
             using A = decltype(tag);
-            eng_rotate<A><<<nrb_, kT, 0, s_>>>(dslots_.as<SlotDev>(), rmap_.as<int>());
+            eng_rotate<A><<<dim3(nrb_, share), kT, 0, s_>>>(dslots_.as<SlotDev>(), rmap_.as<int>());
         });
         QS_CUDA(cudaGetLastError());
         ++launches_;
         if (any_tc) {
             // the shared-memory size, once per device
             static thread_local int attr_dev = -1;
-            int dev = 0;
-            QS_CUDA(cudaGetDevice(&dev));
             if (attr_dev != dev) {
                 QS_CUDA(cudaFuncSetAttribute(eng_rotate_tc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)kTcSmem));
                 attr_dev = dev;
             }
-            // at least two blocks per SM: row blocks split into shares
-            int nsm = 152;
-            QS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-            const int split = std::max(1, std::min(8, (2 * nsm + nrb_ - 1) / std::max(1, nrb_)));
-            eng_rotate_tc<double><<<dim3(nrb_, split), kTcRows, kTcSmem, s_>>>(dslots_.as<SlotDev>(), rmap_.as<int>(),
+            const int tiles = std::max(1, std::min(kGramRows / kTcRows, 2 * nsm / nrb_));
+            eng_rotate_tc<double><<<dim3(nrb_, tiles), kTcRows, kTcSmem, s_>>>(dslots_.as<SlotDev>(), rmap_.as<int>(),
                                                                    tc_err_.as<int>());
             QS_CUDA(cudaGetLastError());
             ++launches_;

@@ -1,10 +1,11 @@
 // qs_engine.h -- the batched Krylov engine: many Krylov processes ("slots"),
 // each on its own assembled operator and its own vectors, advanced together.
 //
-// One Lanczos/Arnoldi step of every stepping slot is a fixed sequence of nine
-// launches (SpMV; dots + reduce; the update with the norm and the next dots +
-// reduce; the second Gram-Schmidt pass where a step asks for it: reduce, update + reduce;
-// scale; six when every slot runs the three-term recurrence), each
+// One Lanczos/Arnoldi step of every stepping slot is a fixed sequence of
+// launches (SpMV; dots + reduce; update, the next dots + reduce; the second
+// Gram-Schmidt pass where a step asks for it: update + reduce; scale: ten, or
+// eight where the dots ride in the update, and six when every slot runs the
+// three-term recurrence), each
 // covering all slots through a block -> slot map.  The step
 // counters live on the device, so the sequence is captured once in a CUDA
 // graph and replayed; the host only meets the device when a slot has filled
@@ -16,8 +17,8 @@
 // arithmetic on the FP32 pipe); both take 8 bytes per real component.  Each
 // slot has its own real/complex vector flag, so a slot's arithmetic does not
 // depend on which other slots share the launches.  The tiles (SpMV
-// slices and BLAS rows per block) follow from a slot's rows alone, so every
-// reduction, and with it every result, repeats from run to run.
+// slices and BLAS rows per block) follow from a slot's rows and recurrence
+// alone, so every reduction, and with it every result, repeats from run to run.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -70,7 +71,7 @@ struct SlotDev {
     // waits for its scaling
     double* nrm;
     int32_t m, j, state;
-    int32_t j0;             // the column this run of steps started from
+    int32_t fused;          // the vector passes run on the fused kernels
     // orthogonalisation of a step: 0 classical Gram-Schmidt twice (CGS2);
     // 1 CGS with the DGKS correction only when ||w'|| < 0.717 ||w|| (ARPACK's
     // dsaitr test); 2 Lanczos three-term recurrence (Hermitian operators,
@@ -92,7 +93,7 @@ enum class Store : int32_t { F64 = 0, DF = 1, F32 = 2 };
 
 // rpb: rows per BLAS block; spb: SELL slices per SpMV block (tiles_for)
 struct Tiles {
-    int rpb = 768, spb = 8;
+    int rpb = 4096, spb = 8;
 };
 
 // One slot's part of a rotate() call.
@@ -193,6 +194,7 @@ class Engine {
     // m for Gram-Schmidt ones) and whether any slot takes a second pass
     int dmax_ = 1;
     bool cgs_ = false;
+    bool fused_ = false, tiled_ = false;   // some slot's vector passes are / are not fused
     int step_launches_ = 9;
     size_t cap_partial_ = 0, cap_rmap_ = 0, cap_smap_ = 0;
     bool dirty_ = true, maps_dirty_ = true;
