@@ -2177,26 +2177,33 @@ void grid_barrier_check(int phantom, double limit_ms, int blocks) {
 
 // Which stepping slots take the cluster step, and with how many CTAs: by the
 // slot and the storage, so that a slot's result is the same alone and in any
-// batch.  Up to 8,192 rows eight CTAs win everywhere (2,703 rows, ground state:
-// 3.4 against 4.5 ms on the graph replay).  Above, sixteen CTAs save the launch
-// gaps of nine kernels a step but have 16 SMs' FP64 rate, where the graph spreads a
-// slot over all of them; so the limit is where the work of a row overtakes the
-// gaps (ground states on GB300, one Gram-Schmidt pass on most steps, cluster / graph
-// in ms):
-//   real matrix:  14,310 rows 3.4/3.8, 19,448 rows 3.6/3.8, 24,310 rows 4.05/3.83,
-//                 28,968 rows 6.5/4.6; evolution 16,384 rows 6.6/7.6, 32,768 9.2/8.5
-//   complex, FP64 (four multiply-adds an entry on the FP64 pipe):
-//                 8,398 rows 6.5/6.2, 9,225 rows 8.1/7.6, 16,796 rows 9.8/6.2
-//   complex, double-float: 9,225 rows 5.3/6.3, 14,000 rows 3.9/4.1, 16,796 rows
-//                 5.8/5.2; FP32: 3.9/4.5, 2.4/2.5, 3.8/3.6
-constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 20480, kClusterRowsComplex = 14336;
+// batch.  Up to 8,192 rows eight CTAs, above sixteen, which save the launch
+// gaps of a step's kernels but have 16 SMs' FP64 rate, where the graph spreads
+// a slot over all of them.
+// Gram-Schmidt slots: up to 32,768 rows.  The two forms add in different
+// orders, and with the order an eigenvector's sign can change (tiles_for), so
+// this line stays although the graph is the faster form on part of it (ground
+// states, cluster / graph in ms): real matrix 4,262 rows 3.8/4.6, 12,870 rows
+// 5.7/6.0, 19,448 rows 6.6/6.3, 28,968 rows 7.5/5.0; complex 9,690 rows 8.0/7.1,
+// 16,796 rows 14.5/8.8, 29,372 rows 22.2/9.2; double-float 12,870 rows 5.0/5.6,
+// 28,968 rows 6.5/4.5, complex 16,796 rows 8.1/7.9.
+// Three-term slots, whose output has no free sign: where the two cross
+// (evolution to four times): real FP64 12,870 rows 2.5/2.7, 16,796 rows 3.3/3.0;
+// double-float 19,448 rows 2.5/2.7, 24,310 rows 2.8/2.75; complex FP64 9,690 rows
+// 3.0/3.1, 14,000 rows 3.6/3.3; double-float 16,796 rows 3.0/3.1, 22,610 rows 3.3/3.1.
+constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 32768;
+constexpr int64_t kClusterThree = 14336, kClusterThreeDf = 20480;
+constexpr int64_t kClusterThreeComplex = 10240, kClusterThreeComplexDf = 18432;
 
 int Engine::cluster_size_for(const SlotDev& d) const {
     const char* e = std::getenv("QS_CLUSTER_STEP");
     if (e && e[0] == '0') return 0;
     if (!(e && e[0] == '1') && persistent_wanted()) return 0;
     if (d.n <= kClusterRows8) return 8;
-    const int64_t limit = !d.cm ? kClusterRows16 : st_ == Store::F64 ? kClusterRows8 : kClusterRowsComplex;
+    const bool f64 = st_ == Store::F64;
+    const int64_t limit = d.orth != 2 ? kClusterRows16
+                          : d.cm      ? (f64 ? kClusterThreeComplex : kClusterThreeComplexDf)
+                                      : (f64 ? kClusterThree : kClusterThreeDf);
     if (d.n <= limit || (e && e[0] == '1')) return cluster16_ok() ? 16 : 8;
     return 0;
 }

@@ -80,3 +80,32 @@ EVEN = dict(kblock=0, pblock=1, zblock=1)
 def test_signs_of_ground_states(qs, L, sym, i, n, seed, precision, sign):
     c = 0.2 + 0.25 * (i + 0.5) / n
     assert sign_of(qs, "j1j2", L, L // 2, sym, "H", c, seed, precision) == sign
+
+
+# ... and when slots of 8,193 to 32,768 rows change between the cluster step and
+# the graph replay
+@pytest.mark.parametrize("model,L,nup,sym,i,n,seed,precision,which,sign", [
+    ("j1j2", 20, 10, dict(kblock=3), 1, 3, 1009, "fp64", "SA", -1),
+    ("j1j2", 20, 10, dict(kblock=3), 2, 3, 2008, "fp64", "SA", 1),
+    ("j1j2", 21, 10, dict(kblock=2), 0, 3, 3, "fp64", "SA", -1),
+    ("j1j2", 21, 10, dict(kblock=2), 2, 3, 2010, "fp64", "SA", 1),
+    ("xxz", 17, 8, {}, 1, 3, 1010, "fp64", "SA", -1), ("xxz", 17, 8, {}, 1, 3, 1014, "fp64", "SA", 1),
+    ("j1j2", 24, 12, EVEN, 0, 2, 7, "fp64df", "SA", -1), ("j1j2", 24, 12, EVEN, 1, 2, 1008, "fp64", "LA", 1)])
+def test_signs_between_the_step_forms(qs, model, L, nup, sym, i, n, seed, precision, which, sign):
+    c = 0.2 + 0.25 * (i + 0.5) / n
+    assert sign_of(qs, model, L, nup, sym, "H", c, seed, precision, which) == sign
+
+
+@pytest.mark.parametrize("L,nup,sym,precision,rows", [
+    (17, 8, {}, "fp64", 24310), (17, 8, {}, "fp64df", 24310), (17, 8, {}, "fp32", 24310),
+    (20, 10, dict(kblock=3), "fp64", 9225), (21, 10, dict(kblock=2), "fp64df", 16796)])
+def test_solves_take_the_cluster_step(qs, monkeypatch, L, nup, sym, precision, rows):
+    """A solve of up to 32,768 rows adds in the cluster step's order."""
+    b = qs.SpinBasis1D(L, nup=nup, pauli=False, **sym)
+    assert b.Ns == rows
+    H = qs.Hamiltonian(b, models.to_terms(qs, models.j1j2(L, 1.0, 0.3)))
+    got = []
+    for form in ("", "1"):
+        monkeypatch.setenv("QS_CLUSTER_STEP", form)
+        got.append(qs.eigsh(H, k=2, tol=1e-11, precision=precision))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
