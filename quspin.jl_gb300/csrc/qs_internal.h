@@ -314,6 +314,8 @@ struct MatvecCall {
     bool df = false;                // FP64 vectors, double-float products (assembled form)
     bool df_io = false;             // double-float vectors in and out, alpha = 1, beta = 0
     bool fx = false;                // FP64 vectors, exact fixed-point row sums where the operator allows
+    bool solver = false;            // matrix-free operators: each term rounded on its own, which the
+                                    // eigensolvers' signs rest on
     bool fx_ready = false;          // the scaled integer copy of x is already made (later row ranges)
     int64_t slice0 = 0, slice1 = -1; // sliced-ELL slices [slice0, slice1) only (-1: to the end)
 };

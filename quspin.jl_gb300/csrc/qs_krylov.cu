@@ -39,6 +39,7 @@ struct Ctx {
     Blas blas;
     int64_t matvecs = 0;
     bool df = false;   // double-float products of an assembled operator
+    bool solver = false;   // MatvecCall::solver
     Ctx(Op& o, VKind k, bool df_ = false)
         : op(o), n(o.basis->n), vk(k), s(o.stream), blas(k, o.basis->n, o.stream), df(df_) {}
     void* col(DevBuf& V, int j) const { return (char*)V.p + (size_t)j * n * vk_bytes(vk); }
@@ -50,6 +51,7 @@ struct Ctx {
         c.single = vk_single(vk);
         c.df_io = vk_df(vk);
         c.df = (df || c.df_io) && !c.single;
+        c.solver = solver;
         op_matvec_device(op, c, s);
         ++matvecs;
     }
@@ -339,6 +341,7 @@ void eigs_general(Op& op, const qs_eigsh_opts& o, double* values, void* vectors,
     const bool dev = o.mem == QS_MEM_DEVICE;
     const size_t esz = op.complex_mat ? 16 : 8;   // dtype of v0
     Ctx c(op, VKind::C128);
+    c.solver = true;
     std::vector<cd> theta;
     DevBuf X((size_t)n * k * 16);
     int64_t mv = 0;
@@ -446,6 +449,7 @@ void eigsh(Op& op, const qs_eigsh_opts& o, double* values, void* vectors, qs_eig
         DevBuf e(n * esz), col(n * esz);
         std::vector<double> h(n * (cpx ? 2 : 1));
         Ctx c(op, k64);
+        c.solver = true;
         for (int j = 0; j < N; ++j) {
             std::fill(h.begin(), h.end(), 0.0);
             h[cpx ? 2 * j : j] = 1.0;
@@ -545,6 +549,7 @@ void eigsh(Op& op, const qs_eigsh_opts& o, double* values, void* vectors, qs_eig
     // reduced-precision vectors get an FP64 Rayleigh-quotient polish
     const bool single = vk != k64;
     Ctx c(op, vk, o.precision == 2);
+    c.solver = true;
     DevBuf v0((size_t)n * vk_bytes(vk));
     const bool dev = o.mem == QS_MEM_DEVICE;
     if (o.v0) {
@@ -574,6 +579,7 @@ void eigsh(Op& op, const qs_eigsh_opts& o, double* values, void* vectors, qs_eig
             convert_vec((char*)X.p + (size_t)q * n * vk_bytes(vk), vk, (char*)X64.p + (size_t)q * n * esz, k64, n,
                         op.stream);
         Ctx c64(op, k64);
+        c64.solver = true;
         DevBuf Ax(n * esz);
         bool need_refine = false;
         double maxrel = 0.0;

@@ -19,7 +19,10 @@
 // walked by qs_rows.cuh, shared with the assembly.  Bound: integer issue in the
 // orbit search; FP64 is one multiply-add per transition (amplitude times
 // character from a table, the rare sqrt(stab) != 1 and the row's 1/sqrt(stab)
-// apart), which GB300's FP64 pipe takes 16 cycles a warp for.
+// apart), which GB300's FP64 pipe takes 16 cycles a warp for.  The eigensolvers,
+// which run on this product below 4,096 rows, have every term rounded on its own
+// (MatvecCall::solver): the last bits of their projected matrix decide an
+// eigenvector's sign.
 //
 // Rank lookups: full 2^L space -> the state itself; fixed-weight sector
 // without spatial symmetry -> combinadic rank (src/discrete_basis.jl:1879-1906);
@@ -71,6 +74,8 @@ struct MvArgs {
     int table;               // amplitude x character staged per (class, element)
     int any_chars;
     const double* sq;        // sqrt(i), then 1/sqrt(i), i = 0 .. kMaxGroup
+    int solver;              // MatvecCall::solver (the general kernels alone)
+    int full_diag;           // real operator, complex vectors: the complex diagonal as it stands
     const void* diag;        // complex, precision of the call
     const void* diag_re;     // its real part (real operators)
     int conj_amp, conj_chi;
@@ -193,6 +198,8 @@ __device__ __forceinline__ void load_x(const MvArgs& a, int64_t i, T& xr, T& xi)
 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
@@ -204,7 +211,7 @@ __device__ __forceinline__ void times_chi(const MvArgs& a, int ec, T& wr, T& wi)
     if (kCM) {
         T ci = (T)__ldg(a.chi_im + (size_t)ec * a.chi_stride);
         if (a.conj_chi) ci = -ci;
-        const T nr = fma_r(-wi, ci, mul_rn(wr, cr)), ni = fma_r(wi, cr, mul_rn(wr, ci));
+        const T nr = wr * cr - wi * ci, ni = wr * ci + wi * cr;
         wr = nr;
         wi = ni;
     } else {
@@ -248,11 +255,23 @@ __device__ __noinline__ bool run_chars(const MvArgs& a, int k, U s, U& t, double
     return true;
 }
 
+// 1/sqrt(st) in the arithmetic of the call
+template <typename T> __device__ __forceinline__ T inv_root(const MvArgs& a, int st);
+template <> __device__ __forceinline__ double inv_root<double>(const MvArgs& a, int st) {
+    return __ldg(a.sq + kMaxGroup + 1 + st);
+}
+template <> __device__ __forceinline__ float inv_root<float>(const MvArgs& a, int st) {
+    return 1.f / (float)__ldg(a.sq + st);
+}
+
 // acc += w x with the character, sqrt(stab) of the column and the sign of a
-// transition of class cls (a program run by its characters brings its own w)
-template <bool kCM, bool kCV, typename T, bool kPlain>
-__device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab, uint32_t cls, int ec, int st, int sign,
-                                               T wr, T wi, int64_t idx, T& acc_r, T& acc_i) {
+// transition of class cls (a program run by its characters brings its own w).
+// Solver calls: sqrt(stab) of the column times 1/sqrt(stab) of the row (st_r) as
+// one factor of w, and w x of a complex operator rounded before it is added
+// (six FP64 instructions against four).
+template <bool kSym, bool kCM, bool kCV, typename T, bool kPlain>
+__device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab, uint32_t cls, int ec, int st, int st_r,
+                                               int sign, T wr, T wi, int64_t idx, T& acc_r, T& acc_i) {
     if (!kPlain && cls == kCharsClass) {
         times_chi<kCM, T>(a, ec, wr, wi);
     } else if (kPlain || a.table) {
@@ -272,13 +291,19 @@ __device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab,
         wr = -wr;
         wi = -wi;
     }
-    if (st != 1) {
-        const T f = (T)__ldg(a.sq + st);
+    if (st != 1 || (!kPlain && st_r != 1)) {
+        T f = (T)__ldg(a.sq + st);
+        if (!kPlain && st_r != 1) f = mul_rn(f, inv_root<T>(a, st_r));
         wr = mul_rn(wr, f);
         if (kCM) wi = mul_rn(wi, f);
     }
     T xr, xi;
     load_x<T, kCV>(a, idx, xr, xi);
+    if (kCM && !kPlain && a.solver) {
+        acc_r = add_rn(acc_r, fma_r(wr, xr, -mul_rn(wi, xi)));
+        acc_i = add_rn(acc_i, kSym ? fma_r(wr, xi, mul_rn(wi, xr)) : fma_r(wi, xr, mul_rn(wr, xi)));
+        return;
+    }
     acc_r = fma_r(wr, xr, acc_r);
     if (kCM) {
         acc_r = fma_r(-wi, xi, acc_r);
@@ -289,10 +314,11 @@ __device__ __forceinline__ void add_transition(const MvArgs& a, const void* tab,
     }
 }
 
-// y[r] = beta y[r] + alpha (d[r] x[r] + acc / sqrt(stab_r))
-template <bool kSym, bool kCM, bool kCV, typename T>
+// y[r] = beta y[r] + alpha (d[r] x[r] + acc / sqrt(stab_r)); solver calls have
+// the root in their terms
+template <bool kSym, bool kCM, bool kCV, typename T, bool kPlain>
 __device__ __forceinline__ void store_row(const MvArgs& a, int64_t r, T acc_r, T acc_i) {
-    if (kSym) {
+    if (kSym && (kPlain || !a.solver)) {
         const int st = a.stab[r];
         if (st != 1) {
             const T f = (T)__ldg(a.sq + kMaxGroup + 1 + st);
@@ -303,7 +329,7 @@ __device__ __forceinline__ void store_row(const MvArgs& a, int64_t r, T acc_r, T
     // diagonal (user + extracted), conjugated with the operator
     T xr, xi;
     load_x<T, kCV>(a, r, xr, xi);
-    if (kCM) {
+    if (kCM || (kCV && a.full_diag)) {
         const typename V2<T>::t d = ((const typename V2<T>::t*)a.diag)[r];
         const T dr = d.x, di = a.conj_amp ? -d.y : d.y;
         acc_r += dr * xr - di * xi;
@@ -369,6 +395,7 @@ __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
         const bool valid = r < a.n;
         U s = 0;
         if (valid) s = (k32 && kMode == 1) ? (U)unrank32(r, binom32, a.L, a.nup) : row_state<U>(a, kSym ? 2 : kMode, r);
+        const int st_r = kSym && !kPlain && a.solver && valid ? a.stab[r] : 1;
         T acc_r = 0, acc_i = 0;
         for (int c0 = 0; c0 < R.nprog; c0 += kRowChunk) {
             if (R.nprog > kRowChunk) {
@@ -393,10 +420,11 @@ __global__ void __launch_bounds__(kMvThreads) matvec_kernel(MvArgs a) {
                 if (kSym) row_orbit<U>(R, g, t, m, ec, st);
                 const int64_t idx = row_column<U, kMode>(R, spl, rtab, m);
                 if (kSym && idx < 0) return;
-                add_transition<kCM, kCV, T, kPlain>(a, dyn, cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
+                add_transition<kSym, kCM, kCV, T, kPlain>(a, dyn, cls, ec, st, st_r, sign, wr, wi, idx,
+                                                       acc_r, acc_i);
             });
         }
-        if (valid) store_row<kSym, kCM, kCV, T>(a, r, acc_r, acc_i);
+        if (valid) store_row<kSym, kCM, kCV, T, kPlain>(a, r, acc_r, acc_i);
     }
 }
 
@@ -472,6 +500,7 @@ __global__ void __launch_bounds__(kMvThreads) matvec_warp_rank_kernel(MvArgs a) 
         const int64_t r = base + lane;
         const bool rv = r < a.n;
         const U s = rv ? ((const U*)a.reps)[r] : (U)0;
+        const int st_r = a.solver && rv ? a.stab[r] : 1;
         T acc_r = 0, acc_i = 0;
         for (int k = 0; k < R.nprog; ++k) {
             const RowProg p = R.progs[k];
@@ -492,9 +521,9 @@ __global__ void __launch_bounds__(kMvThreads) matvec_warp_rank_kernel(MvArgs a) 
             const int64_t idx = rank_warp<U>((const U*)R.reps, a.n, spl, (int)R.nsplit, R.stride, m, alive);
             if (!alive || idx < 0) continue;
             const int sign = __popcll((unsigned long long)(s & (U)p.zy)) & 1;
-            add_transition<kCM, kCV, T, false>(a, dyn, p.cls, ec, st, sign, wr, wi, idx, acc_r, acc_i);
+            add_transition<true, kCM, kCV, T, false>(a, dyn, p.cls, ec, st, st_r, sign, wr, wi, idx, acc_r, acc_i);
         }
-        if (rv) store_row<true, kCM, kCV, T>(a, r, acc_r, acc_i);
+        if (rv) store_row<true, kCM, kCV, T, false>(a, r, acc_r, acc_i);
     }
 }
 
@@ -751,7 +780,7 @@ void launch_mode(const MvArgs& a, bool cm, bool cv, cudaStream_t s) {
         else launch_rows(matvec_kernel<U, kMode, false, false, T, P_>, grid, threads, dyn, s, a);          \
     } while (0)
     if constexpr (sizeof(U) == 4 && (kMode == 1 || kMode == 3)) {
-        if (a.table && !a.any_chars && !a.row.any_zy && !a.row.check_weight) {
+        if (a.table && !a.any_chars && !a.row.any_zy && !a.row.check_weight && !a.solver) {
             QS_ROWS(true);
             return;
         }
@@ -970,6 +999,7 @@ void op_matvec_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     a.br = c.beta.re;
     a.bi = c.beta.im;
     a.beta_zero = (c.beta.re == 0.0 && c.beta.im == 0.0);
+    a.solver = a.full_diag = c.solver;
     a.x = c.x;
     a.y = c.y;
     // the pull form of op(A) runs the chain of op(A)^T; a transposed call runs

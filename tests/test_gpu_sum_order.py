@@ -109,3 +109,15 @@ def test_solves_take_the_cluster_step(qs, monkeypatch, L, nup, sym, precision, r
         monkeypatch.setenv("QS_CLUSTER_STEP", form)
         got.append(qs.eigsh(H, k=2, tol=1e-11, precision=precision))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+# ... and when the terms of the matrix-free product (operators of fewer than
+# 4,096 rows) are rounded in another order
+@pytest.mark.parametrize("L,sym,i,seed,sign", [
+    (14, EVEN, 0, 4, 1), (14, EVEN, 1, 1014, 1), (14, EVEN, 2, 2013, 1), (14, EVEN, 3, 3008, -1),
+    (18, EVEN, 0, 3, 1), (18, EVEN, 1, 1001, -1), (18, EVEN, 3, 3009, 1),
+    (20, EVEN, 2, 2003, 1), (20, EVEN, 3, 3008, -1),
+    (14, dict(kblock=2), 0, 18, -1), (14, dict(kblock=2), 1, 1003, -1), (14, dict(kblock=2), 2, 2015, 1),
+    (14, dict(kblock=2), 3, 3007, -1), (14, dict(kblock=2), 3, 3017, -1)])
+def test_signs_of_matrix_free_solves(qs, L, sym, i, seed, sign):
+    assert sign_of(qs, "j1j2", L, L // 2, sym, "Q", 0.2 + 0.25 * (i + 0.5) / 4, seed) == sign
