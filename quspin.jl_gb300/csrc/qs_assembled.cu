@@ -182,8 +182,7 @@ void launch_build(const Basis& b, const BuildArgs& a, int grid, cudaStream_t s) 
     const bool wide = b.symmetric ? b.wide : (b.wide || mode == 0);
     const size_t dyn = !wide && (mode == 1 || mode == 3) ? (size_t)a.row.rank.size * sizeof(uint32_t) : 0;
     auto go = [&](auto kernel) {
-        if (dyn > 16 * 1024)
-            QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+        allow_row_smem(kernel, dyn);
         kernel<<<grid, kThreads, dyn, s>>>(a);
         QS_CUDA(cudaGetLastError());
     };

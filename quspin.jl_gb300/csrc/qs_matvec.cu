@@ -49,7 +49,6 @@ namespace {
 
 constexpr int kMvThreads = kRowThreads;
 constexpr int kMaxSplit = 2048;
-constexpr int kMvTable = 1024;   // (class, element) values staged in shared memory, at most
 
 template <typename T> struct V2;
 template <> struct V2<double> { using t = double2; };
@@ -744,17 +743,15 @@ void row_args(const Op& op, bool bwd, MvArgs& a) {
     if (ones) a.nelem = 1;
     a.amp = op.d_amp.as<double2>();
     a.nclass = op.nclass;
-    a.table = (int64_t)op.nclass * a.nelem <= kMvTable;
+    a.table = (int64_t)op.nclass * a.nelem <= kRowValues;
     a.any_chars = op.any_chars;
     a.sq = b.d_sqrt.as<double>();
 }
 
-// Launches a row kernel with `dyn` bytes of dynamic shared memory; the rank
-// tables of the longest chains pass the default 48 KB.
+// Launches a row kernel with `dyn` bytes of dynamic shared memory.
 template <class K>
 void launch_rows(K kernel, int grid, int threads, size_t dyn, cudaStream_t s, const MvArgs& a) {
-    if (dyn > 16 * 1024)
-        QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    allow_row_smem(kernel, dyn);
     kernel<<<grid, threads, dyn, s>>>(a);
 }
 

@@ -25,6 +25,21 @@ namespace qs {
 constexpr int kRowThreads = 256;   // threads of a row kernel, at most
 constexpr int kRowChunk = 128;     // programs held in shared memory at once
 
+constexpr int kRowValues = 1024;   // (class, element) values staged in shared memory, at most
+
+// Dynamic shared memory of a row kernel past the 16 KB that fit beside its
+// static arrays: the limit belongs to the kernel, not to a call, and a launch
+// above it fails, so every call allows the same, the most a sector can need
+// (complex FP64 values, and the rank tables of 16 particles on 32 sites: 36 rows
+// of 256 entries); calls from several threads meet the same limit.
+constexpr size_t kRowDyn = (size_t)kRowValues * 16 + 36 * 256 * sizeof(uint32_t);
+template <class K>
+void allow_row_smem(K kernel, size_t dyn) {
+    if (dyn > kRowDyn) throw Error(QS_ERR_UNSUPPORTED, "row kernel tables exceed their shared memory");
+    if (dyn > 16 * 1024)
+        QS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowDyn));
+}
+
 // What the row kernels need to know about the basis and the programs.
 struct RowArgs {
     const void* reps;
