@@ -864,7 +864,13 @@ namespace {
 void prepare_row_programs(Op& op, std::vector<RowProg>& rows, std::vector<double>& amp) {
     const Basis& b = *op.basis;
     rows.assign(op.progs.size(), RowProg{});
-    std::map<std::pair<double, double>, uint32_t> seen;
+    // by the values' bits: a coupling that is not a number is a class of its own
+    std::map<std::pair<uint64_t, uint64_t>, uint32_t> seen;
+    auto bits = [](double v) {
+        uint64_t u;
+        std::memcpy(&u, &v, sizeof(u));
+        return u;
+    };
     op.any_zy = op.check_weight = op.any_chars = false;
     for (size_t k = 0; k < op.progs.size(); ++k) {
         const TermProg& p = op.progs[k];
@@ -883,12 +889,13 @@ void prepare_row_programs(Op& op, std::vector<RowProg>& rows, std::vector<double
         r.zy = p.zmask ^ p.ymask;
         // popc(~s & z) = popc(z) - popc(s & z): the constant part joins the amplitude
         const double sg = (__builtin_popcountll(p.zmask) & 1) ? -1.0 : 1.0;
-        const std::pair<double, double> v{sg * p.amp0_re, sg * p.amp0_im};
+        const double re = sg * p.amp0_re, im = sg * p.amp0_im;
+        const std::pair<uint64_t, uint64_t> v{bits(re), bits(im)};
         auto it = seen.find(v);
         if (it == seen.end()) {
             it = seen.emplace(v, (uint32_t)(amp.size() / 2)).first;
-            amp.push_back(v.first);
-            amp.push_back(v.second);
+            amp.push_back(re);
+            amp.push_back(im);
         }
         r.cls = it->second;
         if (r.zy) op.any_zy = true;
