@@ -259,6 +259,7 @@ struct Op {
     std::vector<uint32_t> prog_class;
     int nclass = 0;
     bool any_zy = false, check_weight = false, any_chars = false;
+    bool diag_im = false;           // the user diagonal has imaginary parts
     DevBuf d_diags;                 // holds the five forms of the diagonal
     DevBuf d_diag;                  // complex diagonal (user + extracted), 2*n doubles
     DevBuf d_diag32;                // single-precision copy

@@ -960,6 +960,8 @@ void op_prepare_device(Op& op) {
         user.alloc(2 * b.n * sizeof(double), op.stream);
         QS_CUDA(cudaMemcpyAsync(user.p, op.user_diag.data(), user.bytes, cudaMemcpyHostToDevice, op.stream));
     }
+    op.diag_im = false;
+    for (const std::complex<double>& v : op.user_diag) op.diag_im = op.diag_im || v.imag() != 0.0;
     BufPack diags;
     diags.add(op.d_diag, 2 * b.n * sizeof(double));
     diags.add(op.d_diag32, 2 * b.n * sizeof(float));
@@ -1003,7 +1005,8 @@ void op_matvec_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     a.br = c.beta.re;
     a.bi = c.beta.im;
     a.beta_zero = (c.beta.re == 0.0 && c.beta.im == 0.0);
-    a.solver = a.full_diag = c.solver;
+    a.solver = c.solver;
+    a.full_diag = c.solver || op.diag_im;
     a.x = c.x;
     a.y = c.y;
     // the pull form of op(A) runs the chain of op(A)^T; a transposed call runs
