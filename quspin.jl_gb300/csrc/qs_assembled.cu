@@ -1981,7 +1981,8 @@ TransientAssembly::~TransientAssembly() {
     }
 }
 
-bool op_matvec_host_overlap(Op& op, const MatvecCall& c0, void* y_host, size_t eb) {
+bool op_matvec_host_overlap(Op& op, const MatvecCall& c0, void* y_host, size_t eb, const void* x_host,
+                            size_t x_bytes) {
     const Assembled& M = op.asm_;
     const bool T = (c0.flags & QS_TRANSPOSE) != 0;
     const bool fx = c0.fx && !c0.single && M.fx_classes > 0;
@@ -2003,7 +2004,7 @@ bool op_matvec_host_overlap(Op& op, const MatvecCall& c0, void* y_host, size_t e
         op_spmv_device(op, c, op.stream);
         QS_CUDA(cudaEventRecord(op.range_done[k], op.stream));
     }
-    touch_host(y_host, (size_t)n * eb);   // while the ranges compute
+    touch_host(y_host, (size_t)n * eb, x_host, x_bytes);   // while the ranges compute
     for (int k = 0; k < K; ++k) {
         QS_CUDA(cudaStreamWaitEvent(op.copy_stream, op.range_done[k], 0));
         const int64_t r0 = M.nslices * k / K * kSellSlice;

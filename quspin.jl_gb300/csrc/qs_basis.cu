@@ -1863,11 +1863,17 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
     PoolBuf din, dout;
     const double2* pin = reinterpret_cast<const double2*>(in);
     double2* pout = reinterpret_cast<double2*>(out);
+    const void* kept = in;   // host memory that the call reads
+    size_t kept_bytes = (size_t)nin * sizeof(double2);
     if (!device) {
         din.alloc((size_t)nin * sizeof(double2), s);
         dout.alloc((size_t)nout * sizeof(double2), s);
         QS_CUDA(cudaMemcpyAsync(din.p, in, din.bytes, cudaMemcpyHostToDevice, s));
-        if (mode == 0 && accumulate) QS_CUDA(cudaMemcpyAsync(dout.p, out, dout.bytes, cudaMemcpyHostToDevice, s));
+        if (mode == 0 && accumulate) {
+            QS_CUDA(cudaMemcpyAsync(dout.p, out, dout.bytes, cudaMemcpyHostToDevice, s));
+            kept = out;
+            kept_bytes = dout.bytes;
+        }
         pin = din.as<double2>();
         pout = dout.as<double2>();
     }
@@ -1889,7 +1895,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
         else embed_kernel<uint32_t><<<grid, 256, 0, s>>>(e);
         QS_CUDA(cudaGetLastError());
         note_launches(1);
-        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
+        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s, kept, kept_bytes);
         QS_CUDA(cudaStreamSynchronize(s));
         return;
     }
@@ -1923,7 +1929,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
         }
         QS_CUDA(cudaGetLastError());
         note_launches(1);
-        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
+        if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s, kept, kept_bytes);
         QS_CUDA(cudaStreamSynchronize(s));
         return;
     }
@@ -1952,7 +1958,7 @@ void basis_project(Basis& b, bool pcon, int mode, const double* in, double* out,
     else project_kernel<uint32_t><<<grid, 128, 0, s>>>(a);
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s);
+    if (!device) copy_to_host(out, pout, (size_t)nout * sizeof(double2), s, kept, kept_bytes);
     QS_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -365,9 +365,9 @@ int qs_op_matvec(qs_op* op, int32_t flags, const double* alpha, const void* x, i
             c.y = o.d_y.p;
             // the assembled product in row ranges, each range read back while the
             // next computes; otherwise one product and one read-back
-            if (!qs::op_matvec_host_overlap(o, c, ys, yb)) {
+            if (!qs::op_matvec_host_overlap(o, c, ys, yb, xs, n * xb)) {
                 qs::op_matvec_device(o, c, o.stream);
-                if (beta_zero) qs::touch_host(ys, n * yb);   // (with beta the caller's y is already there)
+                if (beta_zero) qs::touch_host(ys, n * yb, xs, n * xb);   // (with beta the caller's y is already there)
                 QS_CUDA(cudaMemcpyAsync(ys, o.d_y.p, n * yb, cudaMemcpyDeviceToHost, o.stream));
             }
             QS_CUDA(cudaStreamSynchronize(o.stream));

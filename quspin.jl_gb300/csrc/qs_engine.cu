@@ -3241,7 +3241,7 @@ void evolve_stepwise(Op& op, const double* v0, const std::vector<double>& offset
             }
             prev = offsets[i];
         }
-        copy_to_host(out + (size_t)i * 2 * n, cur.p, bytes, st);
+        copy_to_host(out + (size_t)i * 2 * n, cur.p, bytes, st, v0, bytes);
     }
     QS_CUDA(cudaStreamSynchronize(st));
     note_launches(E.launches());

@@ -95,10 +95,15 @@ void* mapped_host_address(void* p);
 // overwritten whole, so that the pages exist before a device copy lands in them.  A copy into heap pages that
 // no one has touched faults them in one by one from the device: 17 ms for 21 MB
 // on a GB300's Grace host, against 1 ms for the touches and 0.17 ms for the
-// copy (malloc hands out such pages after it has trimmed its heap).
-void touch_host(void* p, size_t bytes);
+// copy (malloc hands out such pages after it has trimmed its heap).  Ordinary
+// memory only: the pages of page-locked memory are there, and device memory is
+// for the copy to refuse.  in: host memory that a copy under way may still be
+// reading (the call's input, or the output that it adds to); an output that
+// overlaps it is left alone.
+void touch_host(void* p, size_t bytes, const void* in = nullptr, size_t in_bytes = 0);
 // touch_host(dst), then the copy of device memory into it on s.
-void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s, const void* in = nullptr,
+                  size_t in_bytes = 0);
 
 // Several buffers in one allocation: add() each with its host contents (null:
 // left unset), then place() them.  A cudaMalloc and cudaFree pair takes 13 us
@@ -356,8 +361,10 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s);
 bool op_spmm_device(Op& op, const MatvecCall& c, int64_t nrhs, cudaStream_t s);
 // y = op x for one host vector with the assembled sliced-ELL product split in
 // row ranges, each range's rows of y copied back while later ranges compute;
-// false (nothing done) when the operator or the call does not allow it
-bool op_matvec_host_overlap(Op& op, const MatvecCall& c, void* y_host, size_t elem_bytes);
+// false (nothing done) when the operator or the call does not allow it; x_host:
+// the call's input
+bool op_matvec_host_overlap(Op& op, const MatvecCall& c, void* y_host, size_t elem_bytes, const void* x_host,
+                            size_t x_bytes);
 // the assembled matrix on the host: CSR off-diagonal part (rowptr n + 1,
 // cols and complex values nnz; a row may repeat a column) and the diagonal
 void op_export_csr(Op& op, int64_t* rowptr, int64_t* cols, double* values, double* diag);

@@ -759,7 +759,7 @@ void expm_multiply(Op& op, cd a, const double* v, double* out, double tol, int k
     convert_vec(d64.p, VKind::C128, dv.p, vk, n, op.stream);
     expmv_vector(c, dv.p, a, tol, krylov_dim, 0, dout.p);
     convert_vec(dout.p, vk, d64.p, VKind::C128, n, op.stream);
-    copy_to_host(out, d64.p, n * 16, op.stream);
+    copy_to_host(out, d64.p, n * 16, op.stream, v, n * 16);
     QS_CUDA(cudaStreamSynchronize(op.stream));
 }
 
@@ -799,7 +799,7 @@ void evolve(Op& op, const double* v0, double t0, const double* times, int nt, in
             src = st.p;
         }
         convert_vec(src, vk, d64.p, VKind::C128, n, op.stream);
-        copy_to_host(out + (size_t)col * 2 * n, d64.p, n * 16, op.stream);
+        copy_to_host(out + (size_t)col * 2 * n, d64.p, n * 16, op.stream, v0, n * 16);
         QS_CUDA(cudaStreamSynchronize(op.stream));
     };
     if (nt == 0) return;

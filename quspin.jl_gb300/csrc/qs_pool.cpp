@@ -130,7 +130,13 @@ void* mapped_host_address(void* p) {
     return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-void touch_host(void* p, size_t bytes) {
+void touch_host(void* p, size_t bytes, const void* in, size_t in_bytes) {
+    if (!p || !bytes) return;
+    const char *a = static_cast<const char*>(p), *b = static_cast<const char*>(in);
+    if (b && a < b + in_bytes && b < a + bytes) return;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) cudaGetLastError();
+    else if (at.type != cudaMemoryTypeUnregistered) return;
     static const size_t page = [] {
         const long v = sysconf(_SC_PAGESIZE);
         return v > 0 ? (size_t)v : (size_t)4096;
@@ -142,8 +148,8 @@ void touch_host(void* p, size_t bytes) {
     for (size_t o = 0; o < bytes; o += page - ((uintptr_t)(q + o) & (page - 1))) q[o] = 0;
 }
 
-void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
-    touch_host(dst, bytes);
+void copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t s, const void* in, size_t in_bytes) {
+    touch_host(dst, bytes, in, in_bytes);
     QS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
 }
 

@@ -621,7 +621,9 @@ void basis_project_dense(Basis& b, bool pcon, int mode, const double* in, double
     }
     QS_CUDA(cudaGetLastError());
     note_launches(1);
-    if (!device) copy_to_host(out, pout, (size_t)nout * ncols * 16, s);
+    if (!device)
+        copy_to_host(out, pout, (size_t)nout * ncols * 16, s, accumulate ? out : in,
+                     (size_t)(accumulate ? nout : nin) * ncols * 16);
     QS_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -280,7 +280,7 @@ void lanczos_combine(LanczosSet& L, int s, const double* coeff, int ncoef, doubl
         o = tmp.as<double2>();
     }
     combine(column(L, s, 0), L.cv, L.n, used, Y.as<double2>(), ncoef, o, st);
-    if (!device) copy_to_host(out, tmp.p, tmp.bytes, st);
+    if (!device) copy_to_host(out, tmp.p, tmp.bytes, st, coeff, Y.bytes);
     QS_CUDA(cudaStreamSynchronize(st));
 }
 
