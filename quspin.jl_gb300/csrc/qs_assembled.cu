@@ -1450,10 +1450,10 @@ void op_assemble(Op& op) {
         for (int i = 1; i <= kMaxGroup; ++i) df_split_host(1.0 / std::sqrt((double)i), rq[2 * i], rq[2 * i + 1]);
         tables.add(M.rsq_df, rq.size() * sizeof(float), rq.data());
     }
-    tables.place(M.tables);
+    cudaStream_t s = op.stream;
+    tables.place(M.tables, s);
     M.xsplit.alloc((size_t)b.n * 4 * sizeof(float));
 
-    cudaStream_t s = op.stream;
     // value code of a program's class reaching element e, without the
     // stabiliser class: ((a nC + c) nD) 2 + sign
     BuildArgs a{};

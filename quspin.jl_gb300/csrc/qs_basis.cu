@@ -764,7 +764,7 @@ void finish_sector(Basis& b, BufPack& pack) {
             chi_one[e] = (std::fabs(b.group.chi_re[e] - 1.0) < 1e-9 && std::fabs(b.group.chi_im[e]) < 1e-9) ? 1 : 0;
         pack.add(d_chi_one, kMaxGroup, chi_one.data());
     }
-    pack.place(b.d_tables);
+    pack.place(b.d_tables, b.stream);
     if (!b.symmetric) b.n = b.n_parent;
     else if (b.wide) enumerate_sector<uint64_t>(b, d_chi_one);
     else enumerate_sector<uint32_t>(b, d_chi_one);

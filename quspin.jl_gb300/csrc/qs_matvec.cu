@@ -953,7 +953,7 @@ void op_prepare_device(Op& op) {
     tables.add(op.d_rowprogs, rows.size() * sizeof(RowProg), rows.data());
     tables.add(op.d_amp, amp.size() * sizeof(double), amp.data());
     tables.add(dprogs, nd * sizeof(TermProg), op.diag_progs.empty() ? nullptr : op.diag_progs.data());
-    tables.place(op.d_tables);
+    tables.place(op.d_tables, op.stream);
     // diagonal: user diagonal plus, when extracted, the diagonal programs
     PoolBuf user;
     if (!op.user_diag.empty()) {
@@ -968,7 +968,7 @@ void op_prepare_device(Op& op) {
     diags.add(op.d_diag_df, b.n * 4 * sizeof(float));
     diags.add(op.d_diag_re, b.n * sizeof(double));
     diags.add(op.d_diag32_re, b.n * sizeof(float));
-    diags.place(op.d_diags);
+    diags.place(op.d_diags, op.stream);
     MvArgs a = base_args(op);
     a.progs = dprogs.as<TermProg>();
     a.nprog = (int)op.diag_progs.size();
