@@ -1565,7 +1565,7 @@ void op_spmv_device(Op& op, const MatvecCall& c, cudaStream_t s) {
     if (M.has_sell) {
         SellArgs a{};
         a.sptr = M.sell_ptr.as<int64_t>();
-            a.len = M.sell_len.as<uint16_t>();
+        a.len = M.sell_len.as<uint16_t>();
         a.words = M.sell_words.as<uint32_t>();
         a.cols = M.sell_cols.as<int32_t>();
         a.codes = M.sell_codes.as<uint16_t>();

@@ -70,11 +70,11 @@ struct TermProg {
 // The same program as the row kernels read it (qs_rows.cuh): alive iff
 // (s & care) == value, image s ^ flip, sign (-1)^popc(s & zy) times its class's
 // amplitude (the constant part of the sign is in the class).  Programs that
-// touch a site twice (chars) pass the test on every state and are run by their
-// characters.
+// touch a site twice (kCharsClass) pass the test on every state and are run by
+// their characters.
 struct RowProg {
     uint64_t care, value, flip, zy;
-    uint32_t cls, chars;
+    uint32_t cls;
 };
 constexpr uint32_t kCharsClass = 0xffffffffu;   // class of a program run by its characters
 

@@ -1555,7 +1555,7 @@ int Engine::add(Op& op, int m, bool cv, int tmp_cols, int orth) {
     const int tc = tmp_cols > 0 ? std::min(tmp_cols, m) : m - 1;
     sl.tmp.alloc((size_t)tc * n * es, s_);
     QS_CUDA(cudaMemsetAsync(sl.V.p, 0, sl.V.bytes, s_));
-    // h1 (m), h2 (m), rec ((m+1) m) as double2, nrm (4 doubles)
+    // h1 (m), h2 (m), rec ((m+1) m) as double2, nrm (8 doubles)
     const size_t nsmall = (size_t)2 * m + (size_t)(m + 1) * m;
     sl.small.alloc(nsmall * sizeof(double2) + 8 * sizeof(double), s_);
     QS_CUDA(cudaMemsetAsync(sl.small.p, 0, sl.small.bytes, s_));

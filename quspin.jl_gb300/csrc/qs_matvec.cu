@@ -169,7 +169,7 @@ __device__ __forceinline__ U row_state(const MvArgs& a, int mode, int64_t r) {
     return s;
 }
 
-// The fixed-weight state of combinadic rank r (inverse of combinadic_rank32),
+// The fixed-weight state of combinadic rank r (inverse of combinadic_rank),
 // with the C(bit, p) table in shared memory.
 __device__ __forceinline__ uint32_t unrank32(int64_t r, const uint32_t* binom32, int L, int nup) {
     uint32_t s = 0, rem = (uint32_t)r;
@@ -878,7 +878,6 @@ void prepare_row_programs(Op& op, std::vector<RowProg>& rows, std::vector<double
         if (!p.distinct) {
             // care = value = 0: alive on every state until its characters say otherwise
             r.cls = kCharsClass;
-            r.chars = 1;
             op.any_chars = true;
             op.check_weight = b.nup >= 0;
             continue;
