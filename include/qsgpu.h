@@ -296,7 +296,10 @@ typedef struct {
  * operator (as qs_eigsh_batch).  A matrix-free operator of at least 4,096
  * states whose assembled form fits in a quarter of free device memory is
  * assembled for the length of the call and runs there too (the form is dropped on return; environment
- * QS_TRANSIENT_ASSEMBLY=0 keeps the call matrix-free). */
+ * QS_TRANSIENT_ASSEMBLY=0 keeps the call matrix-free).  A vector's sign (phase)
+ * obeys no rule of its own: it follows from the start vector and the order in
+ * which the solver adds, which depends on the operator, opts and the form it
+ * runs in alone, so it repeats from run to run and from build to build. */
 QS_API int qs_eigsh(qs_op *op, const qs_eigsh_opts *opts, double *values, void *vectors, qs_eigsh_info *info);
 
 /* eigsh(op; k, which, v0, tol, ncv, maxiter) for a non-Hermitian operator
@@ -312,8 +315,9 @@ QS_API int qs_eigs(qs_op *op, const qs_eigsh_opts *opts, double *values, void *v
  * sector of one model): the Lanczos iterations of all operators run in
  * lockstep on their assembled forms (assembled here if needed): for
  * operators of more than 32,768 states each step is one launch per kernel over
- * all of them, replayed from a captured CUDA graph; smaller operators run their steps up to each restart in one launch with a thread-block
- * cluster per operator.  Operators that converge drop out.  Replaces the per-sector loop of
+ * all of them, replayed from a captured CUDA graph; smaller operators run
+ * their steps up to each restart in one launch with a thread-block cluster per
+ * operator.  Operators that converge drop out.  Replaces the per-sector loop of
  * block_diag_hamiltonian / BlockOps (tools.jl:2213-2420) followed by eigsh on
  * each block.  values: nops * k, ascending per operator; vectors: NULL or nops
  * pointers (each NULL or Ns_i x k in the operator's dtype, host); infos: NULL
