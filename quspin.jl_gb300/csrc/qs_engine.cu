@@ -273,11 +273,17 @@ struct RowSpan {
     }
 };
 __device__ __forceinline__ int row_block(int bx) { return bx / (kT / (int)blockDim.x); }
-__device__ __forceinline__ RowSpan row_span(const SlotDev& S, int bx) {
+// step: a step's sums, which slots that can take the cluster step add in its
+// blocks (the slices of cblocks CTAs, one after another), so that both forms of
+// the step give the same bits; else (normalisation) in blocks of rpb rows.
+__device__ __forceinline__ RowSpan row_span(const SlotDev& S, int bx, bool step = true) {
     const int parts = kT / (int)blockDim.x;
     const int rb = bx / parts, t = (bx % parts) * (int)blockDim.x + (int)threadIdx.x;
-    const int64_t r0 = (int64_t)(rb - S.rb_begin) * S.rpb;
-    return RowSpan{r0 + t, min(S.n, r0 + S.rpb), rb, t / 32};
+    const int64_t b = rb - S.rb_begin;
+    if (step && S.cblocks)
+        return RowSpan{S.nslices * b / S.cblocks * kSellSlice + t, min(S.n, S.nslices * (b + 1) / S.cblocks * kSellSlice),
+                       rb, t / 32};
+    return RowSpan{b * S.rpb + t, min(S.n, (b + 1) * S.rpb), rb, t / 32};
 }
 
 // ------------------------------------------------------------ dots
@@ -618,7 +624,7 @@ __device__ __forceinline__ void dots_block(const SlotDev* sl, const int* __restr
     const int i0 = first + by * jt<A>();
     if (i0 >= nv) return;
     const bool want_wn = by == 0 && (mode == 1 || (mode == 0 && S.orth == 1));
-    const RowSpan R = row_span(S, bx);
+    const RowSpan R = row_span(S, bx, mode != 2);
     double* row = R.sums(partial, mmax);
     A re[jt<A>()], im[jt<A>()], wn = zero<A>();
 #pragma unroll
@@ -715,7 +721,8 @@ __device__ __forceinline__ void advance_slot(SlotDev& S) {
 }
 // The slot's sums of index i (thread 0 of the block returns them); one: a
 // block's total is in its first warp's place.
-__device__ __forceinline__ double2 reduce_sums(const SlotDev& S, const double* partial, int mmax, int i, bool one) {
+__device__ __forceinline__ double2 reduce_sums(const SlotDev& S, const double* partial, int mmax, int i, bool one,
+                                               bool step) {
     const bool cx = S.cv && S.orth != 2 && i != mmax;
     double re = 0, im = 0;
     for (int b = threadIdx.x; b < S.rb_count; b += blockDim.x) {
@@ -733,6 +740,17 @@ __device__ __forceinline__ double2 reduce_sums(const SlotDev& S, const double* p
         }
         re += tr;
         im += ti;
+    }
+    if (step && S.cblocks) {
+        // at most 16 blocks, each in a lane of the first warp: one after another
+        const double br = re, bi = im;
+        re = im = 0;
+        if (threadIdx.x < 32)
+            for (int b = 0; b < S.cblocks; ++b) {
+                re += __shfl_sync(0xffffffffu, br, b);
+                im += __shfl_sync(0xffffffffu, bi, b);
+            }
+        return make_double2(re, im);
     }
     for (int o = 16; o > 0; o >>= 1) {
         re += __shfl_xor_sync(0xffffffffu, re, o);
@@ -790,9 +808,9 @@ __device__ __forceinline__ void reduce_block(SlotDev* sl, int mmax, int mode, co
     const int ld = S.m + 1;
     const int j = S.j;
     double2* col = S.rec + (size_t)j * ld;
-    const double2 t = reduce_sums(S, partial, mmax, mode == 1 ? mmax : i, one);
+    const double2 t = reduce_sums(S, partial, mmax, mode == 1 ? mmax : i, one, mode != 4);
     double2 h = make_double2(0.0, 0.0);
-    if (mode == 1 && i != mmax) h = reduce_sums(S, partial, mmax, i, one);
+    if (mode == 1 && i != mmax) h = reduce_sums(S, partial, mmax, i, one, true);
     if (threadIdx.x) return;
     const double nb = sqrt(fmax(t.x, 0.0));
     if (mode == 0) {
@@ -1096,7 +1114,7 @@ __device__ __forceinline__ void scale_block(const SlotDev* sl, const int* __rest
         return;
     const A f = from_d<A>(S.nrm[1]);
     void* w = colp<A>(S, mode == 0 ? S.j : S.ncol);
-    const RowSpan R = row_span(S, bx);
+    const RowSpan R = row_span(S, bx, mode == 0);
     if (S.cv) scale_rows<A, true>(w, R.r, R.r1, kT, f);
     else scale_rows<A, false>(w, R.r, R.r1, kT, f);
 }
@@ -1187,12 +1205,19 @@ __device__ __forceinline__ void rotate_rows_tile(const SlotDev& S, int64_t r0, i
     }
 }
 
+// rows of a rotation block: the slot's row blocks, or (cblocks, more of them than
+// blocks of rpb rows) an equal part of its rows in whole tiles of 128
+__device__ __forceinline__ int64_t rotate_block(const SlotDev& S) {
+    return S.cblocks ? ((S.n + S.rb_count - 1) / S.rb_count + 127) / 128 * 128 : S.rpb;
+}
+
 template <class A>
 __global__ void __launch_bounds__(kT, 2) eng_rotate(const SlotDev* __restrict__ sl, const int* __restrict__ rmap) {
     const SlotDev& S = sl[rmap[blockIdx.x]];
     if (S.state != kSlotRotate || S.rot_tc) return;
     // blockIdx.y: this block's share of the row block (gridDim.y shares)
-    const int64_t b0 = (int64_t)(blockIdx.x - S.rb_begin) * S.rpb, b1 = min(S.n, b0 + S.rpb);
+    const int64_t per = rotate_block(S);
+    const int64_t b0 = min(S.n, (int64_t)(blockIdx.x - S.rb_begin) * per), b1 = min(S.n, b0 + per);
     const int64_t share = (b1 - b0 + gridDim.y - 1) / gridDim.y;
     const int64_t r0 = min(b1, b0 + (int64_t)blockIdx.y * share), r1 = min(b1, r0 + share);
     if (S.p <= 8) {
@@ -1285,7 +1310,8 @@ __global__ void __launch_bounds__(kTcRows, 1) eng_rotate_tc(const SlotDev* __res
     const int64_t lb = blockIdx.x - S.rb_begin;
     // blockIdx.y: this block's share of the row block (gridDim.y shares of
     // whole tiles), so that a small engine still fills the GPU
-    const int64_t rb0 = lb * S.rpb, rb1 = min(S.n, rb0 + S.rpb);
+    const int64_t per = rotate_block(S);
+    const int64_t rb0 = min(S.n, lb * per), rb1 = min(S.n, rb0 + per);
     const int64_t share = ((rb1 - rb0 + gridDim.y - 1) / gridDim.y + kTcRows - 1) / kTcRows * kTcRows;
     const int64_t r0 = min(rb1, rb0 + (int64_t)blockIdx.y * share), r1 = min(rb1, r0 + share);
     const int64_t e0 = r0 * comps, e1 = r1 * comps;
@@ -1441,7 +1467,9 @@ VKind store_kind(Store st, bool cv) {
 // rpb of Gram-Schmidt slots: 4,096.  The eigenvectors of a solve come from
 // its projected matrix, whose eigensolver gives a column either sign, decided
 // by the matrix's last bits; so the order of these sums is part of a solve's
-// output and stays as it is (RowSpan says how it is spread over the GPU).
+// output and stays as it is (RowSpan says how it is spread over the GPU).  Slots
+// of up to kClusterRows16 rows, whose steps were all run by the cluster step
+// once, add a step's sums in its blocks (SlotDev::cblocks).
 // rpb of three-term slots (evolution: no sign is free): whole waves of 304
 // equal blocks of at most 8,192 and at least 768 rows.
 // spb: one slice per warp spreads a slot of 90,000 rows over 352 blocks (5.9
@@ -1449,6 +1477,8 @@ VKind store_kind(Store st, bool cv) {
 // blocks enough and two slices per warp save the value table's staging
 // (4.7 M rows: 128.8 against 130.4 ms).
 constexpr int kGramRows = 4096, kWaveBlocks = 304;
+
+constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 32768;   // slots of eight CTAs, of sixteen
 
 Tiles tiles_for(int64_t n, int64_t nslices, int orth) {
     Tiles t;
@@ -1572,6 +1602,8 @@ int Engine::add(Op& op, int m, bool cv, int tmp_cols, int orth) {
     d.carry = -1;
     d.orth = orth;
     d.fused = fused_slot(st_, n, cv, orth);
+    // (at least as many as the slot has blocks of 4,096 rows)
+    d.cblocks = orth == 2 || n > kClusterRows16 ? 0 : n > kClusterRows8 && cluster16_ok() ? 16 : 8;
     sl.tcols = tc;
     const Tiles t = tiles_for(n, M.nslices, orth);
     d.rpb = t.rpb;
@@ -1608,7 +1640,7 @@ void Engine::build_maps() {
             continue;
         }
         d.rb_begin = nrb_;
-        d.rb_count = (int)((d.n + d.rpb - 1) / d.rpb);
+        d.rb_count = d.cblocks ? d.cblocks : (int)((d.n + d.rpb - 1) / d.rpb);
         d.sb_begin = nsb_;
         d.sb_count = (int)((d.nslices + d.spb - 1) / d.spb);
         nrb_ += d.rb_count;
@@ -1722,8 +1754,8 @@ static int launch_step_t(const SlotDev* ds, SlotDev* dsw, const int* rm, const i
 // decision without a broadcast.  CTA 0 writes the step's record column; the
 // slot's row range ends on a cluster barrier before the next product gathers
 // from it.  Nothing crosses clusters, so a slot's result does not depend on
-// the others; the reduction order (one partial per CTA) differs from the
-// graph replay's (one per row block), so results agree to rounding.
+// the others.  The graph replay adds the sums of Gram-Schmidt slots in the same
+// blocks and order (SlotDev::cblocks), so those get the same bits from both.
 __device__ __forceinline__ uint32_t cl_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -2175,37 +2207,30 @@ void grid_barrier_check(int phantom, double limit_ms, int blocks) {
     if (h.gen != (unsigned)rounds) throw Error(QS_ERR_CUDA, "grid barrier completed a wrong number of rounds");
 }
 
-// Which stepping slots take the cluster step, and with how many CTAs: by the
-// slot and the storage, so that a slot's result is the same alone and in any
-// batch.  Up to 8,192 rows eight CTAs, above sixteen, which save the launch
-// gaps of a step's kernels but have 16 SMs' FP64 rate, where the graph spreads
-// a slot over all of them.
-// Gram-Schmidt slots: up to 32,768 rows.  The two forms add in different
-// orders, and with the order an eigenvector's sign can change (tiles_for), so
-// this line stays although the graph is the faster form on part of it (ground
-// states, cluster / graph in ms): real matrix 4,262 rows 3.8/4.6, 12,870 rows
-// 5.7/6.0, 19,448 rows 6.6/6.3, 28,968 rows 7.5/5.0; complex 9,690 rows 8.0/7.1,
-// 16,796 rows 14.5/8.8, 29,372 rows 22.2/9.2; double-float 12,870 rows 5.0/5.6,
-// 28,968 rows 6.5/4.5, complex 16,796 rows 8.1/7.9.
-// Three-term slots, whose output has no free sign: where the two cross
-// (evolution to four times): real FP64 12,870 rows 2.5/2.7, 16,796 rows 3.3/3.0;
-// double-float 19,448 rows 2.5/2.7, 24,310 rows 2.8/2.75; complex FP64 9,690 rows
-// 3.0/3.1, 14,000 rows 3.6/3.3; double-float 16,796 rows 3.0/3.1, 22,610 rows 3.3/3.1.
-constexpr int64_t kClusterRows8 = 8192, kClusterRows16 = 32768;
-constexpr int64_t kClusterThree = 14336, kClusterThreeDf = 20480;
-constexpr int64_t kClusterThreeComplex = 10240, kClusterThreeComplexDf = 18432;
+// Which stepping slots take the cluster step: by the slot and the storage.  Up
+// to kClusterRows8 rows eight CTAs, above sixteen, which save the launch gaps of
+// a step's kernels but have 8 or 16 SMs' FP64 rate, where the graph spreads a slot
+// over all of them.  Gram-Schmidt slots of up to kClusterRows16 rows get the same
+// bits from both (SlotDev::cblocks), larger ones and three-term slots the same to
+// rounding.  The lines are where the two cross (cluster / graph in ms).
+// Ground states, real: FP64 4,262 rows 3.8/3.8, 8,359 rows 4.1/4.1, 12,870 rows
+// 5.7/5.4, 28,968 rows 7.5/4.7; double-float 12,870 rows 5.0/5.1, 16,796 rows
+// 7.8/6.8; FP32 19,448 rows 2.7/3.0, 24,310 rows 6.7/5.9.  Complex: FP64 800 rows
+// 4.0/5.2, 2,424 rows 6.2/5.6, 9,225 rows 12.1/8.2; double-float 9,690 rows 4.8/5.0,
+// 14,000 rows 5.7/5.1; FP32 14,000 rows 2.9/3.0, 16,796 rows 3.8/3.5.
+// Evolution to four times, real: FP64 12,870 rows 2.5/2.8, 16,796 rows 3.3/3.1;
+// double-float 19,448 rows 2.5/2.7, 24,310 rows 2.8/2.75; complex: FP64 9,690 rows
+// 3.0/3.2, 14,000 rows 3.6/3.3; double-float 16,796 rows 3.0/3.1, 22,610 rows 3.4/3.2.
+constexpr int64_t kClusterGram[2][3] = {{8192, 14336, 20480}, {2048, 10240, 14336}};     // real, complex matrix:
+constexpr int64_t kClusterThree[2][3] = {{14336, 20480, 20480}, {10240, 18432, 18432}};  // FP64, double-float, FP32
 
 int Engine::cluster_size_for(const SlotDev& d) const {
     const char* e = std::getenv("QS_CLUSTER_STEP");
     if (e && e[0] == '0') return 0;
     if (!(e && e[0] == '1') && persistent_wanted()) return 0;
-    if (d.n <= kClusterRows8) return 8;
-    const bool f64 = st_ == Store::F64;
-    const int64_t limit = d.orth != 2 ? kClusterRows16
-                          : d.cm      ? (f64 ? kClusterThreeComplex : kClusterThreeComplexDf)
-                                      : (f64 ? kClusterThree : kClusterThreeDf);
-    if (d.n <= limit || (e && e[0] == '1')) return cluster16_ok() ? 16 : 8;
-    return 0;
+    const int64_t limit = (d.orth != 2 ? kClusterGram : kClusterThree)[d.cm ? 1 : 0][(int)st_];
+    if (d.n > limit && !(e && e[0] == '1')) return 0;
+    return d.n > kClusterRows8 && cluster16_ok() ? 16 : 8;
 }
 
 // Sixteen CTAs per cluster are a non-portable size: allowed per kernel, and

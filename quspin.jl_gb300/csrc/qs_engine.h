@@ -72,6 +72,9 @@ struct SlotDev {
     double* nrm;
     int32_t m, j, state;
     int32_t fused;          // the vector passes run on the fused kernels
+    // blocks of a step's sums as the cluster step adds them: its CTAs' slices, one
+    // after another (0: blocks of rpb rows)
+    int32_t cblocks;
     // orthogonalisation of a step: 0 classical Gram-Schmidt twice (CGS2);
     // 1 CGS with the DGKS correction only when ||w'|| < 0.717 ||w|| (ARPACK's
     // dsaitr test); 2 Lanczos three-term recurrence (Hermitian operators,

@@ -96,19 +96,22 @@ def test_signs_between_the_step_forms(qs, model, L, nup, sym, i, n, seed, precis
     assert sign_of(qs, model, L, nup, sym, "H", c, seed, precision, which) == sign
 
 
-@pytest.mark.parametrize("L,nup,sym,precision,rows", [
-    (17, 8, {}, "fp64", 24310), (17, 8, {}, "fp64df", 24310), (17, 8, {}, "fp32", 24310),
-    (20, 10, dict(kblock=3), "fp64", 9225), (21, 10, dict(kblock=2), "fp64df", 16796)])
-def test_solves_take_the_cluster_step(qs, monkeypatch, L, nup, sym, precision, rows):
-    """A solve of up to 32,768 rows adds in the cluster step's order."""
+# one CTA's slices empty, eight and sixteen CTAs, both ends of their ranges
+@pytest.mark.parametrize("precision", ["fp64", "fp64df", "fp32"])
+@pytest.mark.parametrize("L,nup,sym,rows", [
+    (8, 4, {}, 70), (14, 7, EVEN, 85), (14, 6, dict(kblock=3), 212), (22, 11, EVEN, 8359), (17, 8, {}, 24310),
+    (20, 10, dict(kblock=3), 9225), (21, 10, dict(kblock=2), 16796), (33, 3, {}, 5456), (22, 11, dict(kblock=1), 32065)])
+def test_step_forms_give_the_same_bits(qs, monkeypatch, L, nup, sym, rows, precision):
+    """Solves of up to 32,768 rows: the cluster step, the graph replay and the rule."""
     b = qs.SpinBasis1D(L, nup=nup, pauli=False, **sym)
     assert b.Ns == rows
     H = qs.Hamiltonian(b, models.to_terms(qs, models.j1j2(L, 1.0, 0.3)))
     got = []
-    for form in ("", "1"):
+    for form in ("", "0", "1"):
         monkeypatch.setenv("QS_CLUSTER_STEP", form)
         got.append(qs.eigsh(H, k=2, tol=1e-11, precision=precision))
-    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    for vals, vecs in got[1:]:
+        assert np.array_equal(vals, got[0][0]) and np.array_equal(vecs, got[0][1])
 
 
 # ... and when the terms of the matrix-free product (operators of fewer than
